@@ -182,6 +182,9 @@ gdt_status tune_spmv(gdt_context ctx, gdt_matrix m, double* times_ms = nullptr);
 // SELL-32 copy of m: slice table built once per pattern (GDT_EUNSUPPORTED when there is no room or the
 // offsets do not fit 32 bits), values and columns copied when the values changed or `refill` is set
 gdt_status sell_prepare(gdt_context ctx, gdt_matrix m, cudaStream_t s, bool refill);
+// the copy without the zero values, for solves whose vectors are finite by their own checks (a product
+// keeps them: 0 * inf is not 0): width (device, one per 32-row slice) receives the entries per row
+gdt_status sell_prepare_nonzero(gdt_context ctx, gdt_matrix m, cudaStream_t s, int* width);
 void sell_free(gdt_matrix m);
 // index of the SELL-32 schedule in gdt_matrix_tune / gdt_matrix_set_schedule
 constexpr int kSellSchedule = 8;

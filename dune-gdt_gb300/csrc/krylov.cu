@@ -640,29 +640,31 @@ void ilu_apply(gdt_context ctx, gdt_matrix m, const Ilu& f, const double* r, dou
 
 
 // ------------------------------------------------------------------------- persistent CG ---
-// One cooperative launch runs every iteration of Jacobi-preconditioned (or plain) CG. The kernel
-// boundaries of the graph form become grid barriers, three per iteration: after q = A p, after the
-// x/r update, after the direction update. Every block reduces the per-block partial sums itself, in
-// block order, so all blocks hold bit-identical alpha, beta and convergence decisions without a
-// broadcast step. This pays most where an iteration is bound by launch, ramp-up and tail latency
-// rather than bandwidth (matrices and vectors that stay in the 129 MB L2), and also where the SpMV
-// streams the matrix from HBM (no kernel boundaries, no row-pointer indirection). The Chronopoulos-Gear form (one
-// reduction and two barriers per iteration) measured slower here (277 against 250 ms for the SWIPDG
-// system of 256^2 squares) and needed up to 65 % more iterations on badly conditioned 1D and 2D
-// systems, so the iteration stays the standard one of the graph form. The SpMV reads a SELL-32 copy
-// of the matrix (slices of 32 rows stored column-major, padded to the slice's longest row): a lane
-// owns one row and reads its entries with loads that are coalesced across the warp, so a pass over
-// 32 rows costs two dependent memory latencies (entries, gathers) and no shared memory. (Staging each
-// warp's CSR slice in shared memory instead cost three latencies per pass and 8-way bank conflicts
-// when the lanes read their rows: 17.6 us of a 43 us iteration on that SWIPDG system.) The matrix
-// and the Jacobi diagonal are read-only in the kernel (non-coherent loads); the vectors are written
-// by other blocks between barriers and read with plain loads, which the barrier's fences order.
-constexpr int PT = 1024;  // threads per block (one block per SM)
-
+// One cooperative launch runs every iteration of Jacobi-preconditioned (or plain) CG; two grid-wide
+// sums per iteration take the place of the graph form's kernel boundaries.
+//
+// What bounds an iteration here is not bandwidth but the FP64 pipe (one warp instruction per 19 SM
+// cycles) and the grid-wide waits, so the kernel is built around those two:
+//  * The x, r and direction updates are one pass. beta needs rho' = r'.z', which classically waits for
+//    a sum over the updated residual. With r' = r - alpha q it is rho - 2 alpha (z.q) + alpha^2 (q.D^-1 q),
+//    and both products are summed together with p.q right after q = A p (cf. Meurant 1987). beta takes
+//    that value; alpha and the stopping test take the sums over the residual itself, so nothing
+//    accumulates: the iteration counts are those of the classical form, also on badly conditioned 1D
+//    systems, where the shorter alpha^2 (q.D^-1 q) - rho (z.q = p.q) needs up to 38 % more.
+//  * A grid-wide sum and the barrier it implies are one exchange (grid_exchange below).
+//  * A thread owns its rows for the whole solve: x, r, p, D^-1 and q of k_pcg_resident never leave its
+//    registers (p is also written for the neighbours' gathers), and a block keeps as much of its
+//    matrix as fits in shared memory.
+//  * Entries that are exactly zero (the hypotenuse couplings of P1 on right-angled simplices, the
+//    columns of Dirichlet rows) are dropped from the SELL-32 copy: no loads and no FMAs for them.
+//  * Work is spread over all SMs, down to one 32-row slice per block.
+// The matrix and D^-1 are read-only in the kernels (non-coherent loads); p is written by other blocks
+// between the sums and read with plain loads, which the fences of grid_exchange order.
 struct PcgArgs {
   int n;
   int nslices;
   const int2* meta;   // SELL-32 (offset, width) per slice
+  const int* width;   // entries per row of the slice after dropping zeros
   const int* col;     // SELL-32 columns
   const double* val;  // SELL-32 values
   const double* dinv;
@@ -670,152 +672,46 @@ struct PcgArgs {
   double* r;
   double* p;
   double* q;
-  double* z;  // dinv r, kept by the update for the direction step
   KState* st;
-  double* part;       // 3 * gridDim.x doubles: p.q | r.z, r.r per block
-  unsigned int* bar;  // 64-bit arrival count at bar[0], generation at bar[kBarGen], fault at bar[kBarFault]
-  unsigned long long wait_ns;  // longest wait at a grid barrier
+  unsigned long long* slots;   // packets of grid_exchange
+  unsigned int* fault;         // set when a wait ran out
+  unsigned long long wait_ns;  // longest wait in a grid_exchange
+  int cap;                     // matrix entries a block may keep in shared memory (resident form)
+  int stream;                  // the matrix exceeds L2: mark its lines evict-first
 };
-// q = A p over the warp's slices (rows of at most 32 entries); returns this thread's share of p.q.
-// The slices of a warp are the same in every iteration: lane m holds the (offset, width) of the
-// warp's m-th slice, so a pass gets them by a shuffle instead of a load.
-__device__ __forceinline__ double pcg_spmv(const PcgArgs& a, int2 mymeta) {
-  const int lane = threadIdx.x & 31;
-  const int nw = gridDim.x * (PT / 32);
-  double pq = 0.0;
-  int m = 0;
-  for (int slice = blockIdx.x * (PT / 32) + (threadIdx.x >> 5); slice < a.nslices; slice += nw, ++m) {
-    int2 md;
-    if (m < 32) {
-      md.x = __shfl_sync(0xffffffffu, mymeta.x, m);
-      md.y = __shfl_sync(0xffffffffu, mymeta.y, m);
-    } else {
-      md = __ldg(a.meta + slice);
-    }
-    const int row = slice * 32 + lane;
-    const bool act = row < a.n;
-    const double pr = act ? a.p[row] : 0.0;
-    const double* v = a.val + md.x + lane;
-    const int* c = a.col + md.x + lane;
-    double s0 = 0.0, s1 = 0.0;
-#pragma unroll
-    for (int t0 = 0; t0 < 32; t0 += 12) {
-      if (t0 < md.y) {  // warp-uniform
-        double vv[12];
-        int cc[12];
-#pragma unroll
-        for (int j = 0; j < 12; ++j) {
-          const bool in = t0 + j < md.y;
-          vv[j] = in ? __ldg(v + (t0 + j) * 32) : 0.0;
-          cc[j] = in ? __ldg(c + (t0 + j) * 32) : 0;
-        }
-#pragma unroll
-        for (int j = 0; j < 12; j += 2) {
-          if (t0 + j < md.y) s0 = fma(vv[j], a.p[cc[j]], s0);
-          if (t0 + j + 1 < md.y) s1 = fma(vv[j + 1], a.p[cc[j + 1]], s1);
-        }
-      }
-    }
-    const double s = s0 + s1;
-    if (act) {
-      a.q[row] = s;
-      pq = fma(pr, s, pq);
-    }
-  }
-  return pq;
-}
 
-__global__ void __launch_bounds__(PT, 1) k_pcg_persistent(PcgArgs a) {
-  __shared__ double red[2 * 32];
-  __shared__ double bc[2];
-  int2 mymeta = make_int2(0, 0);
-  {
-    const int slice = blockIdx.x * (PT / 32) + (threadIdx.x >> 5) + (threadIdx.x & 31) * gridDim.x * (PT / 32);
-    if (slice < a.nslices) mymeta = __ldg(a.meta + slice);
+// The grid-wide sums of an iteration. One exchange is a sum of up to three values per thread and the grid barrier
+// in one (all blocks co-resident): the block sums go out as one 32-byte packet, four words of 48 payload
+// bits each beside 16 bits of the number of the sum, and every block polls all packets until their
+// words carry that number. All blocks add the packets in the same order, so all hold the same bits and
+// none has to broadcast a decision. Two packet buffers alternate: a block can only write sum k + 2 after
+// all have written k + 1, that is after all have read k.
+// Polls delay the stores to the line they read, so a block's packet has 256 bytes of its own (152 blocks
+// exchange in 0.98 us like that, in 2.4 us with packets of 16 bytes side by side) and is read once, not
+// once per value (three values: 3.3 us with a packet and a polling warp each).
+// An FP64 instruction occupies a quarter of the SM for 64 cycles, whichever warp issues it. So the block sums
+// are formed by one warp per value from the threads' values in shared memory (a shuffle tree in every
+// warp would issue five instructions for each one of these), and the scalars that follow, a
+// reciprocal and a few products, by thread 0 alone.
+// Every wait is bounded (time and count); a wait that runs out sets the fault flag, and every block
+// leaves from then on.
+constexpr int kSlot = 32;  // 64-bit words per block and buffer
+
+// The scalars of the iteration, kept by thread 0 of every block (the same bits in all of them).
+struct PcgScalars {
+  double rho, alpha, beta, rr, stop;
+  int iter, max_iter, conv, brk;
+  __device__ void load(const KState* st) {
+    rho = st->rho;
+    alpha = st->alpha;
+    beta = st->beta;
+    rr = st->rr;
+    stop = st->tol2 * st->rr0;
+    iter = st->iter;
+    max_iter = st->max_iter;
+    conv = brk = 0;
   }
-  KState* st = a.st;
-  if (entry_flag(&st->converged)) return;
-  double rho = st->rho, alpha = st->alpha, beta = st->beta, rr = st->rr;
-  const double stop = st->tol2 * st->rr0;
-  const int max_iter = st->max_iter;
-  int iter = st->iter, conv = 0, brk = 0;
-  const int nb = gridDim.x;
-  const int stride = nb * PT;
-  unsigned int epoch = 0;
-  while (true) {
-    // q = A p, p.q -> alpha
-    double v1[1] = {pcg_spmv(a, mymeta)};
-    block_reduce<1>(v1, red);
-    if (threadIdx.x == 0) a.part[blockIdx.x] = v1[0];
-    if (!grid_barrier(a.bar, epoch, a.wait_ns)) break;
-    grid_allreduce<1>(a.part, v1, bc);
-    alpha = rho / v1[0];
-    if (!(v1[0] > 0.0) || !isfinite(v1[0])) {
-      brk = conv = 1;
-      break;
-    }
-    // x += alpha p, r -= alpha q; r.z (z = dinv r) and r.r
-    // (two elements per thread and pass, all their loads issued before the first store)
-    double v2[2] = {0.0, 0.0};
-    for (int i0 = blockIdx.x * PT + threadIdx.x; i0 < a.n; i0 += 2 * stride) {
-      double pv[2], qv[2], xv[2], rv[2], dv[2];
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int i = i0 + u * stride;
-        const bool in = i < a.n;
-        pv[u] = in ? a.p[i] : 0.0;
-        qv[u] = in ? a.q[i] : 0.0;
-        xv[u] = in ? a.x[i] : 0.0;
-        rv[u] = in ? a.r[i] : 0.0;
-        dv[u] = in ? __ldg(a.dinv + i) : 0.0;
-      }
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int i = i0 + u * stride;
-        if (i < a.n) {
-          a.x[i] = fma(alpha, pv[u], xv[u]);
-          const double ri = fma(-alpha, qv[u], rv[u]);
-          const double zi = dv[u] * ri;
-          a.r[i] = ri;
-          a.z[i] = zi;
-          v2[0] = fma(ri, zi, v2[0]);
-          v2[1] = fma(ri, ri, v2[1]);
-        }
-      }
-    }
-    block_reduce<2>(v2, red);
-    if (threadIdx.x == 0) {
-      a.part[nb + blockIdx.x] = v2[0];
-      a.part[2 * nb + blockIdx.x] = v2[1];
-    }
-    if (!grid_barrier(a.bar, epoch, a.wait_ns)) break;
-    grid_allreduce<2>(a.part + nb, v2, bc);
-    beta = v2[0] / rho;
-    rho = v2[0];
-    rr = v2[1];
-    iter += 1;
-    if (rr <= stop || iter >= max_iter) conv = 1;
-    if (!isfinite(rr)) brk = conv = 1;
-    if (conv) break;
-    // p = dinv r + beta p
-    for (int i0 = blockIdx.x * PT + threadIdx.x; i0 < a.n; i0 += 3 * stride) {
-      double pv[3], zv[3];
-#pragma unroll
-      for (int u = 0; u < 3; ++u) {
-        const int i = i0 + u * stride;
-        const bool in = i < a.n;
-        pv[u] = in ? a.p[i] : 0.0;
-        zv[u] = in ? a.z[i] : 0.0;
-      }
-#pragma unroll
-      for (int u = 0; u < 3; ++u) {
-        const int i = i0 + u * stride;
-        if (i < a.n) a.p[i] = fma(beta, pv[u], zv[u]);
-      }
-    }
-    if (!grid_barrier(a.bar, epoch, a.wait_ns)) break;
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
+  __device__ void store(KState* st) const {
     st->rho = rho;
     st->alpha = alpha;
     st->beta = beta;
@@ -824,12 +720,403 @@ __global__ void __launch_bounds__(PT, 1) k_pcg_persistent(PcgArgs a) {
     st->breakdown = brk;
     st->converged = 1;
   }
+};
+
+template <int T>
+struct PcgShared {
+  double part[3][T];
+  double packet[3][T];  // of block b at [..][b]
+  double own[3];
+  double total[3];
+  double last[2];
+  PcgScalars k;
+  int go;
+  int fault;
+};
+
+__device__ __forceinline__ double sum_strided(const double* v, int groups) {
+  // lane l: v[l] + v[32 + l] + ... in a fixed order, four sums side by side
+  double s[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) s[j] = j < groups ? v[32 * j] : 0.0;
+#pragma unroll 1
+  for (int j0 = 4; j0 < groups; j0 += 4)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (j0 + j < groups) s[j] += v[32 * (j0 + j)];
+  double b = s[0];
+  if (groups > 2) b = (s[0] + s[1]) + (s[2] + s[3]);
+  else if (groups > 1) b = s[0] + s[1];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) b += __shfl_xor_sync(0xffffffffu, b, o);
+  return b;
 }
 
-// Rows of at most 32 entries (the SELL-32 SpMV's limit). Measured against the graph form: 40.6 against
-// 51.7 us per iteration for the L2-resident SWIPDG system of 256^2 squares, and 209 against 264 us
-// for the 128^3 Q1 system (727.7 MB streamed from HBM per SpMV), same iteration counts: AUTO takes it
-// wherever it applies.
+// Sum of v over the grid, returned in all lanes of warp k for value k (k < NV); the first `warps` warps hold rows.
+// RELEASE: the block's writes before the call are visible to every block after its next block barrier;
+// without it only the order of their reads before the call and this block's writes after it is kept.
+// At most T blocks.
+template <bool RELEASE, int NV, int T>
+__device__ __forceinline__ double grid_exchange(const PcgArgs& a, unsigned int& epoch, const double (&v)[NV], int warps,
+                                                PcgShared<T>& sh) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nb = gridDim.x;
+  ++epoch;
+  if (warp < warps) {
+#pragma unroll
+    for (int k = 0; k < NV; ++k) sh.part[k][threadIdx.x] = v[k];
+  }
+  __syncthreads();
+  unsigned long long* const base = a.slots + (size_t)kSlot * nb * (epoch & 1u);
+  const unsigned long long tag = (unsigned long long)epoch << 48;
+  if (warp < NV) {
+    const double b = sum_strided(sh.part[warp] + lane, warps);
+    if (lane == 0) sh.own[warp] = b;
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * NV) : "memory");
+    if (threadIdx.x == 0) {
+      unsigned long long w[3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) w[k] = k < NV ? __double_as_longlong(sh.own[k]) : 0ull;
+      if (RELEASE) fence_acq_rel_gpu();
+      asm volatile("st.relaxed.gpu.global.v4.u64 [%0], {%1, %2, %3, %4};" ::"l"(base + kSlot * blockIdx.x),
+                   "l"((w[0] & 0xffffffffffffull) | tag), "l"((w[0] >> 48) | ((w[1] & 0xffffffffull) << 16) | tag),
+                   "l"((w[1] >> 32) | ((w[2] & 0xffffull) << 32) | tag), "l"((w[2] >> 16) | tag)
+                   : "memory");
+    }
+  }
+  if (warp * 32 < nb) {
+    unsigned long long w[4] = {0, 0, 0, 0}, t0 = 0;
+    bool wait = (int)threadIdx.x < nb;
+    for (unsigned int spins = 1;; ++spins) {
+      if (wait) {
+        if (RELEASE)
+          asm volatile("ld.acquire.gpu.global.v4.u64 {%0, %1, %2, %3}, [%4];"
+                       : "=l"(w[0]), "=l"(w[1]), "=l"(w[2]), "=l"(w[3])
+                       : "l"(base + kSlot * threadIdx.x)
+                       : "memory");
+        else
+          asm volatile("ld.relaxed.gpu.global.v4.u64 {%0, %1, %2, %3}, [%4];"
+                       : "=l"(w[0]), "=l"(w[1]), "=l"(w[2]), "=l"(w[3])
+                       : "l"(base + kSlot * threadIdx.x)
+                       : "memory");
+        wait = (((w[0] ^ tag) | (w[1] ^ tag) | (w[2] ^ tag) | (w[3] ^ tag)) >> 48) != 0;
+      }
+      if (!__any_sync(0xffffffffu, wait)) break;
+      if (spins == 1u) t0 = global_ns();
+      else if (spins == 2u || (spins & 255u) == 0u) {
+        const bool out = spins > (1u << 24) || global_ns() - t0 > a.wait_ns;
+        if (out) atomicExch(a.fault, 1u);
+        if (__any_sync(0xffffffffu, out || *reinterpret_cast<volatile unsigned int*>(a.fault) != 0u)) {
+          if (lane == 0) sh.fault = 1;
+          break;
+        }
+      }
+    }
+    // (a thread past the last block holds zeros)
+    sh.packet[0][threadIdx.x] = __longlong_as_double((w[0] & 0xffffffffffffull) | (w[1] << 48));
+    sh.packet[1][threadIdx.x] = __longlong_as_double(((w[1] >> 16) & 0xffffffffull) | (w[2] << 32));
+    if (NV > 2) sh.packet[2][threadIdx.x] = __longlong_as_double(((w[2] >> 32) & 0xffffull) | (w[3] << 16));
+  }
+  __syncthreads();
+  return warp < NV ? sum_strided(sh.packet[warp] + lane, (nb + 31) >> 5) : 0.0;
+}
+
+// v = (p.q, z.q, q.D^-1 q) over the rows of the thread: alpha and beta in sh.k; false when done. The stopping test
+// of the iteration before is made here too: its sums (sh.last) are formed while the other warps
+// already multiply, so a solve ends with one product it does not use.
+template <int T>
+__device__ __forceinline__ bool pcg_step(const PcgArgs& a, unsigned int& epoch, const double (&v)[3], int warps,
+                                         PcgShared<T>& sh) {
+  const bool first = epoch == 0;
+  const double total = grid_exchange<false>(a, epoch, v, warps, sh);
+  if (threadIdx.x < 96) {
+    const double inv = threadIdx.x == 0 ? 1.0 / total : 0.0;
+    if ((threadIdx.x & 31) == 0) sh.total[threadIdx.x >> 5] = total;
+    asm volatile("bar.sync 1, 96;" ::: "memory");
+    if (threadIdx.x == 0) {
+      PcgScalars& k = sh.k;
+      if (!first) {
+        k.rho = sh.last[0];
+        k.rr = sh.last[1];
+        k.iter += 1;
+        if (k.rr <= k.stop || k.iter >= k.max_iter) k.conv = 1;
+        if (!isfinite(k.rr)) k.brk = k.conv = 1;
+      }
+      if (!k.conv) {
+        k.alpha = k.rho * inv;
+        k.beta = fma(k.alpha * inv, sh.total[2], fma(-2.0 * inv, sh.total[1], 1.0));
+        if (!(total > 0.0) || !isfinite(total)) k.brk = k.conv = 1;
+      }
+      sh.go = !k.conv && !sh.fault;
+    }
+  }
+  __syncthreads();
+  return sh.go != 0;
+}
+
+// v = (r.z, r.r) of the updated residual; p is visible to every block from here on
+template <int T>
+__device__ __forceinline__ void pcg_publish(const PcgArgs& a, unsigned int& epoch, const double (&v)[2], int warps,
+                                            PcgShared<T>& sh) {
+  const double total = grid_exchange<true>(a, epoch, v, warps, sh);
+  if (threadIdx.x < 64 && (threadIdx.x & 31) == 0) sh.last[threadIdx.x >> 5] = total;
+}
+
+// s += v[J] p[J] + ... + v[cnt - 1] p[cnt - 1] (cnt warp-uniform). A predicated-off FP64 instruction takes its 64 cycles
+// like any other (measured: a masked second row doubled a pass), hence nested branches, not masks.
+template <int J, int CH>
+__device__ __forceinline__ void fma_chain(int cnt, const double (&v)[CH], const double (&p)[CH], double& s) {
+  if constexpr (J < CH) {
+    if (cnt > J) {
+      s = fma(v[J], p[J], s);
+      fma_chain<J + 1>(cnt, v, p, s);
+    }
+  }
+}
+
+// sum of a row's products, entries t of the lane's row at v[32 t], c[32 t]; w is warp-uniform. All loads of
+// CH entries are issued before their FMAs. One accumulator: with 16 or more warps on the SM each
+// warp's turn at the FP64 pipe comes after the FMA's latency, and a second one would cost an add.
+template <int CH, class LoadV, class LoadC>
+__device__ __forceinline__ double pcg_row(int w, const double* p, LoadV v, LoadC c) {
+  double s = 0.0;
+#pragma unroll 1
+  for (int t0 = 0; t0 < w; t0 += CH) {
+    double vv[CH], pv[CH];
+#pragma unroll
+    for (int j = 0; j < CH; ++j) {
+      vv[j] = pv[j] = 0.0;
+      if (t0 + j < w) {
+        vv[j] = v(t0 + j);
+        pv[j] = p[c(t0 + j)];
+      }
+    }
+    fma_chain<0>(w - t0, vv, pv, s);
+  }
+  return s;
+}
+
+__device__ __forceinline__ unsigned long long matrix_policy(int stream) {
+  unsigned long long pol;
+  if (stream) asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
+  else asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(pol));
+  return pol;
+}
+__device__ __forceinline__ double ld_matrix(const double* a, unsigned long long pol) {
+  double v;
+  asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(a), "l"(pol));
+  return v;
+}
+__device__ __forceinline__ int ld_matrix(const int* a, unsigned long long pol) {
+  int v;
+  asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.s32 %0, [%1], %2;" : "=r"(v) : "l"(a), "l"(pol));
+  return v;
+}
+
+// The resident form: one block of RT threads per SM, a contiguous range of slices per block, R slices per
+// warp, everything a row needs in registers. Two warps per scheduler keep the FP64 pipe busy (a dependent
+// FMA can issue as soon as the pipe is free), and each warp more would add its 32 values to every block sum.
+constexpr int RT = 256;
+constexpr int RMAX = 16;
+
+template <int R>
+__global__ void __launch_bounds__(RT, 1) k_pcg_resident(const __grid_constant__ PcgArgs a) {
+  __shared__ PcgShared<RT> sh;
+  __shared__ int s_off[RT / 32 * R + 1];
+  extern __shared__ __align__(16) unsigned char pcg_smem[];
+  double* const mv = reinterpret_cast<double*>(pcg_smem);
+  int* const mc = reinterpret_cast<int*>(mv + a.cap);
+  constexpr int CH = R <= 8 ? 16 : 9;  // entries in flight per row, as the registers allow
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (entry_flag(&a.st->converged)) return;
+  const int s0 = int((long long)a.nslices * blockIdx.x / gridDim.x);
+  const int ns = int((long long)a.nslices * (blockIdx.x + 1) / gridDim.x) - s0;
+  const int warps = min(ns, RT / 32);  // that have rows
+  if (threadIdx.x == 0) {
+    sh.fault = 0;
+    sh.k.load(a.st);
+  }
+  // shared-memory offsets of the block's slices, in order (one warp scans)
+  for (int k = threadIdx.x; k < RT / 32 * R; k += RT) s_off[k + 1] = k < ns ? a.width[s0 + k] * 32 : 0;
+  if (threadIdx.x == 0) s_off[0] = 0;
+  __syncthreads();
+  if (warp == 0) {
+    int run = 0;
+    for (int k0 = 0; k0 < RT / 32 * R; k0 += 32) {
+      int e = k0 + lane < RT / 32 * R ? s_off[k0 + lane + 1] : 0;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, e, o);
+        if (lane >= o) e += up;
+      }
+      e += run;
+      if (k0 + lane < RT / 32 * R) s_off[k0 + lane + 1] = e;
+      run = __shfl_sync(0xffffffffu, e, 31);
+    }
+  }
+  __syncthreads();
+  const unsigned long long pol = matrix_policy(a.stream);
+  double x[R], r[R], p[R], d[R];
+#pragma unroll
+  for (int k = 0; k < R; ++k) {
+    const int ls = warp + RT / 32 * k;
+    const int row = (s0 + ls) * 32 + lane;
+    const bool in = ls < ns && row < a.n;
+    x[k] = in ? a.x[row] : 0.0;
+    r[k] = in ? a.r[row] : 0.0;
+    p[k] = in ? a.p[row] : 0.0;
+    d[k] = in ? __ldg(a.dinv + row) : 0.0;
+    if (ls < ns && s_off[ls + 1] <= a.cap) {
+      const int off = s_off[ls] + lane, w = (s_off[ls + 1] - s_off[ls]) >> 5, src = __ldg(&a.meta[s0 + ls].x) + lane;
+      for (int t = 0; t < w; ++t) {
+        mv[off + 32 * t] = __ldg(a.val + src + 32 * t);
+        mc[off + 32 * t] = __ldg(a.col + src + 32 * t);
+      }
+    }
+  }
+  unsigned int epoch = 0;
+  while (true) {
+    double q[R];
+    double v3[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const int ls = warp + RT / 32 * i;
+      const int off = s_off[ls], w = (s_off[ls + 1] - off) >> 5;  // 0 for a slice the block does not have
+      if (s_off[ls + 1] <= a.cap) {
+        const double* sv = mv + off + lane;
+        const int* sc = mc + off + lane;
+        q[i] = pcg_row<CH>(w, a.p, [&](int t) { return sv[32 * t]; }, [&](int t) { return sc[32 * t]; });
+      } else {
+        const int src = __ldg(&a.meta[s0 + ls].x) + lane;
+        const double* gv = a.val + src;
+        const int* gc = a.col + src;
+        q[i] = pcg_row<CH>(w, a.p, [&](int t) { return ld_matrix(gv + 32 * t, pol); },
+                           [&](int t) { return ld_matrix(gc + 32 * t, pol); });
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+      if (warp + RT / 32 * i < ns) {  // warp-uniform
+        const double dq = d[i] * q[i];
+        v3[0] = fma(p[i], q[i], v3[0]);
+        v3[1] = fma(r[i], dq, v3[1]);
+        v3[2] = fma(q[i], dq, v3[2]);
+      }
+    if (!pcg_step(a, epoch, v3, warps, sh)) break;
+    const double alpha = sh.k.alpha, beta = sh.k.beta;
+    double v[2] = {0.0, 0.0};
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const int ls = warp + RT / 32 * i;
+      if (ls < ns) {
+        const int row = (s0 + ls) * 32 + lane;
+        x[i] = fma(alpha, p[i], x[i]);
+        r[i] = fma(-alpha, q[i], r[i]);
+        const double z = d[i] * r[i];
+        p[i] = fma(beta, p[i], z);
+        if (row < a.n) a.p[row] = p[i];
+        v[0] = fma(r[i], z, v[0]);
+        v[1] = fma(r[i], r[i], v[1]);
+      }
+    }
+    pcg_publish(a, epoch, v, warps, sh);
+  }
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const int ls = warp + RT / 32 * i;
+    const int row = (s0 + ls) * 32 + lane;
+    if (ls < ns && row < a.n) a.x[row] = x[i];
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) sh.k.store(a.st);
+}
+
+// The streaming form, for systems whose rows do not fit the registers of the grid: the same iteration with the
+// vectors in memory (each block the same contiguous rows in both passes).
+constexpr int PT = 1024;  // threads per block (one block per SM)
+
+__global__ void __launch_bounds__(PT, 1) k_pcg_stream(const __grid_constant__ PcgArgs a) {
+  __shared__ PcgShared<PT> sh;
+  if (entry_flag(&a.st->converged)) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int s0 = int((long long)a.nslices * blockIdx.x / gridDim.x);
+  const int s1 = int((long long)a.nslices * (blockIdx.x + 1) / gridDim.x);
+  const int row1 = min(a.n, s1 * 32);
+  const unsigned long long pol = matrix_policy(a.stream);
+  if (threadIdx.x == 0) {
+    sh.fault = 0;
+    sh.k.load(a.st);
+  }
+  unsigned int epoch = 0;
+  while (true) {
+    double v3[3] = {0.0, 0.0, 0.0};
+    for (int slice = s0 + warp; slice < s1; slice += PT / 32) {
+      const int row = slice * 32 + lane;
+      const bool in = row < a.n;
+      const double pr = in ? a.p[row] : 0.0, rr = in ? a.r[row] : 0.0, dr = in ? __ldg(a.dinv + row) : 0.0;
+      const int src = __ldg(&a.meta[slice].x) + lane, w = __ldg(a.width + slice);
+      const double* gv = a.val + src;
+      const int* gc = a.col + src;
+      double s = 0.0;
+#pragma unroll 1
+      for (int t0 = 0; t0 < w; t0 += 9) {
+        double vv[9];
+        int cc[9];
+#pragma unroll
+        for (int j = 0; j < 9; ++j) {
+          const bool on = t0 + j < w;  // warp-uniform
+          vv[j] = on ? ld_matrix(gv + 32 * (t0 + j), pol) : 0.0;
+          cc[j] = on ? ld_matrix(gc + 32 * (t0 + j), pol) : 0;
+        }
+#pragma unroll
+        for (int j = 0; j < 9; ++j)
+          if (t0 + j < w) s = fma(vv[j], a.p[cc[j]], s);
+      }
+      if (in) a.q[row] = s;
+      const double ds = dr * s;
+      v3[0] = fma(pr, s, v3[0]);
+      v3[1] = fma(rr, ds, v3[1]);
+      v3[2] = fma(s, ds, v3[2]);
+    }
+    if (!pcg_step(a, epoch, v3, PT / 32, sh)) break;
+    const double alpha = sh.k.alpha, beta = sh.k.beta;
+    double v[2] = {0.0, 0.0};
+    // (two rows per thread and pass, all their loads issued before the first store)
+    for (int i0 = s0 * 32 + threadIdx.x; i0 < row1; i0 += 2 * PT) {
+      double pv[2], qv[2], xv[2], rv[2], dv[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int i = i0 + u * PT;
+        const bool in = i < row1;
+        pv[u] = in ? a.p[i] : 0.0;
+        qv[u] = in ? a.q[i] : 0.0;
+        xv[u] = in ? a.x[i] : 0.0;
+        rv[u] = in ? a.r[i] : 0.0;
+        dv[u] = in ? __ldg(a.dinv + i) : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int i = i0 + u * PT;
+        if (i < row1) {
+          a.x[i] = fma(alpha, pv[u], xv[u]);
+          const double ri = fma(-alpha, qv[u], rv[u]);
+          const double zi = dv[u] * ri;
+          a.r[i] = ri;
+          a.p[i] = fma(beta, pv[u], zi);
+          v[0] = fma(ri, zi, v[0]);
+          v[1] = fma(ri, ri, v[1]);
+        }
+      }
+    }
+    pcg_publish(a, epoch, v, PT / 32, sh);
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) sh.k.store(a.st);
+}
+
+// Rows of at most 32 entries (the SELL-32 SpMV's limit). Per iteration, before (three counter barriers, shuffle
+// reductions, scalars in every thread) and now: 4,225 rows of Q1 squares 25.5 and 5.6 us; 68,921 of an
+// unstructured tetrahedral mesh 31.2 and 9.6; 98,304 of SWIPDG 26.0 and 9.9; 155,480 of P1 tetrahedra 29.7
+// and 11.5; 2,146,689 of 128^3 Q1 (streaming, 727.7 MB of matrix) 209 and 179. The graph form takes
+// 51.7 us for 393,216 rows of SWIPDG and 264 us for 128^3: AUTO takes this form wherever it applies.
 bool persistent_applies(gdt_context ctx, gdt_matrix m) {
   if (ctx->timing || ctx->solver_launch == GDT_SOLVER_LAUNCH_GRAPH) return false;
   return m->max_row >= 1 && m->max_row <= 32 && m->rows >= 1;
@@ -838,30 +1125,52 @@ bool persistent_applies(gdt_context ctx, gdt_matrix m) {
 // Runs the iterations after residual_init; the caller reads the final state from st. Returns
 // GDT_EUNSUPPORTED, before anything ran, where no cooperative launch of the kernel can be made
 // (the caller then runs the graph form).
-gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, double* p, double* q, double* z,
+gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, double* p, double* q, int* width,
                           const double* dinv, KState* st, cudaStream_t s) {
-  const void* fn = reinterpret_cast<const void*>(&k_pcg_persistent);
-  int dev = 0, coop = 0, per_sm = 0;
+  int dev = 0, coop = 0, per_sm = 0, optin = 0;
   GDT_TRY_CUDA(ctx, cudaGetDevice(&dev));
   GDT_TRY_CUDA(ctx, cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+  GDT_TRY_CUDA(ctx, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   if (!coop) return GDT_EUNSUPPORTED;  // the caller runs the graph form
-  GDT_TRY_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, PT, 0));
-  if (per_sm < 1) return GDT_EUNSUPPORTED;
-  int blocks = ctx->num_sms;  // one block per SM
+  int blocks = std::min(ctx->num_sms, RT);  // one block per SM
   if (ctx->persistent_blocks > 0) blocks = std::min(blocks, ctx->persistent_blocks);
-  // no more blocks than warps have slices
   const int nslices = int((m->rows + 31) / 32);
-  const int needed = (nslices + PT / 32 - 1) / (PT / 32);
-  if (needed < blocks) blocks = std::max(1, needed);
+  // four slices, one per scheduler, before the next block: 4,225 rows in 34 blocks of four warps take 5.6 us
+  // an iteration, in 133 blocks of one warp 6.0 us
+  blocks = std::max(1, std::min(blocks, (nslices + 3) / 4));
+  // slices per warp of the resident form; where a block has more rows than its registers hold, the
+  // streaming form
+  const int per_warp = ((nslices + blocks - 1) / blocks + RT / 32 - 1) / (RT / 32);
+  const void* fn = per_warp <= 1   ? reinterpret_cast<const void*>(&k_pcg_resident<1>)
+                   : per_warp <= 2 ? reinterpret_cast<const void*>(&k_pcg_resident<2>)
+                   : per_warp <= 4 ? reinterpret_cast<const void*>(&k_pcg_resident<4>)
+                   : per_warp <= 8 ? reinterpret_cast<const void*>(&k_pcg_resident<8>)
+                   : per_warp <= RMAX ? reinterpret_cast<const void*>(&k_pcg_resident<RMAX>)
+                                      : reinterpret_cast<const void*>(&k_pcg_stream);
+  const int threads = per_warp <= RMAX ? RT : PT;
+  int cap = 0;
+  size_t dyn = 0;
+  if (per_warp <= RMAX) {
+    cudaFuncAttributes fa;
+    GDT_TRY_CUDA(ctx, cudaFuncGetAttributes(&fa, fn));
+    const long long want = 32LL * m->max_row * ((nslices + blocks - 1) / blocks);
+    const long long room = (optin - (long long)fa.sharedSizeBytes) / 12 / 32 * 32;
+    cap = int(std::max(0LL, std::min(want, room)));
+    dyn = size_t(cap) * 12;
+    GDT_TRY_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(dyn)));
+  }
+  GDT_TRY_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, dyn));
+  if (per_sm < 1) return GDT_EUNSUPPORTED;
   {
     // the values are copied at every solve: the caller may have written them through the CSR pointer
-    const gdt_status ss = sell_prepare(ctx, m, s, true);
+    const gdt_status ss = sell_prepare_nonzero(ctx, m, s, width);
     if (ss != GDT_OK) return ss;
   }
   PcgArgs a;
   a.n = int(m->rows);
   a.nslices = nslices;
   a.meta = reinterpret_cast<const int2*>(m->sell_meta);
+  a.width = width;
   a.col = m->sell_col;
   a.val = m->sell_val;
   a.dinv = dinv;
@@ -869,18 +1178,19 @@ gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, d
   a.r = r;
   a.p = p;
   a.q = q;
-  a.z = z;
   a.st = st;
-  a.part = ctx->scratch;
-  // the barrier words live in the upper half of the scratch (the partials use its start)
-  a.bar = reinterpret_cast<unsigned int*>(ctx->scratch + kScratchDoubles / 2);
+  // packets and fault flag in the upper half of the scratch (kernels of the setup use its start)
+  unsigned long long* const words = reinterpret_cast<unsigned long long*>(ctx->scratch + kScratchDoubles / 2);
+  const size_t packets = size_t(2 * kSlot) * blocks;  // two buffers
+  if (packets + 16 > kScratchDoubles / 2) return fail(ctx, GDT_EUNSUPPORTED, "persistent solver: grid too large");
+  a.slots = words + 16;
+  a.fault = reinterpret_cast<unsigned int*>(words);
   a.wait_ns = ctx->persistent_wait_ns > 0 ? (unsigned long long)ctx->persistent_wait_ns : kBarrierNs;
-  if (3 * blocks > kScratchDoubles / 2) return fail(ctx, GDT_EUNSUPPORTED, "persistent solver: grid too large");
-  GDT_TRY_CUDA(ctx, cudaMemsetAsync(a.bar, 0, sizeof(unsigned long long), s));
-  GDT_TRY_CUDA(ctx, cudaMemsetAsync(a.bar + kBarGen, 0, sizeof(unsigned int), s));
-  GDT_TRY_CUDA(ctx, cudaMemsetAsync(a.bar + kBarFault, 0, sizeof(unsigned int), s));
+  a.cap = cap;
+  a.stream = 12LL * m->sell_len > (64LL << 20);
+  GDT_TRY_CUDA(ctx, cudaMemsetAsync(words, 0, sizeof(unsigned long long) * (packets + 16), s));
   void* args[] = {&a};
-  const cudaError_t le = cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(PT), args, 0, s);
+  const cudaError_t le = cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(threads), args, dyn, s);
   if (le == cudaErrorCooperativeLaunchTooLarge) {  // fewer SMs available than the device has
     cudaGetLastError();
     return GDT_EUNSUPPORTED;
@@ -888,7 +1198,7 @@ gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, d
   GDT_TRY_CUDA(ctx, le);
   ctx->launches++;
   unsigned int fault = 0;
-  GDT_TRY_CUDA(ctx, cudaMemcpyAsync(&fault, a.bar + kBarFault, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
+  GDT_TRY_CUDA(ctx, cudaMemcpyAsync(&fault, a.fault, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
   GDT_TRY_CUDA(ctx, cudaStreamSynchronize(s));
   if (fault) return fail(ctx, GDT_ECUDA, "persistent solver: a grid barrier wait ran out");
   return GDT_OK;
@@ -1086,9 +1396,9 @@ gdt_status solve(gdt_context ctx, gdt_matrix m, const double* b, double* x, cons
         bool persistent = persistent_applies(ctx, m);
         if (persistent) {
           residual_init<double>(L, m->rp, m->col, m->val, x, b, r, one, p, st);
-          double* z = (double*)alloc(vb);
-          if (!z) return fail(ctx, GDT_ENOMEM, "solver vectors");
-          const gdt_status ps = pcg_persistent(ctx, m, x, r, p, q, z, one, st, s);
+          int* width = (int*)alloc(sizeof(int) * ((n + 31) / 32));
+          if (!width) return fail(ctx, GDT_ENOMEM, "solver vectors");
+          const gdt_status ps = pcg_persistent(ctx, m, x, r, p, q, width, one, st, s);
           if (ps == GDT_EUNSUPPORTED) persistent = false;  // x untouched: the graph form starts afresh
           else if (ps != GDT_OK) return ps;
           else ctx->last_solver_launch = GDT_SOLVER_LAUNCH_PERSISTENT;

@@ -68,6 +68,34 @@ __global__ void k_sell_fill(int n, int nslices, const int* __restrict__ rp, cons
   }
 }
 
+// the same with the zero values left out: width[slice] = the most nonzeros of a row of the slice; a row's
+// entries beyond its own nonzeros (and beyond width) are padding, those beyond width are not written
+__global__ void k_sell_fill_nonzero(int n, int nslices, const int* __restrict__ rp, const int* __restrict__ col,
+                                    const double* __restrict__ val, const int2* __restrict__ meta,
+                                    int* __restrict__ scol, double* __restrict__ sval, int* __restrict__ width) {
+  const int slice = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (slice >= nslices) return;
+  const int lane = threadIdx.x & 31;
+  const int row = slice * 32 + lane;
+  const long long base = (long long)meta[slice].x + lane;
+  const int beg = row < n ? rp[row] : 0, end = row < n ? rp[row + 1] : 0;
+  int t = 0;
+  for (int k = beg; k < end; ++k) {
+    const double v = val[k];
+    if (v != 0.0) {
+      scol[base + 32LL * t] = col[k];
+      sval[base + 32LL * t] = v;
+      ++t;
+    }
+  }
+  const int w = __reduce_max_sync(0xffffffffu, t);
+  for (; t < w; ++t) {
+    scol[base + 32LL * t] = row < n ? row : 0;
+    sval[base + 32LL * t] = 0.0;
+  }
+  if (lane == 0) width[slice] = w;
+}
+
 void sell_free(gdt_matrix m) {
   if (m->sell_meta) cudaFree(m->sell_meta);
   if (m->sell_col) cudaFree(m->sell_col);
@@ -78,7 +106,8 @@ void sell_free(gdt_matrix m) {
   m->sell_version = -1;
 }
 
-gdt_status sell_prepare(gdt_context ctx, gdt_matrix m, cudaStream_t s, bool refill) {
+// the slice table of the pattern and room for the copy (its values are filled by the callers below)
+static gdt_status sell_table(gdt_context ctx, gdt_matrix m, cudaStream_t s) {
   const int n = int(m->rows);
   const int nslices = (n + 31) / 32;
   const int blocks = (nslices * 32 + 255) / 256;
@@ -124,13 +153,30 @@ gdt_status sell_prepare(gdt_context ctx, gdt_matrix m, cudaStream_t s, bool refi
     m->sell_len = off;
     m->sell_version = -1;
   }
+  return GDT_OK;
+}
+
+gdt_status sell_prepare(gdt_context ctx, gdt_matrix m, cudaStream_t s, bool refill) {
+  const gdt_status st = sell_table(ctx, m, s);
+  if (st != GDT_OK) return st;
   if (refill || m->sell_version != m->val_version) {
-    k_sell_fill<<<blocks, 256, 0, s>>>(n, nslices, m->rp, m->col, m->val, reinterpret_cast<const int2*>(m->sell_meta),
-                                       m->sell_col, m->sell_val);
+    const int n = int(m->rows), nslices = (n + 31) / 32;
+    k_sell_fill<<<(nslices * 32 + 255) / 256, 256, 0, s>>>(
+        n, nslices, m->rp, m->col, m->val, reinterpret_cast<const int2*>(m->sell_meta), m->sell_col, m->sell_val);
     m->sell_version = m->val_version;
     return check_launch(ctx, "sell fill");
   }
   return GDT_OK;
+}
+
+gdt_status sell_prepare_nonzero(gdt_context ctx, gdt_matrix m, cudaStream_t s, int* width) {
+  const gdt_status st = sell_table(ctx, m, s);
+  if (st != GDT_OK) return st;
+  const int n = int(m->rows), nslices = (n + 31) / 32;
+  m->sell_version = -1;  // not the full copy: the next reader of that one refills it
+  k_sell_fill_nonzero<<<(nslices * 32 + 255) / 256, 256, 0, s>>>(
+      n, nslices, m->rp, m->col, m->val, reinterpret_cast<const int2*>(m->sell_meta), m->sell_col, m->sell_val, width);
+  return check_launch(ctx, "sell fill");
 }
 
 SellView sell_view(gdt_matrix m) {
