@@ -1230,7 +1230,8 @@ class BatchedDiffusion:
     the squares split into two triangles (element="p1", element e = 2 cell + t) or continuous Q1 on
     the squares (element="q1", element e = cell), homogeneous Dirichlet. kappa per quadrant of the
     2 x 2 split (`mu`, [n, 4]) or per element (`kappa`, concatenated at `element_offsets`).
-    Each problem is solved by a team of threads: the 8 CTAs of a cluster, one CTA or one warp;
+    Each problem is solved by a team of threads: several CTAs ("cluster"; in FP64 as many as the work
+    asks for), one CTA or one warp;
     `tune()` times the team kinds per size class and keeps the fastest (the autotuner),
     `set_teams()` sets them by hand."""
 

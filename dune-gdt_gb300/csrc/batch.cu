@@ -6,8 +6,13 @@
 // single-problem path) and solved with CG + Jacobi inside ONE persistent launch (captured in a CUDA
 // graph and replayed).
 //
-// GB300 design. The grid is a set of 8-CTA thread-block clusters that pull work items from a queue,
-// largest problems first (one atomic per item). An item is solved by teams of one of three sizes:
+// GB300 design. In FP64, problems of the default team kind ("cluster") run in batch_team_kernel
+// (batch_team.cuh): one block per SM, the SMs divided into teams sized by the work. 64 problems of 64, 128,
+// 256 and 512 squares take 245 ms there and 990 ms in the kernel below, whose 8-CTA clusters leave most
+// SMs idle behind the 16 largest problems. The kernel below runs the other team kinds, mixed
+// precision, and everything where no cooperative launch can be made. Its grid is a set of 8-CTA
+// thread-block clusters that pull work items from a queue, largest problems first (one atomic per
+// item). An item is solved by teams of one of three sizes:
 //   cluster: the 8 CTAs of the cluster share one problem (rows split into 8 chunks); reductions end
 //            with a hardware cluster barrier and a read of the 8 CTA partials through distributed
 //            shared memory, summed in rank order by every CTA (deterministic);
@@ -27,8 +32,9 @@
 //
 // Failure handling (per problem, the others are unaffected): non-finite data (kappa or the load) is
 // detected after assembly by a team reduction, the problem is skipped with x = 0 and reported as
-// GDT_ENAN; a problem that reaches max_iter is reported as GDT_ENOCONV. The iteration count is the
-// only budget: the kernel has no wait that could run out.
+// GDT_ENAN; a problem that reaches max_iter is reported as GDT_ENOCONV. The fixed-size team kernel has no wait
+// that could run out; those of batch_team_kernel are bounded (as the persistent solvers'), and one that
+// runs out ends the launch with GDT_ETIMEOUT for the problems not solved and GDT_ECUDA from the call.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -38,7 +44,7 @@
 #include <numeric>
 #include <vector>
 
-#include "structured.cuh"
+#include "batch_team.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -52,6 +58,14 @@ struct BatchItem {
   int pad;
   long long stride;
 };
+
+// division of the blocks of batch_team_kernel into teams, and of the problems into the two lists
+struct TeamPlan {
+  std::vector<TeamPlace> places;
+  std::vector<int> probs;
+  int count[2] = {0, 0};
+  long long words = 0;  // scratch of all teams
+};
 }  // namespace gdt
 
 struct gdt_batch_s {
@@ -59,13 +73,23 @@ struct gdt_batch_s {
   int element = GDT_BATCH_P1_SIMPLEX;
   std::vector<long long> cells, offsets, eoffsets;
   std::vector<int> teams;                // per problem: GDT_BATCH_TEAM_*
-  std::vector<gdt::BatchItem> items;     // the queue of the current team assignment
-  std::vector<int> probs;
+  // the queue of the current team assignment, for the fixed-size team kernel: every problem (mixed
+  // precision), and those that do not run in team_kernel (FP64)
+  std::vector<gdt::BatchItem> items, items_rest;
+  std::vector<int> probs, probs_rest;
+  gdt::TeamPlan plan;                    // of the problems that run in batch_team_kernel
   long long* d_off = nullptr;
   long long* d_eoff = nullptr;
   int* d_cells = nullptr;
-  gdt::BatchItem* d_items = nullptr;     // room for nprob items
+  gdt::BatchItem* d_items = nullptr;     // room for nprob items of each of the two queues
   int* d_probs = nullptr;
+  gdt::TeamPlace* d_place = nullptr;
+  int* d_tprobs = nullptr;
+  unsigned long long* d_exchange = nullptr;  // fault flag, list counters, packets
+  double* team_scratch = nullptr;
+  long long team_words = 0;
+  int team_blocks = 0;                   // blocks of the cooperative launch (0: none can be made)
+  int team_smem = 0;                     // its dynamic shared memory in doubles
   int* d_queue = nullptr;
   int* d_iters = nullptr;
   double* d_relres = nullptr;
@@ -649,6 +673,101 @@ long long build_items(const gdt_batch_s& b, std::vector<int> subset, std::vector
   return need;
 }
 
+// Teams for the problems `subset` on `blocks` blocks: k0 teams of s0 blocks that start with the larger problems
+// and k1 teams of s1 blocks for the others, the division with the shortest estimated run (every team
+// taking the largest problem left on its list when it is free). The estimate of an iteration is the FP64
+// work of a block's rows (12 or 16 instructions of 31 ns per warp and scheduler) plus its two exchanges
+// (1.5 us within a block, 4.5 us between blocks); iterations grow with the cells per side.
+// Large teams pay their exchanges on every problem, small ones leave SMs idle behind a large problem:
+// 16 problems each of 64, 128, 256 and 512 squares run on 19 teams of 8.
+TeamPlan plan_teams(const gdt_batch_s& b, std::vector<int> subset, int blocks, long long most_words) {
+  TeamPlan plan;
+  std::stable_sort(subset.begin(), subset.end(), [&](int x, int y) { return b.cells[x] > b.cells[y]; });
+  const int np = int(subset.size());
+  const int arrays = b.element == GDT_BATCH_Q1_CUBE ? team_arrays<9>() : team_arrays<7>();
+  const double ops = b.element == GDT_BATCH_Q1_CUBE ? 16.0 : 12.0;
+  auto cost = [&](int prob, int s) {
+    const double n = double(b.cells[prob]);
+    return 4.0 * n * ((n + 1) * (n + 1) / s / 128.0 * ops * 31e-3 + (s == 1 ? 1.5 : 4.5));
+  };
+  auto words = [&](int prob) { return arrays * team_stride(b.cells[prob]); };
+  // list lengths to try: the ends of the size classes
+  std::vector<int> ends;
+  for (int i = 1; i <= np; ++i)
+    if (i == np || b.cells[subset[i]] != b.cells[subset[i - 1]]) ends.push_back(i);
+  while (ends.size() > 5) {
+    std::vector<int> half;
+    for (size_t i = 1; i < ends.size(); i += 2) half.push_back(ends[i]);
+    if (half.back() != np) half.push_back(np);
+    ends = half;
+  }
+  std::vector<int> sizes;
+  for (int s : {1, 2, 3, 4, 5, 6, 8, 10, 12, 16, 19, 25, 38, 50, 76})
+    if (s < blocks) sizes.push_back(s);
+  sizes.push_back(blocks);
+  double best = -1.0;
+  int bs0 = blocks, bk0 = 1, bs1 = 0, bk1 = 0, bm = np;
+  auto consider = [&](int s0, int k0, int s1, int k1, int m) {
+    const long long need = k0 * words(subset[0]) + (k1 && m < np ? k1 * words(subset[m]) : 0);
+    if (need > most_words && !(k0 == 1 && k1 == 0)) return;
+    // finish times of the teams as heaps, each problem to the team that is free first
+    std::vector<std::pair<double, int>> t;  // (free at, -list): ties go to the teams of list 0
+    auto later = [](const std::pair<double, int>& x, const std::pair<double, int>& y) { return x > y; };
+    for (int i = 0; i < k0; ++i) t.push_back({0.0, 0});
+    for (int i = 0; i < k1; ++i) t.push_back({0.0, 1});
+    int next[2] = {0, m};
+    double end = 0.0;
+    while (!t.empty()) {
+      std::pop_heap(t.begin(), t.end(), later);
+      auto& team = t.back();
+      const int list = team.second == 0 && next[0] < m ? 0 : 1;
+      if (next[list] >= (list == 0 ? m : np)) {
+        end = std::max(end, team.first);
+        t.pop_back();
+        continue;
+      }
+      team.first += cost(subset[next[list]++], team.second == 0 ? s0 : s1);
+      if (best >= 0.0 && team.first >= best) return;
+      std::push_heap(t.begin(), t.end(), later);
+    }
+    if (best < 0.0 || end < best) {
+      best = end;
+      bs0 = s0, bk0 = k0, bs1 = s1, bk1 = k1, bm = m;
+    }
+  };
+  if (np <= 4096) {
+    for (size_t i = sizes.size(); i-- > 0;) consider(sizes[i], std::min(np, blocks / sizes[i]), 0, 0, np);
+    if (np <= 1024)
+      for (int s0 : sizes)
+        for (int m : ends) {
+          const int k0 = std::min(m, blocks / s0);
+          if (m < np)
+            for (int s1 : sizes)
+              if (s1 <= s0 && blocks - k0 * s0 >= s1) consider(s0, k0, s1, std::min(np - m, (blocks - k0 * s0) / s1), m);
+        }
+  } else {  // enough problems to keep every block busy with its own, as far as the memory goes
+    for (size_t i = sizes.size(); i-- > 0;)
+      if (blocks / sizes[i] * words(subset[0]) <= most_words) bs0 = sizes[i], bk0 = blocks / sizes[i];
+  }
+  plan.count[0] = bm;
+  plan.count[1] = np - bm;
+  plan.probs = subset;
+  long long off = 0;
+  for (int i = 0; i < bk0 + bk1; ++i) {
+    const int size = i < bk0 ? bs0 : bs1;
+    TeamPlace pl;
+    pl.first = int(plan.places.size());
+    pl.count = size;
+    pl.list = i < bk0 ? 0 : 1;
+    pl.pad = 0;
+    pl.scratch = off;
+    for (int j = 0; j < size; ++j) plan.places.push_back(pl);
+    off += i < bk0 ? words(subset[0]) : words(subset[bm]);
+  }
+  plan.words = off;
+  return plan;
+}
+
 gdt_status ensure_scratch(gdt_context ctx, gdt_batch b, long long words) {
   if (words <= b->scratch_words) return GDT_OK;
   cudaFree(b->scratch64);
@@ -666,17 +785,63 @@ gdt_status ensure_scratch(gdt_context ctx, gdt_batch b, long long words) {
   return GDT_OK;
 }
 
-// the queue of the whole batch under the current team assignment, on the device
+// words of the fixed-size team kernel's scratch per cluster for `items`, problems in `probs`
+long long words_of(const gdt_batch_s& b, const std::vector<BatchItem>& items) {
+  const long long words = stencil_of(b.element) + 5;
+  long long need = 0;
+  for (const BatchItem& it : items) need = std::max(need, it.count * words * it.stride);
+  return need;
+}
+
+// plan and lists of the problems `subset` for batch_team_kernel, on the device
+gdt_status upload_plan(gdt_context ctx, gdt_batch b, const std::vector<int>& subset) {
+  b->plan = TeamPlan();
+  if (subset.empty()) return GDT_OK;
+  // no more memory than the clusters of the fixed-size team kernel would take (in 8-byte words)
+  std::vector<BatchItem> items;
+  std::vector<int> probs;
+  const std::vector<int> saved = b->teams;
+  for (int p : subset) b->teams[p] = GDT_BATCH_TEAM_CLUSTER;
+  const long long most = build_items(*b, subset, items, probs) * b->nclusters / 2 * 3;
+  b->teams = saved;
+  b->plan = plan_teams(*b, subset, b->team_blocks, most);
+  if (b->plan.words > b->team_words) {
+    cudaFree(b->team_scratch);
+    b->team_scratch = nullptr;
+    b->team_words = 0;
+    const cudaError_t e = cudaMalloc(&b->team_scratch, sizeof(double) * b->plan.words);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      return fail(ctx, e == cudaErrorMemoryAllocation ? GDT_ENOMEM : GDT_ECUDA, "batch scratch");
+    }
+    b->team_words = b->plan.words;
+  }
+  GDT_TRY_CUDA(ctx, cudaMemcpy(b->d_place, b->plan.places.data(), sizeof(TeamPlace) * b->plan.places.size(),
+                               cudaMemcpyHostToDevice));
+  GDT_TRY_CUDA(ctx, cudaMemcpy(b->d_tprobs, b->plan.probs.data(), sizeof(int) * b->plan.probs.size(),
+                               cudaMemcpyHostToDevice));
+  return GDT_OK;
+}
+
+// the queues of the whole batch under the current team assignment, on the device
 gdt_status upload_queue(gdt_context ctx, gdt_batch b) {
   // a launch in flight on the context stream may still read the old queue and scratch
   if (ctx->stream) GDT_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  std::vector<int> all(b->nprob);
+  std::vector<int> all(b->nprob), team, rest;
   std::iota(all.begin(), all.end(), 0);
-  const long long need = build_items(*b, all, b->items, b->probs);
+  for (int p : all) (b->team_blocks > 0 && b->teams[p] == GDT_BATCH_TEAM_CLUSTER ? team : rest).push_back(p);
+  build_items(*b, all, b->items, b->probs);
+  build_items(*b, rest, b->items_rest, b->probs_rest);
   GDT_TRY_CUDA(ctx, cudaMemcpy(b->d_items, b->items.data(), sizeof(BatchItem) * b->items.size(), cudaMemcpyHostToDevice));
   GDT_TRY_CUDA(ctx, cudaMemcpy(b->d_probs, b->probs.data(), sizeof(int) * b->probs.size(), cudaMemcpyHostToDevice));
+  if (!rest.empty()) {
+    GDT_TRY_CUDA(ctx, cudaMemcpy(b->d_items + b->nprob, b->items_rest.data(), sizeof(BatchItem) * b->items_rest.size(),
+                                 cudaMemcpyHostToDevice));
+    GDT_TRY_CUDA(ctx, cudaMemcpy(b->d_probs + b->nprob, b->probs_rest.data(), sizeof(int) * b->probs_rest.size(),
+                                 cudaMemcpyHostToDevice));
+  }
   b->generation++;
-  return ensure_scratch(ctx, b, need);
+  return upload_plan(ctx, b, team);
 }
 
 // P1 stiffness of the two triangle types of a square cell and Q1 stiffness of a square (both scale
@@ -747,11 +912,12 @@ gdt_status check_solve_args(gdt_context ctx, gdt_batch b, const SolveArgs& s) {
   return GDT_OK;
 }
 
-BatchArgs make_args(gdt_batch b, const SolveArgs& s) {
+// arguments of the fixed-size team kernel for the queue of all problems or of those outside the plan
+BatchArgs make_args(gdt_batch b, const SolveArgs& s, bool all) {
   BatchArgs a;
-  a.nitems = int(b->items.size());
-  a.items = b->d_items;
-  a.probs = b->d_probs;
+  a.nitems = int((all ? b->items : b->items_rest).size());
+  a.items = b->d_items + (all ? 0 : b->nprob);
+  a.probs = b->d_probs + (all ? 0 : b->nprob);
   a.off = b->d_off;
   a.eoff = b->d_eoff;
   a.cells = b->d_cells;
@@ -774,16 +940,80 @@ BatchArgs make_args(gdt_batch b, const SolveArgs& s) {
   return a;
 }
 
-void launch(gdt_batch b, const BatchArgs& a, cudaStream_t s) {
-  cudaMemsetAsync(b->d_queue, 0, sizeof(int), s);
-  const dim3 grid(b->nclusters_prec[a.mixed ? 1 : 0] * CL);
-  if (b->element == GDT_BATCH_Q1_CUBE) {
-    if (a.mixed) batch_kernel<9, true><<<grid, BT, 0, s>>>(a);
-    else batch_kernel<9, false><<<grid, BT, 0, s>>>(a);
-  } else {
-    if (a.mixed) batch_kernel<7, true><<<grid, BT, 0, s>>>(a);
-    else batch_kernel<7, false><<<grid, BT, 0, s>>>(a);
+TeamBatchArgs make_team_args(gdt_context ctx, gdt_batch b, const SolveArgs& s) {
+  TeamBatchArgs a;
+  a.place = b->d_place;
+  a.probs = b->d_tprobs;
+  a.count[0] = b->plan.count[0];
+  a.count[1] = b->plan.count[1];
+  a.off = b->d_off;
+  a.eoff = b->d_eoff;
+  a.cells = b->d_cells;
+  a.kappa = s.kappa;
+  a.kappa_elems = s.kappa_kind == GDT_BATCH_KAPPA_ELEMENTS;
+  a.force = s.force;
+  a.tol2 = s.tol * s.tol;
+  a.max_iter = s.max_iter;
+  a.x = s.x;
+  a.stencil_out = s.stencil_out;
+  a.iters = b->d_iters;
+  a.relres = b->d_relres;
+  a.status = b->d_status;
+  a.scratch = b->team_scratch;
+  a.ex.fault = reinterpret_cast<unsigned int*>(b->d_exchange);
+  a.taken = reinterpret_cast<int*>(b->d_exchange + 1);
+  a.ex.slots = b->d_exchange + kSlot;
+  a.ex.wait_ns = ctx->persistent_wait_ns > 0 ? (unsigned long long)ctx->persistent_wait_ns : kBarrierNs;
+  a.ex.first = a.ex.count = 0;
+  a.smem_words = b->team_smem;
+  local_stiffness(b->element, a.K);
+  return a;
+}
+
+const void* team_kernel_of(int element) {
+  return element == GDT_BATCH_Q1_CUBE ? reinterpret_cast<const void*>(&batch_team_kernel<9>)
+                                      : reinterpret_cast<const void*>(&batch_team_kernel<7>);
+}
+
+// whether problems of the plan run in batch_team_kernel (the others, and all of them in mixed precision, in
+// the fixed-size team kernel)
+bool uses_plan(gdt_batch b, int precision) {
+  return precision == GDT_PRECISION_FP64 && !b->plan.places.empty();
+}
+
+gdt_status launch(gdt_context ctx, gdt_batch b, const SolveArgs& sa, cudaStream_t s) {
+  cudaError_t e = cudaSuccess;
+  const bool planned = uses_plan(b, sa.precision);
+  if (planned) {
+    TeamBatchArgs a = make_team_args(ctx, b, sa);
+    void* args[] = {&a};
+    const int blocks = int(b->plan.places.size());
+    e = cudaMemsetAsync(b->d_exchange, 0, sizeof(unsigned long long) * kSlot * (1 + 2 * size_t(blocks)), s);
+    if (e == cudaSuccess)
+      e = cudaLaunchCooperativeKernel(team_kernel_of(b->element), dim3(blocks), dim3(TB), args,
+                                      sizeof(double) * size_t(b->team_smem), s);
   }
+  if (e == cudaSuccess && (!planned || !b->items_rest.empty())) {
+    const BatchArgs a = make_args(b, sa, !planned);
+    e = cudaMemsetAsync(b->d_queue, 0, sizeof(int), s);
+    const dim3 grid(b->nclusters_prec[a.mixed ? 1 : 0] * CL);
+    if (b->element == GDT_BATCH_Q1_CUBE) {
+      if (a.mixed) batch_kernel<9, true><<<grid, BT, 0, s>>>(a);
+      else batch_kernel<9, false><<<grid, BT, 0, s>>>(a);
+    } else {
+      if (a.mixed) batch_kernel<7, true><<<grid, BT, 0, s>>>(a);
+      else batch_kernel<7, false><<<grid, BT, 0, s>>>(a);
+    }
+  }
+  if (e != cudaSuccess) return fail(ctx, GDT_ECUDA, std::string("batch launch: ") + cudaGetErrorString(e));
+  return GDT_OK;
+}
+
+// scratch of the fixed-size team kernel, where that kernel has something to do
+gdt_status prepare_scratch(gdt_context ctx, gdt_batch b, int precision) {
+  const bool planned = uses_plan(b, precision);
+  if (planned && b->items_rest.empty()) return GDT_OK;
+  return ensure_scratch(ctx, b, words_of(*b, planned ? b->items_rest : b->items));
 }
 
 // per-problem results of the last launch over `subset` into info; the status of the call
@@ -803,10 +1033,12 @@ gdt_status collect(gdt_context ctx, gdt_batch b, const std::vector<int>& subset,
   I.all_converged = 1;
   I.max_rel_residual = 0.0;
   I.nonfinite_problems = 0;
+  bool timed_out = false;
   for (int i : subset) {
     I.total_dofs += b->offsets[i + 1] - b->offsets[i];
     const int v = it[i] >= 0 ? it[i] : -it[i] - 1;
     if (stv[i] != GDT_OK) I.all_converged = 0;
+    timed_out = timed_out || stv[i] == GDT_ETIMEOUT;
     if (stv[i] == GDT_ENAN) {
       I.nonfinite_problems++;
       continue;
@@ -815,6 +1047,7 @@ gdt_status collect(gdt_context ctx, gdt_batch b, const std::vector<int>& subset,
     I.min_iterations = std::min(I.min_iterations, v);
     I.max_rel_residual = std::max(I.max_rel_residual, rr[i]);
   }
+  if (timed_out) return fail(ctx, GDT_ECUDA, "batch: a grid barrier wait ran out");
   if (I.nonfinite_problems) return fail(ctx, GDT_ENAN, "a batched problem has non-finite data (skipped, x = 0)");
   if (!I.all_converged) return fail(ctx, GDT_ENOCONV, "a batched problem did not converge");
   return GDT_OK;
@@ -823,7 +1056,8 @@ gdt_status collect(gdt_context ctx, gdt_batch b, const std::vector<int>& subset,
 gdt_status solve_impl(gdt_context ctx, gdt_batch b, const SolveArgs& sa, gdt_batch_info* info) {
   gdt_status st = check_solve_args(ctx, b, sa);
   if (st != GDT_OK) return st;
-  const BatchArgs a = make_args(b, sa);
+  st = prepare_scratch(ctx, b, sa.precision);
+  if (st != GDT_OK) return st;
   cudaStream_t s = ctx->stream;
   cudaStream_t own = nullptr;
   if (!s) {
@@ -836,20 +1070,21 @@ gdt_status solve_impl(gdt_context ctx, gdt_batch b, const SolveArgs& sa, gdt_bat
   key = mix(key, reinterpret_cast<unsigned long long>(sa.kappa));
   key = mix(key, reinterpret_cast<unsigned long long>(sa.x));
   key = mix(key, reinterpret_cast<unsigned long long>(sa.stencil_out));
-  key = mix(key, (unsigned long long)sa.kappa_kind * 7 + (unsigned long long)a.mixed);
+  key = mix(key, (unsigned long long)sa.kappa_kind * 7 + (unsigned long long)sa.precision);
   key = mix(key, std::hash<double>()(sa.force));
   key = mix(key, std::hash<double>()(sa.tol));
   key = mix(key, (unsigned long long)sa.max_iter);
   key = mix(key, b->generation);
   key = mix(key, reinterpret_cast<unsigned long long>(b->scratch64));
+  key = mix(key, (unsigned long long)ctx->persistent_wait_ns);
   if (!b->exec || b->key != key) {
     if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->graph) cudaGraphDestroy(b->graph);
     b->exec = nullptr;
     b->graph = nullptr;
     if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-      launch(b, a, s);
-      if (cudaStreamEndCapture(s, &b->graph) != cudaSuccess || cudaGraphInstantiate(&b->exec, b->graph, 0) != cudaSuccess)
+      const gdt_status ls = launch(ctx, b, sa, s);
+      if (cudaStreamEndCapture(s, &b->graph) != cudaSuccess || ls != GDT_OK || cudaGraphInstantiate(&b->exec, b->graph, 0) != cudaSuccess)
         b->exec = nullptr;
     }
     cudaGetLastError();
@@ -858,9 +1093,9 @@ gdt_status solve_impl(gdt_context ctx, gdt_batch b, const SolveArgs& sa, gdt_bat
   if (b->exec) {
     if (cudaGraphLaunch(b->exec, s) != cudaSuccess) st = fail(ctx, GDT_ECUDA, "batch graph launch");
   } else {
-    launch(b, a, s);
+    st = launch(ctx, b, sa, s);
   }
-  ctx->launches++;
+  ctx->launches += uses_plan(b, sa.precision) && !b->items_rest.empty() ? 2 : 1;
   if (st == GDT_OK) {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) st = fail(ctx, GDT_ECUDA, std::string("batch_kernel: ") + cudaGetErrorString(e));
@@ -930,8 +1165,28 @@ gdt_status gdt_batch_create_ex(gdt_context ctx, int64_t nproblems, const int64_t
   }
   b->nclusters = std::max(b->nclusters_prec[0], b->nclusters_prec[1]);
   std::vector<int> c32(b->cells.begin(), b->cells.end());
-  cudaError_t e = cudaMalloc(&b->d_items, sizeof(BatchItem) * nproblems);
-  if (e == cudaSuccess) e = cudaMalloc(&b->d_probs, sizeof(int) * nproblems);
+  {
+    // one block of batch_team_kernel per SM, where a cooperative launch of it can be made
+    const void* fn = team_kernel_of(element);
+    int coop = 0, optin = 0, per_sm = 0;
+    cudaFuncAttributes fa;
+    if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device) == cudaSuccess && coop &&
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device) == cudaSuccess &&
+        cudaFuncGetAttributes(&fa, fn) == cudaSuccess) {
+      b->team_smem = int((optin - (long long)fa.sharedSizeBytes) / 8);
+      if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, b->team_smem * 8) == cudaSuccess &&
+          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, TB, size_t(b->team_smem) * 8) == cudaSuccess &&
+          per_sm >= 1)
+        b->team_blocks = std::min(ctx->num_sms, TB);
+    }
+    if (ctx->persistent_blocks > 0) b->team_blocks = std::min(b->team_blocks, ctx->persistent_blocks);
+    cudaGetLastError();
+  }
+  cudaError_t e = cudaMalloc(&b->d_items, sizeof(BatchItem) * 2 * nproblems);
+  if (e == cudaSuccess) e = cudaMalloc(&b->d_probs, sizeof(int) * 2 * nproblems);
+  if (e == cudaSuccess) e = cudaMalloc(&b->d_place, sizeof(TeamPlace) * TB);
+  if (e == cudaSuccess) e = cudaMalloc(&b->d_tprobs, sizeof(int) * nproblems);
+  if (e == cudaSuccess) e = cudaMalloc(&b->d_exchange, sizeof(unsigned long long) * kSlot * (1 + 2 * TB));
   if (e == cudaSuccess) e = cudaMalloc(&b->d_off, sizeof(long long) * (nproblems + 1));
   if (e == cudaSuccess) e = cudaMalloc(&b->d_eoff, sizeof(long long) * (nproblems + 1));
   if (e == cudaSuccess) e = cudaMalloc(&b->d_cells, sizeof(int) * nproblems);
@@ -968,6 +1223,10 @@ gdt_status gdt_batch_destroy(gdt_batch b) {
   if (b->graph) cudaGraphDestroy(b->graph);
   cudaFree(b->d_items);
   cudaFree(b->d_probs);
+  cudaFree(b->d_place);
+  cudaFree(b->d_tprobs);
+  cudaFree(b->d_exchange);
+  cudaFree(b->team_scratch);
   cudaFree(b->d_off);
   cudaFree(b->d_eoff);
   cudaFree(b->d_cells);
@@ -1051,24 +1310,31 @@ gdt_status gdt_batch_tune(gdt_context ctx, gdt_batch b, const double* kappa, int
       double t_ms = -1.0;
       if (team != GDT_BATCH_TEAM_WARP || nd <= kWarpMaxDofs) {
         for (int i : cls.second) b->teams[i] = team;
-        std::vector<BatchItem> items;
-        std::vector<int> probs;
-        const long long need = build_items(*b, cls.second, items, probs);
-        st = ensure_scratch(ctx, b, need);
+        // the queue and plan of this class alone
+        if (cudaStreamSynchronize(s) != cudaSuccess) {
+          st = fail(ctx, GDT_ECUDA, "batch synchronize");
+          break;
+        }
+        const bool planned =
+            b->team_blocks > 0 && team == GDT_BATCH_TEAM_CLUSTER && precision == GDT_PRECISION_FP64;
+        st = upload_plan(ctx, b, planned ? cls.second : std::vector<int>());
         if (st != GDT_OK) break;
-        if (cudaMemcpyAsync(b->d_items, items.data(), sizeof(BatchItem) * items.size(), cudaMemcpyHostToDevice, s) !=
+        build_items(*b, cls.second, b->items, b->probs);
+        b->items_rest.clear();
+        st = prepare_scratch(ctx, b, precision);
+        if (st != GDT_OK) break;
+        if (cudaMemcpy(b->d_items, b->items.data(), sizeof(BatchItem) * b->items.size(), cudaMemcpyHostToDevice) !=
                 cudaSuccess ||
-            cudaMemcpyAsync(b->d_probs, probs.data(), sizeof(int) * probs.size(), cudaMemcpyHostToDevice, s) !=
+            cudaMemcpy(b->d_probs, b->probs.data(), sizeof(int) * b->probs.size(), cudaMemcpyHostToDevice) !=
                 cudaSuccess) {
           st = fail(ctx, GDT_ECUDA, "batch tune upload");
           break;
         }
-        BatchArgs a = make_args(b, sa);
-        a.nitems = int(items.size());
-        launch(b, a, s);  // warm-up (first use of the scratch, caches)
+        st = launch(ctx, b, sa, s);  // warm-up (first use of the scratch, caches)
         cudaEventRecord(e0, s);
-        launch(b, a, s);
+        if (st == GDT_OK) st = launch(ctx, b, sa, s);
         cudaEventRecord(e1, s);
+        if (st != GDT_OK) break;
         ctx->launches += 2;
         gdt_batch_info info;
         st = collect(ctx, b, cls.second, s, &info);

@@ -16,7 +16,7 @@
 #include <cmath>
 #include <vector>
 
-#include "linalg.cuh"
+#include "exchange.cuh"
 
 namespace gdt {
 
@@ -651,7 +651,8 @@ void ilu_apply(gdt_context ctx, gdt_matrix m, const Ilu& f, const double* r, dou
 //    that value; alpha and the stopping test take the sums over the residual itself, so nothing
 //    accumulates: the iteration counts are those of the classical form, also on badly conditioned 1D
 //    systems, where the shorter alpha^2 (q.D^-1 q) - rho (z.q = p.q) needs up to 38 % more.
-//  * A grid-wide sum and the barrier it implies are one exchange (grid_exchange below).
+//  * A grid-wide sum and the barrier it implies are one exchange (exchange.cuh), and the scalars
+//    that follow, a reciprocal and a few products, are formed by one thread.
 //  * A thread owns its rows for the whole solve: x, r, p, D^-1 and q of k_pcg_resident never leave its
 //    registers (p is also written for the neighbours' gathers), and a block keeps as much of its
 //    matrix as fits in shared memory.
@@ -659,7 +660,7 @@ void ilu_apply(gdt_context ctx, gdt_matrix m, const Ilu& f, const double* r, dou
 //    columns of Dirichlet rows) are dropped from the SELL-32 copy: no loads and no FMAs for them.
 //  * Work is spread over all SMs, down to one 32-row slice per block.
 // The matrix and D^-1 are read-only in the kernels (non-coherent loads); p is written by other blocks
-// between the sums and read with plain loads, which the fences of grid_exchange order.
+// between the sums and read with plain loads, which the fences of the exchanges order.
 struct PcgArgs {
   int n;
   int nslices;
@@ -673,29 +674,10 @@ struct PcgArgs {
   double* p;
   double* q;
   KState* st;
-  unsigned long long* slots;   // packets of grid_exchange
-  unsigned int* fault;         // set when a wait ran out
-  unsigned long long wait_ns;  // longest wait in a grid_exchange
-  int cap;                     // matrix entries a block may keep in shared memory (resident form)
-  int stream;                  // the matrix exceeds L2: mark its lines evict-first
+  ExchangeView ex;    // the whole grid
+  int cap;            // matrix entries a block may keep in shared memory (resident form)
+  int stream;         // the matrix exceeds L2: mark its lines evict-first
 };
-
-// The grid-wide sums of an iteration. One exchange is a sum of up to three values per thread and the grid barrier
-// in one (all blocks co-resident): the block sums go out as one 32-byte packet, four words of 48 payload
-// bits each beside 16 bits of the number of the sum, and every block polls all packets until their
-// words carry that number. All blocks add the packets in the same order, so all hold the same bits and
-// none has to broadcast a decision. Two packet buffers alternate: a block can only write sum k + 2 after
-// all have written k + 1, that is after all have read k.
-// Polls delay the stores to the line they read, so a block's packet has 256 bytes of its own (152 blocks
-// exchange in 0.98 us like that, in 2.4 us with packets of 16 bytes side by side) and is read once, not
-// once per value (three values: 3.3 us with a packet and a polling warp each).
-// An FP64 instruction occupies a quarter of the SM for 64 cycles, whichever warp issues it. So the block sums
-// are formed by one warp per value from the threads' values in shared memory (a shuffle tree in every
-// warp would issue five instructions for each one of these), and the scalars that follow, a
-// reciprocal and a few products, by thread 0 alone.
-// Every wait is bounded (time and count); a wait that runs out sets the fault flag, and every block
-// leaves from then on.
-constexpr int kSlot = 32;  // 64-bit words per block and buffer
 
 // The scalars of the iteration, kept by thread 0 of every block (the same bits in all of them).
 struct PcgScalars {
@@ -724,102 +706,12 @@ struct PcgScalars {
 
 template <int T>
 struct PcgShared {
-  double part[3][T];
-  double packet[3][T];  // of block b at [..][b]
-  double own[3];
+  ExchangeShared<T> ex;
   double total[3];
   double last[2];
   PcgScalars k;
   int go;
-  int fault;
 };
-
-__device__ __forceinline__ double sum_strided(const double* v, int groups) {
-  // lane l: v[l] + v[32 + l] + ... in a fixed order, four sums side by side
-  double s[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) s[j] = j < groups ? v[32 * j] : 0.0;
-#pragma unroll 1
-  for (int j0 = 4; j0 < groups; j0 += 4)
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (j0 + j < groups) s[j] += v[32 * (j0 + j)];
-  double b = s[0];
-  if (groups > 2) b = (s[0] + s[1]) + (s[2] + s[3]);
-  else if (groups > 1) b = s[0] + s[1];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) b += __shfl_xor_sync(0xffffffffu, b, o);
-  return b;
-}
-
-// Sum of v over the grid, returned in all lanes of warp k for value k (k < NV); the first `warps` warps hold rows.
-// RELEASE: the block's writes before the call are visible to every block after its next block barrier;
-// without it only the order of their reads before the call and this block's writes after it is kept.
-// At most T blocks.
-template <bool RELEASE, int NV, int T>
-__device__ __forceinline__ double grid_exchange(const PcgArgs& a, unsigned int& epoch, const double (&v)[NV], int warps,
-                                                PcgShared<T>& sh) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nb = gridDim.x;
-  ++epoch;
-  if (warp < warps) {
-#pragma unroll
-    for (int k = 0; k < NV; ++k) sh.part[k][threadIdx.x] = v[k];
-  }
-  __syncthreads();
-  unsigned long long* const base = a.slots + (size_t)kSlot * nb * (epoch & 1u);
-  const unsigned long long tag = (unsigned long long)epoch << 48;
-  if (warp < NV) {
-    const double b = sum_strided(sh.part[warp] + lane, warps);
-    if (lane == 0) sh.own[warp] = b;
-    asm volatile("bar.sync 1, %0;" ::"n"(32 * NV) : "memory");
-    if (threadIdx.x == 0) {
-      unsigned long long w[3];
-#pragma unroll
-      for (int k = 0; k < 3; ++k) w[k] = k < NV ? __double_as_longlong(sh.own[k]) : 0ull;
-      if (RELEASE) fence_acq_rel_gpu();
-      asm volatile("st.relaxed.gpu.global.v4.u64 [%0], {%1, %2, %3, %4};" ::"l"(base + kSlot * blockIdx.x),
-                   "l"((w[0] & 0xffffffffffffull) | tag), "l"((w[0] >> 48) | ((w[1] & 0xffffffffull) << 16) | tag),
-                   "l"((w[1] >> 32) | ((w[2] & 0xffffull) << 32) | tag), "l"((w[2] >> 16) | tag)
-                   : "memory");
-    }
-  }
-  if (warp * 32 < nb) {
-    unsigned long long w[4] = {0, 0, 0, 0}, t0 = 0;
-    bool wait = (int)threadIdx.x < nb;
-    for (unsigned int spins = 1;; ++spins) {
-      if (wait) {
-        if (RELEASE)
-          asm volatile("ld.acquire.gpu.global.v4.u64 {%0, %1, %2, %3}, [%4];"
-                       : "=l"(w[0]), "=l"(w[1]), "=l"(w[2]), "=l"(w[3])
-                       : "l"(base + kSlot * threadIdx.x)
-                       : "memory");
-        else
-          asm volatile("ld.relaxed.gpu.global.v4.u64 {%0, %1, %2, %3}, [%4];"
-                       : "=l"(w[0]), "=l"(w[1]), "=l"(w[2]), "=l"(w[3])
-                       : "l"(base + kSlot * threadIdx.x)
-                       : "memory");
-        wait = (((w[0] ^ tag) | (w[1] ^ tag) | (w[2] ^ tag) | (w[3] ^ tag)) >> 48) != 0;
-      }
-      if (!__any_sync(0xffffffffu, wait)) break;
-      if (spins == 1u) t0 = global_ns();
-      else if (spins == 2u || (spins & 255u) == 0u) {
-        const bool out = spins > (1u << 24) || global_ns() - t0 > a.wait_ns;
-        if (out) atomicExch(a.fault, 1u);
-        if (__any_sync(0xffffffffu, out || *reinterpret_cast<volatile unsigned int*>(a.fault) != 0u)) {
-          if (lane == 0) sh.fault = 1;
-          break;
-        }
-      }
-    }
-    // (a thread past the last block holds zeros)
-    sh.packet[0][threadIdx.x] = __longlong_as_double((w[0] & 0xffffffffffffull) | (w[1] << 48));
-    sh.packet[1][threadIdx.x] = __longlong_as_double(((w[1] >> 16) & 0xffffffffull) | (w[2] << 32));
-    if (NV > 2) sh.packet[2][threadIdx.x] = __longlong_as_double(((w[2] >> 32) & 0xffffull) | (w[3] << 16));
-  }
-  __syncthreads();
-  return warp < NV ? sum_strided(sh.packet[warp] + lane, (nb + 31) >> 5) : 0.0;
-}
 
 // v = (p.q, z.q, q.D^-1 q) over the rows of the thread: alpha and beta in sh.k; false when done. The stopping test
 // of the iteration before is made here too: its sums (sh.last) are formed while the other warps
@@ -828,7 +720,7 @@ template <int T>
 __device__ __forceinline__ bool pcg_step(const PcgArgs& a, unsigned int& epoch, const double (&v)[3], int warps,
                                          PcgShared<T>& sh) {
   const bool first = epoch == 0;
-  const double total = grid_exchange<false>(a, epoch, v, warps, sh);
+  const double total = group_exchange<false>(a.ex, epoch, v, warps, sh.ex);
   if (threadIdx.x < 96) {
     const double inv = threadIdx.x == 0 ? 1.0 / total : 0.0;
     if ((threadIdx.x & 31) == 0) sh.total[threadIdx.x >> 5] = total;
@@ -847,7 +739,7 @@ __device__ __forceinline__ bool pcg_step(const PcgArgs& a, unsigned int& epoch, 
         k.beta = fma(k.alpha * inv, sh.total[2], fma(-2.0 * inv, sh.total[1], 1.0));
         if (!(total > 0.0) || !isfinite(total)) k.brk = k.conv = 1;
       }
-      sh.go = !k.conv && !sh.fault;
+      sh.go = !k.conv && !sh.ex.fault;
     }
   }
   __syncthreads();
@@ -858,7 +750,7 @@ __device__ __forceinline__ bool pcg_step(const PcgArgs& a, unsigned int& epoch, 
 template <int T>
 __device__ __forceinline__ void pcg_publish(const PcgArgs& a, unsigned int& epoch, const double (&v)[2], int warps,
                                             PcgShared<T>& sh) {
-  const double total = grid_exchange<true>(a, epoch, v, warps, sh);
+  const double total = group_exchange<true>(a.ex, epoch, v, warps, sh.ex);
   if (threadIdx.x < 64 && (threadIdx.x & 31) == 0) sh.last[threadIdx.x >> 5] = total;
 }
 
@@ -933,7 +825,7 @@ __global__ void __launch_bounds__(RT, 1) k_pcg_resident(const __grid_constant__ 
   const int ns = int((long long)a.nslices * (blockIdx.x + 1) / gridDim.x) - s0;
   const int warps = min(ns, RT / 32);  // that have rows
   if (threadIdx.x == 0) {
-    sh.fault = 0;
+    sh.ex.fault = 0;
     sh.k.load(a.st);
   }
   // shared-memory offsets of the block's slices, in order (one warp scans)
@@ -1043,7 +935,7 @@ __global__ void __launch_bounds__(PT, 1) k_pcg_stream(const __grid_constant__ Pc
   const int row1 = min(a.n, s1 * 32);
   const unsigned long long pol = matrix_policy(a.stream);
   if (threadIdx.x == 0) {
-    sh.fault = 0;
+    sh.ex.fault = 0;
     sh.k.load(a.st);
   }
   unsigned int epoch = 0;
@@ -1183,9 +1075,11 @@ gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, d
   unsigned long long* const words = reinterpret_cast<unsigned long long*>(ctx->scratch + kScratchDoubles / 2);
   const size_t packets = size_t(2 * kSlot) * blocks;  // two buffers
   if (packets + 16 > kScratchDoubles / 2) return fail(ctx, GDT_EUNSUPPORTED, "persistent solver: grid too large");
-  a.slots = words + 16;
-  a.fault = reinterpret_cast<unsigned int*>(words);
-  a.wait_ns = ctx->persistent_wait_ns > 0 ? (unsigned long long)ctx->persistent_wait_ns : kBarrierNs;
+  a.ex.slots = words + 16;
+  a.ex.fault = reinterpret_cast<unsigned int*>(words);
+  a.ex.first = 0;
+  a.ex.count = blocks;
+  a.ex.wait_ns = ctx->persistent_wait_ns > 0 ? (unsigned long long)ctx->persistent_wait_ns : kBarrierNs;
   a.cap = cap;
   a.stream = 12LL * m->sell_len > (64LL << 20);
   GDT_TRY_CUDA(ctx, cudaMemsetAsync(words, 0, sizeof(unsigned long long) * (packets + 16), s));
@@ -1198,7 +1092,7 @@ gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, d
   GDT_TRY_CUDA(ctx, le);
   ctx->launches++;
   unsigned int fault = 0;
-  GDT_TRY_CUDA(ctx, cudaMemcpyAsync(&fault, a.fault, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
+  GDT_TRY_CUDA(ctx, cudaMemcpyAsync(&fault, a.ex.fault, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
   GDT_TRY_CUDA(ctx, cudaStreamSynchronize(s));
   if (fault) return fail(ctx, GDT_ECUDA, "persistent solver: a grid barrier wait ran out");
   return GDT_OK;

@@ -463,7 +463,8 @@ typedef struct gdt_batch_s* gdt_batch;
 
 enum { GDT_BATCH_P1_SIMPLEX = 0, GDT_BATCH_Q1_CUBE = 1 };
 enum { GDT_BATCH_KAPPA_QUADRANTS = 0, GDT_BATCH_KAPPA_ELEMENTS = 1 };
-/* who solves a problem: the 8 CTAs of a thread-block cluster together, one CTA, or one warp */
+/* who solves a problem: several CTAs together (FP64: as many as the work asks for, planned when the batch or its
+ * teams are set; mixed precision: the 8 of a thread-block cluster), one CTA, or one warp */
 enum { GDT_BATCH_TEAM_CLUSTER = 0, GDT_BATCH_TEAM_CTA = 1, GDT_BATCH_TEAM_WARP = 2 };
 
 typedef struct gdt_batch_info {
@@ -491,7 +492,8 @@ gdt_status gdt_batch_element_offsets(gdt_batch b, int64_t* offsets);
 gdt_status gdt_batch_set_teams(gdt_context ctx, gdt_batch b, const int* teams);
 gdt_status gdt_batch_teams(gdt_batch b, int* teams);
 /* assemble (FP64) and solve every problem to ||b - A x|| <= tol ||b|| in one persistent launch (CUDA
- * graph, re-captured when the arguments or the teams change). kappa: device array (see above); x:
+ * graph, re-captured when the arguments or the teams change; in FP64 with mixed team kinds a launch for the
+ * cluster teams, then one for the others). kappa: device array (see above); x:
  * device [total_dofs]; stencil_out: optional device [total_dofs][7 (P1) or 9 (Q1)] receiving the
  * assembled rows in CSR column order (NULL to skip); precision: GDT_PRECISION_FP64 or
  * GDT_PRECISION_MIXED. info (optional) makes the call wait; then a problem with non-finite data makes
@@ -514,7 +516,8 @@ gdt_status gdt_batch_tune(gdt_context ctx, gdt_batch b, const double* kappa, int
                           double* ms);
 /* per-problem iteration counts (negative: -(count + 1) when not converged) and relative residuals (host) */
 gdt_status gdt_batch_iterations(gdt_context ctx, gdt_batch b, int* iterations, double* rel_residuals);
-/* per-problem status of the last solve (host): GDT_OK, GDT_ENOCONV or GDT_ENAN */
+/* per-problem status of the last solve (host): GDT_OK, GDT_ENOCONV, GDT_ENAN, or GDT_ETIMEOUT where a bounded
+ * wait ran out (the solve then returned GDT_ECUDA) */
 gdt_status gdt_batch_status(gdt_context ctx, gdt_batch b, int* status);
 
 /* ------------------------------------------------------------------ adjoint --- */
