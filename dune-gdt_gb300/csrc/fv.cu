@@ -8,15 +8,19 @@
 //   (test/instationary-eocstudies/base.hh:428-447) and ExplicitRungeKuttaTimeStepper with the SSP2
 //   tableau (tools/timestepper/explicit-rungekutta.hh:82-97, 237-270), r = -1.
 //
-// GB300 design: GB300's FP64 pipe (~0.6e12 instructions/s), not HBM, bounds this update, so the 2D
-// stepper computes every face flux exactly once per stage inside a shared-memory tile (tile + periodic
-// halo staged from global memory), and the second SSP stage fuses u1 = u - dt k0, k1 = L(u1) and
+// GB300 design: an FP64 instruction holds a quarter of an SM for 64 cycles, also where it is predicated off, and that
+// pipe, not HBM, bounds this update. So every face flux is computed exactly once per stage, with as few
+// FP64 instructions as the flux allows (fv_face4: two for Burgers LF), and all selecting, comparing and
+// sign handling runs on the integer pipe. The second SSP stage fuses u1 = u - dt k0, k1 = L(u1) and
 // u_new = u + (k0 + k1)(-dt/2) into one pass: per step it reads u (twice) and k0 and writes k0 and
-// u_new (40 bytes per cell). LF uses the local speed max(|f'(u)|, |f'(v)|) multiplied in directly
-// (the reference forms 0.5 / (1 / lambda); both agree to rounding). FP64 instructions per cell and
-// stage (Burgers LF): the squares once per staged cell, three per face (u - v, u^2 + v^2 and one FMA,
-// with 2 max(|u|, |v|) on the integer pipe), three for the update K and at most two for the stage's
-// output: about 10 (first stage) and 13.5 (second) where the per-face form took 25.
+// u_new (40 bytes per cell). Boundary treatments are ghost states in the halo (extrapolation: the inside
+// state, Dirichlet: the prescribed one), for which the face flux is the boundary flux, since
+// g(u, v, n) = -g(v, u, -n) for all three fluxes; a prescribed flux, or none, is selected in place of the
+// computed face. Kernels: 2D tiles (fv2d_tile), 3D tiles that march along z (fv3d_march) and 1D
+// segments (fv1d_segment); grids with a single cell in some direction take fv_apply_kernel.
+// SSP-RK2 steps before (FP64 per face: three instructions; boundary fluxes and 1D / 3D in the generic
+// form, each face twice) and now: 2048^2 Burgers LF 197 and 162 us, with inflow and outflow 359 and 162;
+// 128 x 140 x 120 929 and 158; 100,000 cells 25 and 11; 120 x 97 with boundaries 28 and 7.5.
 #include <cmath>
 #include <limits>
 
@@ -34,14 +38,16 @@ struct FvParams {
   double lf_inv_lambda;  // 0: local LF; else the reference's fixed lambda_ (coefficient 0.5 / lambda_)
   int bkind[6];          // per side (-x, +x, -y, +y, -z, +z): GDT_FV_BOUNDARY_*, or -1 for a periodic side
   double bval[6];
-  // the tiled kernels' form of the flux, 4 g (see face_flux4)
+  // the tiled kernels' form of the flux, 4 g (see fv_face4)
   int form4;             // FORM4_*
   double lam2;           // Burgers LF: 2 lambda_ for a fixed lambda_, 0 for the local one
   double tu[3], tv[3];   // linear transport: 4 g = tu u + tv v (EO: each term only for a positive state)
+  int bounded;           // some side has a boundary treatment
+  double bflux4[6];      // 4 g in +e_k direction through a side with a prescribed flux (or none: 0)
 };
 
-enum { FORM4_GENERIC = 0, FORM4_BURGERS_LF = 1, FORM4_TRANSPORT_LINEAR = 2, FORM4_BURGERS_EO = 3,
-       FORM4_TRANSPORT_EO = 4, FORM4_BURGERS_UPWIND = 5, FORM4_BURGERS_LF_FIXED = 6 };
+enum { FORM4_BURGERS_LF, FORM4_BURGERS_LF_FIXED, FORM4_BURGERS_EO, FORM4_BURGERS_UPWIND, FORM4_TRANSPORT_LINEAR,
+       FORM4_TRANSPORT_EO };
 
 __device__ __forceinline__ double f_of(const FvParams& p, double u, int d) {
   return p.flux == GDT_FLUX_BURGERS ? 0.5 * u * u : p.vel[d] * u;
@@ -104,51 +110,77 @@ __device__ __forceinline__ double boundary_face_flux(const FvParams& p, int dim,
   return upper ? g : -g;
 }
 
-// 4 g(u, v, +e_k), the numerical flux in a form with fewer FP64 instructions (GB300's FP64 pipe
-// bounds the FV update): the factors 1/2 of the flux formulas move into the 1/4 of the update
-// coefficients (scaling by powers of two is exact), the transport fluxes collapse to precomputed
-// linear combinations, and max(|u|, |v|) and the sign tests run on the integer bit patterns (for
-// non-negative doubles the integer order is the floating-point order). Equal to 4 face_flux() up
-// to the rounding of the rearranged sums.
+// The tiled kernels work with 4 g: the factors 1/2 of the flux formulas move into the 1/4 of the update
+// coefficients (scaling by powers of two is exact) and the transport fluxes collapse to precomputed
+// linear combinations.
 __device__ __forceinline__ bool positive(double u) { return __double_as_longlong(u) > 0; }
-// max(|u|, |v|) on the bit patterns, with `add` added to the result's pattern (1 << 52 doubles a
-// normal number). In inline PTX: written in C++, the mask / integer max / exponent add is recognised
-// as fabs, fmax and a doubling and moved onto the FP64 pipe (two more FP64 instructions per face in
-// the instruction counts), which this part issues at one warp instruction per 16 SM cycles.
-__device__ __forceinline__ double abs_max_bits(double u, double v, long long add) {
-  long long r;
-  asm("{\n\t"
-      ".reg .b64 a, b;\n\t"
-      "and.b64 a, %1, 0x7fffffffffffffff;\n\t"
-      "and.b64 b, %2, 0x7fffffffffffffff;\n\t"
-      "max.s64 a, a, b;\n\t"
-      "add.s64 %0, a, %3;\n\t"
-      "}"
-      : "=l"(r)
-      : "l"(__double_as_longlong(u)), "l"(__double_as_longlong(v)), "l"(add));
-  return __longlong_as_double(r);
+// 2 q for a square q >= 0 (or NaN) on its bit pattern: a normal number's exponent plus one, a subnormal's bits
+// shifted, infinity where that overflows
+__device__ __forceinline__ double twice(double q) {
+  unsigned long long b = (unsigned long long)__double_as_longlong(q);
+  constexpr unsigned long long one = 1ull << 52, inf = 0x7ffull << 52;
+  if (b < one) b <<= 1;
+  else if (b < inf - one) b += one;
+  else if (b < inf) b = inf;
+  return __longlong_as_double((long long)b);
 }
-__device__ __forceinline__ double abs_max(double u, double v) { return abs_max_bits(u, v, 0); }
-
+// what a cell contributes to the faces besides its value: 2 u^2 (Burgers LF), u^2 (its fixed-lambda form) or 4 f(u)
+// (Burgers upwind, EO)
+__host__ __device__ constexpr bool uses_squares(int form) {
+  return form == FORM4_BURGERS_LF || form == FORM4_BURGERS_LF_FIXED || form == FORM4_BURGERS_UPWIND ||
+         form == FORM4_BURGERS_EO;
+}
 template <int FORM>
-__device__ __forceinline__ double face_flux4(const FvParams& p, int k, double u, double v) {
-  if constexpr (FORM == FORM4_BURGERS_LF) {  // 2 (f(u) + f(v)) + 2 lambda (u - v), f(u) = u^2 / 2
-    const double lam = abs_max(u, v);
-    return fma(lam + lam, u - v, fma(u, u, v * v));
+__device__ __forceinline__ double cell_square(double u) {
+  return FORM == FORM4_BURGERS_LF_FIXED ? u * u : twice(u * u);
+}
+
+// m = the one of u, v of larger magnitude: sd = d or -d and sel = qu or qv by the table at fv_face4. In inline PTX:
+// written in C++ the mask and comparison are recognised as fabs and a comparison of doubles and moved to the FP64
+// pipe, two more instructions there per face (234 instead of 167 us a step on 2048^2).
+__device__ __forceinline__ void burgers_lf_choose(double u, double v, double d, double qu, double qv, double& sd,
+                                                  double& sel) {
+  asm("{\n\t"
+      ".reg .b64 a, b, m;\n\t"
+      ".reg .pred first, negative, keep;\n\t"
+      "and.b64 a, %2, 0x7fffffffffffffff;\n\t"
+      "and.b64 b, %3, 0x7fffffffffffffff;\n\t"
+      "setp.ge.s64 first, a, b;\n\t"
+      "selp.b64 m, %2, %3, first;\n\t"
+      "setp.lt.s64 negative, m, 0;\n\t"
+      "xor.pred keep, first, negative;\n\t"
+      "selp.b64 m, 0, 0x8000000000000000, keep;\n\t"
+      "xor.b64 %0, %4, m;\n\t"
+      "selp.b64 %1, %6, %5, negative;\n\t"
+      "}"
+      : "=l"(*reinterpret_cast<long long*>(&sd)), "=l"(*reinterpret_cast<long long*>(&sel))
+      : "l"(__double_as_longlong(u)), "l"(__double_as_longlong(v)), "l"(__double_as_longlong(d)),
+        "l"(__double_as_longlong(qu)), "l"(__double_as_longlong(qv)));
+}
+
+// 4 g(u, v, +e_k) with qu, qv = cell_square(u), (v).
+// Burgers LF is u^2 + v^2 + 2 max(|u|, |v|) (u - v). With m the state of larger magnitude that is
+//   2 u^2 + (u - v)^2 for m = u > 0,  2 v^2 - (u - v)^2 for m = u < 0,
+//   2 u^2 - (u - v)^2 for m = v > 0,  2 v^2 + (u - v)^2 for m = v < 0:
+// one subtraction and one FMA on the FP64 pipe, the choices on bit patterns (for non-negative doubles
+// the integer order is the floating-point order).
+template <int FORM>
+__device__ __forceinline__ double fv_face4(const FvParams& p, int k, double u, double v, double qu, double qv) {
+  if constexpr (FORM == FORM4_BURGERS_LF) {
+    const double d = u - v;
+    double sd, sel;
+    burgers_lf_choose(u, v, d, qu, qv, sd, sel);
+    return fma(sd, d, sel);
   } else if constexpr (FORM == FORM4_BURGERS_LF_FIXED) {
-    return fma(p.lam2, u - v, fma(u, u, v * v));
+    return fma(p.lam2, u - v, qu + qv);
   } else if constexpr (FORM == FORM4_TRANSPORT_LINEAR) {
     return fma(p.tu[k], u, p.tv[k] * v);
   } else if constexpr (FORM == FORM4_BURGERS_EO) {  // 4 * (u > 0 ? u^2 / 2 : 0)
-    return positive(u) ? (u + u) * u : 0.0;
+    return positive(u) ? qu : 0.0;
   } else if constexpr (FORM == FORM4_TRANSPORT_EO) {
-    return (positive(u) ? p.tu[k] * u : 0.0) + (positive(v) ? p.tv[k] * v : 0.0);
-  } else if constexpr (FORM == FORM4_BURGERS_UPWIND) {  // f'((u + v) / 2) > 0 ? 4 f(u) : 4 f(v)
-    const double w = (u + v) * 0.5;
-    const double sel = positive(w) ? u : v;
-    return (sel + sel) * sel;
-  } else {
-    return 4.0 * face_flux(p, 2, k, u, v);
+    return fma(p.tu[k], positive(u) ? u : 0.0, p.tv[k] * (positive(v) ? v : 0.0));
+  } else {  // Burgers upwind: f'((u + v) / 2) > 0 ? 4 f(u) : 4 f(v)
+    return positive(u + v) ? qu : qv;
   }
 }
 
@@ -208,96 +240,247 @@ __global__ void fv_apply_kernel(GridDesc g, FvParams p, long long nbatch, const 
   else u_next[off + c] = fma(dt_coef, out[off + c] + acc, ubase[off + c]);
 }
 
-// ------------------------------------------------------------------------------- 2D tiled ---
-constexpr int TX = 32, TY = 32, BY = 8;  // tile TX x TY cells, block TX x BY threads
-
-// 2 max(|u|, |v|) for the local LF speed, on the integer pipe: the larger magnitude's bit pattern with
-// the exponent raised by one (exact for normal numbers; for zero and subnormal speeds the product with
-// u - v, at most twice their size, underflows to zero either way)
-__device__ __forceinline__ double twice_abs_max(double u, double v) { return abs_max_bits(u, v, 1LL << 52); }
-// the Burgers LF forms use the squares of the states, computed once per cell when the tile is staged
-__host__ __device__ constexpr bool uses_squares(int form) {
-  return form == FORM4_BURGERS_LF || form == FORM4_BURGERS_LF_FIXED;
-}
-// 4 g(u, v, +e_k) with the squares qu = u^2, qv = v^2 at hand: three FP64 instructions for Burgers LF
-template <int FORM>
-__device__ __forceinline__ double face4s(const FvParams& p, int k, double u, double v, double qu, double qv) {
-  if constexpr (FORM == FORM4_BURGERS_LF) return fma(twice_abs_max(u, v), u - v, qu + qv);
-  else if constexpr (FORM == FORM4_BURGERS_LF_FIXED) return fma(p.lam2, u - v, qu + qv);
-  else return face_flux4<FORM>(p, k, u, v);
-}
-
-// One stage over a tile of TX x TY cells of state b (blockIdx.z). The fluxes are kept as 4 g, and the
-// update as K = (gx_right - gx_left) + rho (gy_top - gy_bottom), rho = h_x / h_y, so that
-// L(u) = (1 / (4 h_x)) K:
-//   STAGE 0: out = c_out K (fv_apply: c_out = 1 / (4 h_x), giving L(u))
-//   STAGE 3: out = K (the first SSP-RK2 stage keeps K itself: no multiply by one per cell)
+// ------------------------------------------------------------------------------- tiled kernels ---
+// One stage of a step. The fluxes are kept as 4 g, and the update as
+// K = sum_k rho_k (g_k,upper - g_k,lower), rho_k = h_x / h_k, so that L(u) = K / (4 h_x):
+//   STAGE 0: out = c_out K (fv_apply: c_out = 1 / (4 h_x), giving L(u)), or K itself for c_out = 1 (the first
+//            SSP-RK2 stage: no multiply by one per cell)
 //   STAGE 1 (Euler): out = u + c_out K, c_out = -dt / (4 h_x)
 //   STAGE 2 (SSP-RK2): u1 = u + c1 k0 on the tile + halo (k0 = K(u), c1 = -dt / (4 h_x)),
 //            out = u + c_out (k0 + K(u1)), c_out = -dt / (8 h_x)
-// Every FP64 pass runs whole warps over 32 values: the tile interior column by column, the two halo
-// columns and the 33rd x face of every row in passes of their own (a pass with one active lane costs
-// the FP64 pipe as much as a full one). BND: some side has a boundary treatment; the faces on those
-// sides are then replaced by it. FORM: the numerical flux (FORM4_*), compiled as straight-line code.
-template <int STAGE, bool BND, int FORM>
-__global__ void __launch_bounds__(TX* BY) fv2d_tile(GridDesc g, FvParams p, const double* __restrict__ u,
-                                                    const double* __restrict__ k0, double* __restrict__ out,
-                                                    double c1, double c_out, double rho) {
+// FORM: the numerical flux, compiled as straight-line code.
+struct StageArgs {
+  const double* u;
+  const double* k0;
+  double* out;
+  double c1, c_out, rho[3];
+};
+
+// The stages of a step follow each other in the stream, each reading what the one before wrote. They are launched with
+// programmatic serialisation: a stage's blocks may be placed while the last ones of the stage before still
+// run, and wait here, before their first access to the state, until that stage is complete and visible.
+__device__ __forceinline__ void fv_stage_begin() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// lets the next stage's blocks be placed; near the end of a block, since blocks placed early crowd the SMs that are
+// done first (60^3 cells: 42 us a step when called at the start, 25 here, 31 without)
+__device__ __forceinline__ void fv_stage_ends() { asm volatile("griddepcontrol.launch_dependents;"); }
+
+// cell c in -1 .. n (beyond a partial tile: further) of a direction -> the cell whose state it takes
+__device__ __forceinline__ long long fv_cell(long long c, long long n, bool periodic) {
+  if (c < 0) return periodic ? n - 1 : 0;
+  if (c >= n) return periodic && c == n ? 0 : n - 1;
+  return c;
+}
+template <int STAGE>
+__device__ __forceinline__ double fv_load(const StageArgs& a, long long cell) {
+  double v = a.u[cell];
+  if (STAGE == 2) v = fma(a.k0[cell], a.c1, v);
+  return v;
+}
+// the state beyond a side: prescribed, or what fv_cell chose
+__device__ __forceinline__ double fv_ghost(const FvParams& p, int k, long long c, long long n, double v) {
+  if (p.bounded && c < 0 && p.bkind[2 * k] == GDT_FV_BOUNDARY_DIRICHLET) return p.bval[2 * k];
+  if (p.bounded && c >= n && p.bkind[2 * k + 1] == GDT_FV_BOUNDARY_DIRICHLET) return p.bval[2 * k + 1];
+  return v;
+}
+// 4 g through the face below cell c of direction k, or the side's flux in its place
+__device__ __forceinline__ bool fv_side_flux(int kind) {
+  return kind == GDT_FV_BOUNDARY_FLUX || kind == GDT_FV_BOUNDARY_NONE;
+}
+__device__ __forceinline__ double fv_side(const FvParams& p, int k, long long c, long long n, double f) {
+  if (p.bounded && c == 0 && fv_side_flux(p.bkind[2 * k])) return p.bflux4[2 * k];
+  if (p.bounded && c == n && fv_side_flux(p.bkind[2 * k + 1])) return p.bflux4[2 * k + 1];
+  return f;
+}
+template <int STAGE>
+__device__ __forceinline__ void fv_store(const StageArgs& a, long long cell, double K) {
+  if (STAGE == 0) {
+    if (a.c_out == 1.0) a.out[cell] = K;  // (a branch: a selected product would still be computed)
+    else a.out[cell] = a.c_out * K;
+  } else if (STAGE == 1) a.out[cell] = fma(a.c_out, K, a.u[cell]);
+  else a.out[cell] = fma(a.c_out, a.k0[cell] + K, a.u[cell]);
+}
+
+constexpr int TX = 32, BY = 8;  // tile TX x TY cells (TY: 32 or 8), block TX x BY threads
+
+// 2D: a tile of TX x TY cells of state blockIdx.z. Every FP64 pass runs whole warps over 32 values: the tile
+// interior column by column, the two halo columns and the 33rd x face of every row in passes of their
+// own (a pass with one active lane costs the FP64 pipe as much as a full one).
+template <int STAGE, int FORM, int TY>
+__global__ void __launch_bounds__(TX* BY) fv2d_tile(const __grid_constant__ GridDesc g,
+                                                    const __grid_constant__ FvParams p,
+                                                    const __grid_constant__ StageArgs a) {
   constexpr bool SQ = uses_squares(FORM);
   __shared__ double s[TY + 2][TX + 2];             // staged state: s[j + 1][i + 1] = cell (x0 + i, y0 + j)
-  __shared__ double q[SQ ? TY + 2 : 1][TX + 2];    // its squares
+  __shared__ double q[SQ ? TY + 2 : 1][TX + 2];    // its cell_square
   __shared__ double gx[TY][TX + 1];                // gx[j][i]: x face between tile columns i - 1 and i
   __shared__ double gy[TY + 1][TX];                // gy[j][i]: y face between tile rows j - 1 and j
   const long long nx = g.n[0], ny = g.n[1];
   const long long off = (long long)blockIdx.z * nx * ny;
   const long long x0 = (long long)blockIdx.x * TX, y0 = (long long)blockIdx.y * TY;
   const int tx = threadIdx.x, ty = threadIdx.y;
-  // periodic wrap by compare and select (a 64-bit modulo would cost more than the flux arithmetic);
-  // beyond a partial tile: clamped, unused
-  auto wrap = [](long long c, long long n) { return c < 0 ? n - 1 : (c == n ? 0 : (c > n ? n - 1 : c)); };
+  const bool px = p.bkind[0] < 0, py = p.bkind[2] < 0;  // periodic directions
+  const int rows = (int)min((long long)TY, ny - y0);
+  fv_stage_begin();
   auto stage = [&](int j, int i) {
-    const long long cidx = off + wrap(y0 + j - 1, ny) * nx + wrap(x0 + i - 1, nx);
-    double v = u[cidx];
-    if (STAGE == 2) v = fma(k0[cidx], c1, v);
+    const long long cx = x0 + i - 1, cy = y0 + j - 1;
+    double v = fv_load<STAGE>(a, off + fv_cell(cy, ny, py) * nx + fv_cell(cx, nx, px));
+    v = fv_ghost(p, 0, cx, nx, v);
+    v = fv_ghost(p, 1, cy, ny, v);
     s[j][i] = v;
-    if constexpr (SQ) q[j][i] = v * v;
+    if constexpr (SQ) q[j][i] = cell_square<FORM>(v);
   };
-  for (int j = ty; j < TY + 2; j += BY) stage(j, tx + 1);  // interior columns
+  for (int j = ty; j < rows + 2; j += BY) stage(j, tx + 1);  // interior columns
   {
     // the two halo columns, 2 (TY + 2) values, in the block's first warps
     const int e = ty * TX + tx;
-    if (e < 2 * (TY + 2)) stage(e % (TY + 2), e < TY + 2 ? 0 : TX + 1);
+    if (e < 2 * (TY + 2) && e % (TY + 2) < rows + 2) stage(e % (TY + 2), e < TY + 2 ? 0 : TX + 1);
   }
   __syncthreads();
-  auto xface = [&](int j, int i) {  // 4 g through the x face between tile columns i - 1 and i of row j
-    if (BND && p.bkind[0] >= 0 && x0 + i == 0) return 4.0 * boundary_face_flux(p, 2, 0, false, s[j + 1][i + 1]);
-    if (BND && p.bkind[0] >= 0 && x0 + i == nx) return 4.0 * boundary_face_flux(p, 2, 0, true, s[j + 1][i]);
-    if constexpr (SQ) return face4s<FORM>(p, 0, s[j + 1][i], s[j + 1][i + 1], q[j + 1][i], q[j + 1][i + 1]);
-    else return face4s<FORM>(p, 0, s[j + 1][i], s[j + 1][i + 1], 0.0, 0.0);
-  };
-  for (int j = ty; j < TY; j += BY) gx[j][tx] = xface(j, tx);
-  if (ty == 0) gx[tx][TX] = xface(tx, TX);  // the right face of every row: one pass of the first warp
-  for (int j = ty; j <= TY; j += BY) {
+  auto face = [&](int k, int j, int i, int jl, int il) {  // between staged cells (jl, il) and (j, i)
     double f;
-    if (BND && p.bkind[2] >= 0 && y0 + j == 0) f = 4.0 * boundary_face_flux(p, 2, 1, false, s[j + 1][tx + 1]);
-    else if (BND && p.bkind[2] >= 0 && y0 + j == ny) f = 4.0 * boundary_face_flux(p, 2, 1, true, s[j][tx + 1]);
-    else if constexpr (SQ) f = face4s<FORM>(p, 1, s[j][tx + 1], s[j + 1][tx + 1], q[j][tx + 1], q[j + 1][tx + 1]);
-    else f = face4s<FORM>(p, 1, s[j][tx + 1], s[j + 1][tx + 1], 0.0, 0.0);
-    gy[j][tx] = f;
-  }
+    if constexpr (SQ) f = fv_face4<FORM>(p, k, s[jl][il], s[j][i], q[jl][il], q[j][i]);
+    else f = fv_face4<FORM>(p, k, s[jl][il], s[j][i], 0.0, 0.0);
+    return k == 0 ? fv_side(p, 0, x0 + i - 1, nx, f) : fv_side(p, 1, y0 + j - 1, ny, f);
+  };
+  for (int j = ty; j < rows; j += BY) gx[j][tx] = face(0, j + 1, tx + 1, j + 1, tx);
+  if (ty == 0 && tx < rows) gx[tx][TX] = face(0, tx + 1, TX + 1, tx + 1, TX);  // the right face of every row
+  for (int j = ty; j <= rows; j += BY) gy[j][tx] = face(1, j + 1, tx + 1, j, tx + 1);
   __syncthreads();
+  fv_stage_ends();
   const long long gxi = x0 + tx;
   if (gxi >= nx) return;
-  for (int j = ty; j < TY; j += BY) {
-    const long long gyj = y0 + j;
-    if (gyj >= ny) break;
-    const double K = fma(rho, gy[j + 1][tx] - gy[j][tx], gx[j][tx + 1] - gx[j][tx]);
-    const long long cidx = off + gyj * nx + gxi;
-    if (STAGE == 3) out[cidx] = K;
-    else if (STAGE == 0) out[cidx] = c_out * K;
-    else if (STAGE == 1) out[cidx] = fma(c_out, K, u[cidx]);
-    else out[cidx] = fma(c_out, k0[cidx] + K, u[cidx]);
+  for (int j = ty; j < rows; j += BY) {
+    const double K = fma(a.rho[1], gy[j + 1][tx] - gy[j][tx], gx[j][tx + 1] - gx[j][tx]);
+    fv_store<STAGE>(a, off + (y0 + j) * nx + gxi, K);
   }
+}
+
+// 3D: a tile of MX x MY cells marches up a chunk of z planes. Each plane's state is staged with its halo, a thread
+// holds the state of its own column at z and z + 1 and the flux through its lower z face; faces of the x
+// and y directions are computed once and read by the neighbour through shared memory. The two barriers of
+// a plane also separate its reads from the next plane's stores: the state is read before the second, the
+// faces are written after the first.
+constexpr int MX = 32, MY = 8;
+
+template <int STAGE, int FORM>
+__global__ void __launch_bounds__(MX* MY) fv3d_march(const __grid_constant__ GridDesc g,
+                                                     const __grid_constant__ FvParams p,
+                                                     const __grid_constant__ StageArgs a, int chunk, int chunks) {
+  constexpr bool SQ = uses_squares(FORM);
+  __shared__ double s[MY + 2][MX + 2];
+  __shared__ double q[SQ ? MY + 2 : 1][MX + 2];
+  __shared__ double gx[MY][MX + 1];
+  __shared__ double gy[MY + 1][MX];
+  const long long nx = g.n[0], ny = g.n[1], nz = g.n[2];
+  const long long off = (long long)(blockIdx.z / chunks) * nx * ny * nz;
+  const long long x0 = (long long)blockIdx.x * MX, y0 = (long long)blockIdx.y * MY;
+  const long long z0 = (long long)(blockIdx.z % chunks) * chunk, z1 = min(nz, z0 + chunk);
+  const int tx = threadIdx.x, ty = threadIdx.y, e = ty * MX + tx;
+  const bool px = p.bkind[0] < 0, py = p.bkind[2] < 0, pz = p.bkind[4] < 0;
+  const int rows = (int)min((long long)MY, ny - y0);
+  // the thread's own column and, in the first threads, one value of the halo ring (of MX or MY + 2 at each end)
+  const long long own = fv_cell(y0 + ty, ny, py) * nx + fv_cell(x0 + tx, nx, px);
+  int hj = -1, hi = 0;
+  if (e < 2 * MX) {  // rows below and above
+    hj = e < MX ? 0 : rows + 1;
+    hi = tx + 1;
+  } else if (e < 2 * MX + 2 * MY) {  // columns left and right
+    const int h = e - 2 * MX;
+    hj = h % MY + 1;
+    hi = h < MY ? 0 : MX + 1;
+    if (hj > rows) hj = -1;
+  }
+  const long long hx = x0 + hi - 1, hy = y0 + hj - 1;
+  const long long halo = fv_cell(hy, ny, py) * nx + fv_cell(hx, nx, px);
+  // the state of the thread's column in plane z (a column right of the grid, in a partial tile, holds the state
+  // beyond the upper x side)
+  auto column = [&](long long z) {
+    double v = fv_load<STAGE>(a, off + fv_cell(z, nz, pz) * nx * ny + own);
+    if (x0 + tx >= nx) v = fv_ghost(p, 0, x0 + tx, nx, v);
+    return fv_ghost(p, 2, z, nz, v);
+  };
+  auto plane = [&](long long z) { return off + fv_cell(z, nz, pz) * nx * ny; };
+  fv_stage_begin();
+  const double lower = column(z0 - 1);
+  double cur = column(z0);
+  double ring = hj >= 0 ? fv_load<STAGE>(a, plane(z0) + halo) : 0.0;
+  double qcur = SQ ? cell_square<FORM>(cur) : 0.0;
+  double gz = fv_side(p, 2, z0, nz, fv_face4<FORM>(p, 2, lower, cur, SQ ? cell_square<FORM>(lower) : 0.0, qcur));
+  for (long long z = z0; z < z1; ++z) {
+    if (ty < rows) {  // (the row above a partial tile belongs to the ring)
+      s[ty + 1][tx + 1] = cur;
+      if constexpr (SQ) q[ty + 1][tx + 1] = qcur;
+    }
+    if (hj >= 0) {
+      double v = fv_ghost(p, 0, hx, nx, ring);
+      v = fv_ghost(p, 1, hy, ny, v);
+      s[hj][hi] = v;
+      if constexpr (SQ) q[hj][hi] = cell_square<FORM>(v);
+    }
+    // the next plane, in flight over the faces of this one
+    const double next = column(z + 1);
+    if (hj >= 0 && z + 1 < z1) ring = fv_load<STAGE>(a, plane(z + 1) + halo);
+    __syncthreads();
+    auto face = [&](int k, int j, int i, int jl, int il) {  // between staged cells (jl, il) and (j, i)
+      double f;
+      if constexpr (SQ) f = fv_face4<FORM>(p, k, s[jl][il], s[j][i], q[jl][il], q[j][i]);
+      else f = fv_face4<FORM>(p, k, s[jl][il], s[j][i], 0.0, 0.0);
+      return k == 0 ? fv_side(p, 0, x0 + i - 1, nx, f) : fv_side(p, 1, y0 + j - 1, ny, f);
+    };
+    if (ty < rows) {
+      gx[ty][tx] = face(0, ty + 1, tx + 1, ty + 1, tx);
+      gy[ty][tx] = face(1, ty + 1, tx + 1, ty, tx + 1);
+    }
+    if (ty == 0) {
+      if (tx < rows) gx[tx][MX] = face(0, tx + 1, MX + 1, tx + 1, MX);
+      gy[rows][tx] = face(1, rows + 1, tx + 1, rows, tx + 1);
+    }
+    const double qnext = SQ ? cell_square<FORM>(next) : 0.0;
+    const double gup = fv_side(p, 2, z + 1, nz, fv_face4<FORM>(p, 2, cur, next, qcur, qnext));
+    __syncthreads();
+    if (z + 1 == z1) fv_stage_ends();
+    if (x0 + tx < nx && ty < rows) {
+      const double dxy = fma(a.rho[1], gy[ty + 1][tx] - gy[ty][tx], gx[ty][tx + 1] - gx[ty][tx]);
+      fv_store<STAGE>(a, off + (z * ny + y0 + ty) * nx + x0 + tx, fma(a.rho[2], gup - gz, dxy));
+    }
+    gz = gup;
+    cur = next;
+    qcur = qnext;
+  }
+}
+
+// 1D: a segment of SX cells, one per thread; a thread computes the face below its cell, the last one also the face
+// above
+constexpr int SX = 256;
+
+template <int STAGE, int FORM>
+__global__ void __launch_bounds__(SX) fv1d_segment(const __grid_constant__ GridDesc g,
+                                                   const __grid_constant__ FvParams p,
+                                                   const __grid_constant__ StageArgs a) {
+  constexpr bool SQ = uses_squares(FORM);
+  __shared__ double s[SX + 2], q[SQ ? SX + 2 : 1], gx[SX + 1];
+  const unsigned int segments = (unsigned int)((g.n[0] + SX - 1) / SX);
+  const long long nx = g.n[0], off = (long long)(blockIdx.x / segments) * nx;
+  const long long x0 = (long long)(blockIdx.x % segments) * SX;
+  const bool px = p.bkind[0] < 0;
+  const int cells = (int)min((long long)SX, nx - x0);
+  fv_stage_begin();
+  for (int i = threadIdx.x; i < cells + 2; i += SX) {
+    const long long c = x0 + i - 1;
+    const double v = fv_ghost(p, 0, c, nx, fv_load<STAGE>(a, off + fv_cell(c, nx, px)));
+    s[i] = v;
+    if constexpr (SQ) q[i] = cell_square<FORM>(v);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i <= cells; i += SX) {
+    double f;
+    if constexpr (SQ) f = fv_face4<FORM>(p, 0, s[i], s[i + 1], q[i], q[i + 1]);
+    else f = fv_face4<FORM>(p, 0, s[i], s[i + 1], 0.0, 0.0);
+    gx[i] = fv_side(p, 0, x0 + i, nx, f);
+  }
+  __syncthreads();
+  fv_stage_ends();
+  if ((int)threadIdx.x < cells) fv_store<STAGE>(a, off + x0 + threadIdx.x, gx[threadIdx.x + 1] - gx[threadIdx.x]);
 }
 
 FvParams make_params(const GridDesc& g, const gdt_fv_desc* d) {
@@ -306,8 +489,8 @@ FvParams make_params(const GridDesc& g, const gdt_fv_desc* d) {
   p.numflux = d->numflux;
   for (int i = 0; i < 3; ++i) p.vel[i] = d->velocity[i];
   p.lf_inv_lambda = d->lf_lambda;
-  p.form4 = FORM4_GENERIC;
   p.lam2 = 0.0;
+  p.bounded = 0;
   for (int k = 0; k < 3; ++k) p.tu[k] = p.tv[k] = 0.0;
   if (d->flux == GDT_FLUX_BURGERS) {
     if (d->numflux == GDT_NUMFLUX_LAX_FRIEDRICHS) {
@@ -342,58 +525,108 @@ FvParams make_params(const GridDesc& g, const gdt_fv_desc* d) {
     const bool periodic = g.periodic && d->boundary[side] == GDT_FV_BOUNDARY_NONE;
     p.bkind[side] = periodic ? -1 : d->boundary[side];
     p.bval[side] = d->boundary_value[side];
+    if (side < 2 * g.dim && p.bkind[side] >= 0) p.bounded = 1;
+    p.bflux4[side] = p.bkind[side] == GDT_FV_BOUNDARY_FLUX ? ((side & 1) ? 4.0 : -4.0) * p.bval[side] : 0.0;
   }
   return p;
 }
 
-bool has_boundary(const FvParams& p, int dim) {
-  for (int side = 0; side < 2 * dim; ++side)
-    if (p.bkind[side] >= 0) return true;
-  return false;
+// planes per block of fv3d_march: the chunk with the least work on the fullest SM, 13 FP64 instructions per cell of a
+// plane, four for the face and the squares a chunk computes besides, and its two plane loads before the
+// first face counted as six more (20 x 25 x 18 cells: 12.8 us a step with one plane, 29 with four; 60^3:
+// 32 us with one, 25 with two; 128 x 140 x 120: 158 us with eight, 176 with fourteen)
+int march_chunk(gdt_context ctx, const GridDesc& g, long long nbatch) {
+  const long long tiles = ((g.n[0] + MX - 1) / MX) * ((g.n[1] + MY - 1) / MY) * nbatch;
+  long long best = 0;
+  int chosen = 1;
+  for (int chunk = 1; chunk <= 16 && chunk <= g.n[2]; ++chunk) {
+    const long long blocks = tiles * ((g.n[2] + chunk - 1) / chunk);
+    const long long cost = (blocks + ctx->num_sms - 1) / ctx->num_sms * (13 * chunk + 10);
+    if (best == 0 || cost < best) best = cost, chosen = chunk;
+  }
+  return chosen;
 }
 
-template <int STAGE, bool BND>
-void launch_tile_b(dim3 grid, cudaStream_t s, const GridDesc& g, const FvParams& p, const double* u, const double* k0,
-                   double* out, double c1, double c_out, double rho) {
-  const dim3 block(TX, BY);
-  switch (p.form4) {
-    case FORM4_BURGERS_LF: fv2d_tile<STAGE, BND, FORM4_BURGERS_LF><<<grid, block, 0, s>>>(g, p, u, k0, out, c1, c_out, rho); break;
-    case FORM4_BURGERS_LF_FIXED:
-      fv2d_tile<STAGE, BND, FORM4_BURGERS_LF_FIXED><<<grid, block, 0, s>>>(g, p, u, k0, out, c1, c_out, rho);
-      break;
-    case FORM4_TRANSPORT_LINEAR:
-      fv2d_tile<STAGE, BND, FORM4_TRANSPORT_LINEAR><<<grid, block, 0, s>>>(g, p, u, k0, out, c1, c_out, rho);
-      break;
-    case FORM4_BURGERS_EO: fv2d_tile<STAGE, BND, FORM4_BURGERS_EO><<<grid, block, 0, s>>>(g, p, u, k0, out, c1, c_out, rho); break;
-    case FORM4_TRANSPORT_EO:
-      fv2d_tile<STAGE, BND, FORM4_TRANSPORT_EO><<<grid, block, 0, s>>>(g, p, u, k0, out, c1, c_out, rho);
-      break;
-    case FORM4_BURGERS_UPWIND:
-      fv2d_tile<STAGE, BND, FORM4_BURGERS_UPWIND><<<grid, block, 0, s>>>(g, p, u, k0, out, c1, c_out, rho);
-      break;
-    default: fv2d_tile<STAGE, BND, FORM4_GENERIC><<<grid, block, 0, s>>>(g, p, u, k0, out, c1, c_out, rho); break;
+// whether the tiled kernels take the grid: at least two cells per direction (a cell that neighbours itself has no
+// flux) and, in 1D and 3D, where the generic kernel takes any batch, as many blocks as a launch can have
+bool tiled_ok(gdt_context ctx, const GridDesc& g, long long nbatch) {
+  for (int k = 0; k < g.dim; ++k)
+    if (g.n[k] < 2) return false;
+  if (g.dim == 1) return (g.n[0] + SX - 1) / SX * nbatch < (1LL << 31);
+  if (g.dim == 3) {
+    const int chunk = march_chunk(ctx, g, nbatch);
+    return (g.n[1] + MY - 1) / MY <= 65535 && (g.n[2] + chunk - 1) / chunk * nbatch <= 65535;
+  }
+  return true;
+}
+
+template <class... Args>
+void launch_serial(cudaStream_t s, void (*kernel)(Args...), dim3 grid, dim3 block, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = s;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+template <int STAGE, int FORM>
+void launch_form(gdt_context ctx, const GridDesc& g, const FvParams& p, const StageArgs& a, long long nbatch) {
+  cudaStream_t s = ctx->stream;
+  if (g.dim == 2) {
+    // Tiles of 32 rows compute 3 % of the faces twice, tiles of 8 rows 9 %, but a tile of 32 is 2 us of an SM's FP64
+    // pipe: below two of them per SM the small ones share the work out better (SSP-RK2 steps, 32 and 8 rows:
+    // 120 x 97 cells 17.0 and 12.8 us, 300 x 280 16.9 and 13.9, 512 x 500 21.1 and 21.0, 1000^2 47 and 50,
+    // 2048^2 167 and 196)
+    auto grid = [&](int rows) {
+      return dim3((unsigned)((g.n[0] + TX - 1) / TX), (unsigned)((g.n[1] + rows - 1) / rows), (unsigned)nbatch);
+    };
+    const dim3 tall = grid(32), flat = grid(8);
+    if ((long long)tall.x * tall.y * tall.z >= 2LL * ctx->num_sms || flat.y > 65535)
+      launch_serial(s, &fv2d_tile<STAGE, FORM, 32>, tall, dim3(TX, BY), g, p, a);
+    else launch_serial(s, &fv2d_tile<STAGE, FORM, 8>, flat, dim3(TX, BY), g, p, a);
+  } else if (g.dim == 1) {
+    launch_serial(s, &fv1d_segment<STAGE, FORM>, dim3((unsigned)((g.n[0] + SX - 1) / SX * nbatch)), dim3(SX), g, p, a);
+  } else {
+    const int chunk = march_chunk(ctx, g, nbatch);
+    const int chunks = (int)((g.n[2] + chunk - 1) / chunk);
+    const dim3 grid((unsigned)((g.n[0] + MX - 1) / MX), (unsigned)((g.n[1] + MY - 1) / MY), (unsigned)(nbatch * chunks));
+    launch_serial(s, &fv3d_march<STAGE, FORM>, grid, dim3(MX, MY), g, p, a, chunk, chunks);
   }
 }
 
-// one stage of the tiled 2D kernel, instantiated for the flux form and the boundary case
+// one stage of the tiled kernels, instantiated for the flux form
 template <int STAGE>
-void launch_tile(bool bnd, dim3 grid, cudaStream_t s, const GridDesc& g, const FvParams& p, const double* u,
-                 const double* k0, double* out, double c1, double c_out, double rho) {
-  if (bnd) launch_tile_b<STAGE, true>(grid, s, g, p, u, k0, out, c1, c_out, rho);
-  else launch_tile_b<STAGE, false>(grid, s, g, p, u, k0, out, c1, c_out, rho);
+void launch_stage(gdt_context ctx, const GridDesc& g, const FvParams& p, long long nbatch, const double* u,
+                  const double* k0, double* out, double c1, double c_out) {
+  StageArgs a;
+  a.u = u;
+  a.k0 = k0;
+  a.out = out;
+  a.c1 = c1;
+  a.c_out = c_out;
+  for (int k = 0; k < 3; ++k) a.rho[k] = k < g.dim ? g.h[0] / g.h[k] : 0.0;
+  switch (p.form4) {
+    case FORM4_BURGERS_LF: launch_form<STAGE, FORM4_BURGERS_LF>(ctx, g, p, a, nbatch); break;
+    case FORM4_BURGERS_LF_FIXED: launch_form<STAGE, FORM4_BURGERS_LF_FIXED>(ctx, g, p, a, nbatch); break;
+    case FORM4_BURGERS_EO: launch_form<STAGE, FORM4_BURGERS_EO>(ctx, g, p, a, nbatch); break;
+    case FORM4_BURGERS_UPWIND: launch_form<STAGE, FORM4_BURGERS_UPWIND>(ctx, g, p, a, nbatch); break;
+    case FORM4_TRANSPORT_LINEAR: launch_form<STAGE, FORM4_TRANSPORT_LINEAR>(ctx, g, p, a, nbatch); break;
+    default: launch_form<STAGE, FORM4_TRANSPORT_EO>(ctx, g, p, a, nbatch); break;
+  }
 }
-
-bool tiled_ok(const GridDesc& g) { return g.dim == 2 && g.n[0] >= 2 && g.n[1] >= 2; }
 
 }  // namespace
 
 gdt_status fv_apply(gdt_context ctx, const gdt_space_s& sp, const gdt_fv_desc* d, const double* u, double* out) {
   const GridDesc& g = sp.g;
   FvParams p = make_params(g, d);
-  if (tiled_ok(g)) {
-    dim3 grid((unsigned)((g.n[0] + TX - 1) / TX), (unsigned)((g.n[1] + TY - 1) / TY), 1);
-    // L(u) = K / (4 h_x), K = dx + (h_x / h_y) dy
-    launch_tile<0>(has_boundary(p, 2), grid, ctx->stream, g, p, u, nullptr, out, 0.0, 0.25 / g.h[0], g.h[0] / g.h[1]);
+  if (tiled_ok(ctx, g, 1)) {
+    launch_stage<0>(ctx, g, p, 1, u, nullptr, out, 0.0, 0.25 / g.h[0]);  // L(u) = K / (4 h_x)
   } else {
     fv_apply_kernel<<<grid_blocks(g.nelem, 256), 256, 0, ctx->stream>>>(g, p, 1, u, out, nullptr, 0.0, 0, nullptr,
                                                                         0.0);
@@ -463,23 +696,21 @@ gdt_status fv_timestep(gdt_context ctx, const gdt_space_s& sp, const gdt_fv_desc
   double* cur = u;
   double* nxt = (stepper == GDT_TIMESTEPPER_SSPRK2) ? work + N : work;
   double* k0 = work;
-  const bool tiled = tiled_ok(g);
-  const bool bnd = has_boundary(p, g.dim);
-  dim3 grid((unsigned)((g.n[0] + TX - 1) / TX), (unsigned)((g.n[1] + TY - 1) / TY), (unsigned)nbatch);
-  // the tiled kernels' update K = dx + rho dy with L(u) = K / (4 h_x): the stepper keeps K0 = K(u) itself
+  const bool tiled = tiled_ok(ctx, g, nbatch);
+  // the tiled kernels' update K with L(u) = K / (4 h_x): the stepper keeps K0 = K(u) itself
   // (k0 = L(u) = K0 / (4 h_x)) and folds the factor into its coefficients
-  const double rho = tiled ? g.h[0] / g.h[1] : 0.0, ck = 0.25 / g.h[0];
+  const double ck = 0.25 / g.h[0];
   for (long long st = 0; st < steps; ++st) {
     if (stepper == GDT_TIMESTEPPER_EXPLICIT_EULER) {
       if (tiled)
-        launch_tile<1>(bnd, grid, s, g, p, cur, nullptr, nxt, 0.0, -dt * ck, rho);
+        launch_stage<1>(ctx, g, p, nbatch, cur, nullptr, nxt, 0.0, -dt * ck);
       else
         fv_apply_kernel<<<grid_blocks(N, 256), 256, 0, s>>>(g, p, nbatch, cur, nullptr, nullptr, 0.0, 1, nxt, dt);
       ctx->launches++;
     } else {
       if (tiled) {
-        launch_tile<3>(bnd, grid, s, g, p, cur, nullptr, k0, 0.0, 1.0, rho);
-        launch_tile<2>(bnd, grid, s, g, p, cur, k0, nxt, -dt * ck, -0.5 * dt * ck, rho);
+        launch_stage<0>(ctx, g, p, nbatch, cur, nullptr, k0, 0.0, 1.0);
+        launch_stage<2>(ctx, g, p, nbatch, cur, k0, nxt, -dt * ck, -0.5 * dt * ck);
       } else {
         fv_apply_kernel<<<grid_blocks(N, 256), 256, 0, s>>>(g, p, nbatch, cur, k0, nullptr, 0.0, 0, nullptr, 0.0);
         fv_apply_kernel<<<grid_blocks(N, 256), 256, 0, s>>>(g, p, nbatch, nullptr, k0, cur, -dt, 2, nxt, -0.5 * dt);
