@@ -53,29 +53,25 @@ __device__ __forceinline__ double sum_strided(const double* v, int groups) {
   return b;
 }
 
-// Sum of v over the group, returned in all lanes of warp k for value k (k < NV); the first `warps` warps of the block
-// hold values. RELEASE: the block's writes before the call are visible to the group's blocks after
-// their next block barrier; without it only the order of their reads before the call and this block's
-// writes after it is kept. At most T blocks; the epoch counts the group's exchanges.
+// The group's sums of what the block's threads have stored in sh.part[k][32 g + lane] (k < NV, g < groups), returned in
+// all lanes of warp k for value k. RELEASE: the block's writes before the call are visible to the group's
+// blocks after their next block barrier; without it only the order of their reads before the call and
+// this block's writes after it is kept. At most T blocks; the epoch counts the group's exchanges.
 template <bool RELEASE, int NV, int T>
-__device__ __forceinline__ double group_exchange(const ExchangeView& ex, unsigned int& epoch, const double (&v)[NV],
-                                                 int warps, ExchangeShared<T>& sh) {
+__device__ __forceinline__ double exchange_stored(const ExchangeView& ex, unsigned int& epoch, int groups,
+                                                  ExchangeShared<T>& sh) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   ++epoch;
-  if (warp < warps) {
-#pragma unroll
-    for (int k = 0; k < NV; ++k) sh.part[k][threadIdx.x] = v[k];
-  }
   __syncthreads();
   if (ex.count == 1) {
-    const double b = warp < NV ? sum_strided(sh.part[warp] + lane, warps) : 0.0;
+    const double b = warp < NV ? sum_strided(sh.part[warp] + lane, groups) : 0.0;
     __syncthreads();  // part is free for the next exchange
     return b;
   }
   unsigned long long* const base = ex.slots + (size_t)kSlot * (gridDim.x * (epoch & 1u) + ex.first);
   const unsigned long long tag = (unsigned long long)epoch << 48;
   if (warp < NV) {
-    const double b = sum_strided(sh.part[warp] + lane, warps);
+    const double b = sum_strided(sh.part[warp] + lane, groups);
     if (lane == 0) sh.own[warp] = b;
     asm volatile("bar.sync 1, %0;" ::"n"(32 * NV) : "memory");
     if (threadIdx.x == 0) {
@@ -124,6 +120,33 @@ __device__ __forceinline__ double group_exchange(const ExchangeView& ex, unsigne
   }
   __syncthreads();
   return warp < NV ? sum_strided(sh.packet[warp] + lane, (ex.count + 31) >> 5) : 0.0;
+}
+
+// the same for one value per thread and k; the first `warps` warps of the block hold values
+template <bool RELEASE, int NV, int T>
+__device__ __forceinline__ double group_exchange(const ExchangeView& ex, unsigned int& epoch, const double (&v)[NV],
+                                                 int warps, ExchangeShared<T>& sh) {
+  if ((int)(threadIdx.x >> 5) < warps) {
+#pragma unroll
+    for (int k = 0; k < NV; ++k) sh.part[k][threadIdx.x] = v[k];
+  }
+  return exchange_stored<RELEASE, NV>(ex, epoch, warps, sh);
+}
+
+// the same for FP32 values, summed over a warp in FP32 (a few 1e-7, the precision of the vectors the products come
+// from) and from there in FP64. T is at most 1024.
+template <bool RELEASE, int NV, int T>
+__device__ __forceinline__ double group_exchange_f32(const ExchangeView& ex, unsigned int& epoch, float (&v)[NV],
+                                                     ExchangeShared<T>& sh) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+    if (lane == 0) sh.part[k][warp] = double(v[k]);
+    if (T < 1024 && warp == 0 && lane >= T / 32) sh.part[k][lane] = 0.0;
+  }
+  return exchange_stored<RELEASE, NV>(ex, epoch, 1, sh);
 }
 
 }  // namespace gdt

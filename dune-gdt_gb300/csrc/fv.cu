@@ -531,18 +531,19 @@ FvParams make_params(const GridDesc& g, const gdt_fv_desc* d) {
   return p;
 }
 
-// planes per block of fv3d_march: the chunk with the least work on the fullest SM, 13 FP64 instructions per cell of a
-// plane, four for the face and the squares a chunk computes besides, and its two plane loads before the
-// first face counted as six more (20 x 25 x 18 cells: 12.8 us a step with one plane, 29 with four; 60^3:
-// 32 us with one, 25 with two; 128 x 140 x 120: 158 us with eight, 176 with fourteen)
+// planes per block of fv3d_march: the chunk with the least work per SM, 13 FP64 instructions per cell of a plane, four
+// for the face and the squares a chunk computes besides, its two plane loads before the first face counted
+// as six more, and two chunks for what latency and the last wave leave idle (20 x 25 x 18 cells: 12.8 us a
+// step with one plane, 29 with four; 60^3: 32 us with one or four, 25 with two; 128 x 140 x 120: 158 us
+// with eight, 176 with fourteen)
 int march_chunk(gdt_context ctx, const GridDesc& g, long long nbatch) {
-  const long long tiles = ((g.n[0] + MX - 1) / MX) * ((g.n[1] + MY - 1) / MY) * nbatch;
-  long long best = 0;
+  const double tiles = double((g.n[0] + MX - 1) / MX) * double((g.n[1] + MY - 1) / MY) * double(nbatch);
+  double best = 0.0;
   int chosen = 1;
   for (int chunk = 1; chunk <= 16 && chunk <= g.n[2]; ++chunk) {
-    const long long blocks = tiles * ((g.n[2] + chunk - 1) / chunk);
-    const long long cost = (blocks + ctx->num_sms - 1) / ctx->num_sms * (13 * chunk + 10);
-    if (best == 0 || cost < best) best = cost, chosen = chunk;
+    const double blocks = tiles * double((g.n[2] + chunk - 1) / chunk);
+    const double cost = (blocks / ctx->num_sms + 2.0) * (13 * chunk + 10);
+    if (best == 0.0 || cost < best) best = cost, chosen = chunk;
   }
   return chosen;
 }

@@ -1227,6 +1227,14 @@ gdt_status solve(gdt_context ctx, gdt_matrix m, const double* b, double* x, cons
       return ms;
     }
   }
+  if (mixed && ctx->solver_launch != GDT_SOLVER_LAUNCH_GRAPH && !ctx->timing && mixed_stencil_supported(m)) {
+    // the other vertex stencils in one launch where the rows fit the registers of the grid
+    const gdt_status ms = solve_mixed_resident(ctx, m, b, x, o, info, s);
+    if (ms != GDT_EUNSUPPORTED) {
+      ctx->last_solver_launch = GDT_SOLVER_LAUNCH_PERSISTENT;
+      return ms;
+    }
+  }
   if (mixed && mixed_stencil_supported(m)) {
     ctx->last_solver_launch = GDT_SOLVER_LAUNCH_GRAPH;
     return solve_mixed_stencil(ctx, m, b, x, o, info, s);

@@ -119,8 +119,9 @@ gdt_status gdt_measure_l2_bandwidth(gdt_context ctx, double* gbs);
 #define GDT_SOLVER_LAUNCH_PERSISTENT 2
 gdt_status gdt_context_set_solver_launch(gdt_context ctx, int mode);
 /* launch form (GRAPH or PERSISTENT) of the context's last CG solve (FP64, or mixed precision: the 3D
- * Q1 matrix-free inner iterations run persistent under AUTO and PERSISTENT, the other mixed-precision
- * paths as graphs); 0 before the first */
+ * Q1 matrix-free inner iterations, and the other vertex stencils of up to 0.6 M rows (1.2 M with at most 15
+ * entries a row), run persistent under AUTO and PERSISTENT, the other mixed-precision paths as graphs); 0
+ * before the first */
 int gdt_context_last_solver_launch(gdt_context ctx);
 /* Limits of the persistent (cooperative) solver launches (no reference counterpart; diagnostics and
  * tests of the launch form): blocks caps the grid (0: one block per SM, the default), wait_limit_ns
