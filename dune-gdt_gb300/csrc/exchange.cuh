@@ -134,7 +134,7 @@ __device__ __forceinline__ double group_exchange(const ExchangeView& ex, unsigne
 }
 
 // the same for FP32 values, summed over a warp in FP32 (a few 1e-7, the precision of the vectors the products come
-// from) and from there in FP64. T is at most 1024.
+// from) and from there in FP64. The block may have more than T threads.
 template <bool RELEASE, int NV, int T>
 __device__ __forceinline__ double group_exchange_f32(const ExchangeView& ex, unsigned int& epoch, float (&v)[NV],
                                                      ExchangeShared<T>& sh) {
@@ -144,9 +144,51 @@ __device__ __forceinline__ double group_exchange_f32(const ExchangeView& ex, uns
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
     if (lane == 0) sh.part[k][warp] = double(v[k]);
-    if (T < 1024 && warp == 0 && lane >= T / 32) sh.part[k][lane] = 0.0;
+    if (warp == 0 && lane >= (int)(blockDim.x >> 5)) sh.part[k][lane] = 0.0;
   }
   return exchange_stored<RELEASE, NV>(ex, epoch, 1, sh);
+}
+
+// The barrier alone, releasing the block's writes; thread 0 runs `meanwhile` between its arrival and its wait.
+template <int T, class Meanwhile>
+__device__ __forceinline__ void group_barrier(const ExchangeView& ex, unsigned int& epoch, ExchangeShared<T>& sh,
+                                              Meanwhile meanwhile) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  ++epoch;
+  __syncthreads();
+  if (ex.count == 1) {
+    if (threadIdx.x == 0) meanwhile();
+    __syncthreads();
+    return;
+  }
+  unsigned long long* const base = ex.slots + (size_t)kSlot * (gridDim.x * (epoch & 1u) + ex.first);
+  const unsigned long long tag = (unsigned long long)epoch << 48;
+  if (threadIdx.x == 0) {
+    fence_acq_rel_gpu();
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(base + kSlot * (blockIdx.x - ex.first)), "l"(tag) : "memory");
+    meanwhile();
+  }
+  if (warp * 32 < ex.count) {
+    unsigned long long w = 0, t0 = 0;
+    bool wait = (int)threadIdx.x < ex.count;
+    for (unsigned int spins = 1;; ++spins) {
+      if (wait) {
+        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(base + kSlot * threadIdx.x) : "memory");
+        wait = ((w ^ tag) >> 48) != 0;
+      }
+      if (!__any_sync(0xffffffffu, wait)) break;
+      if (spins == 1u) t0 = global_ns();
+      else if (spins == 2u || (spins & 255u) == 0u) {
+        const bool out = spins > (1u << 24) || global_ns() - t0 > ex.wait_ns;
+        if (out) atomicExch(ex.fault, 1u);
+        if (__any_sync(0xffffffffu, out || *reinterpret_cast<volatile unsigned int*>(ex.fault) != 0u)) {
+          if (lane == 0) sh.fault = 1;
+          break;
+        }
+      }
+    }
+  }
+  __syncthreads();
 }
 
 }  // namespace gdt

@@ -31,7 +31,7 @@
 #include <cstring>
 #include <vector>
 
-#include "linalg.cuh"
+#include "exchange.cuh"
 
 namespace gdt {
 namespace {
@@ -54,8 +54,10 @@ struct MfState {
 
 __device__ __forceinline__ bool mf_stopped(const MfState* st) { return entry_flag(&st->converged) != 0; }
 
-// geometry of the padded layouts: vertex (x, y, z), -1 <= x <= nx, at (x + 1) + PX (y + 1) + PXY (z + 1);
-// cell (cx, cy, cz), -1 <= cx <= nx - 1, at (cx + 1) + CPX (cy + 1) + CPXY (cz + 1)
+// Layouts. The operator's input zb: vertex (x, y, z), -1 <= x <= nx, at (x + 1) + PX (y + 1) + PXY (z + 1); the
+// coefficients: cell (cx, cy, cz), -1 <= cx <= nx - 1, at (cx + 1) + CPX (cy + 1) + CPXY (cz + 1). Everything
+// else (p, s, x32, r, w, D_m) is read and written only by the thread that owns the row, and stored by item
+// (a vertex column's chunk of zlen planes): plane t of item i at t * items + i.
 struct Mf3 {
   int nx, ny, nz;
   int PX;
@@ -63,12 +65,17 @@ struct Mf3 {
   int CPX;
   long long CPXY;
   int ncol;      // nx * ny vertex columns
-  int chunks;    // z chunks per column in the operator pass
+  int chunks;    // z chunks per column
   int zlen;      // planes per chunk
+  int items;     // ncol * chunks
   float f[8];    // K_ref[i][j] = f[i ^ j]
-  __host__ __device__ long long vidx(long long v) const {
-    const long long x = v % nx, y = (v / nx) % ny, z = v / ((long long)nx * ny);
-    return (x + 1) + PX * (y + 1) + PXY * (z + 1);
+  __device__ int vidx(int v) const {
+    const int x = v % nx, y = (v / nx) % ny, z = v / ncol;
+    return (x + 1) + PX * (y + 1) + int(PXY) * (z + 1);
+  }
+  __device__ int pidx(int v) const {
+    const int c = v % ncol, z = v / ncol;
+    return z % zlen * items + z / zlen * ncol + c;
   }
 };
 
@@ -112,12 +119,14 @@ template <bool DIR>
 // plane's store; zb and r are read with plain coherent loads, never the read-only path: other blocks
 // wrote them before the last grid barrier)
 __device__ __forceinline__ void mf3_column(const Mf3& g, int x, int y, int z0, int z1, const float* __restrict__ kap,
-                                           const float* zb, const float* r, float* __restrict__ w, float& gam,
-                                           float& del, float& rr) {
+                                           const float* zb, const float* r, float* __restrict__ w, int item,
+                                           float& gam, float& del, float& rr) {
   const long long vb = (x + 1) + (long long)g.PX * (y + 1) + g.PXY;  // vertex (x, y, 0)
   const float* zc = zb + vb;
-  const float* rc = r + vb;
-  float* wc = w + vb;
+  // r and w of the item's rows, plane z at (z - z0) * items
+  const float* rc = r + item;
+  float* wc = w + item;
+  const int items = g.items;
   const float* kc = kap + x + (long long)g.CPX * y + g.CPXY;  // cell (x - 1, y - 1, 0)
   const long long PX = g.PX, PXY = g.PXY, CPX = g.CPX, CPXY = g.CPXY;
   const bool colbnd = DIR && (x == 0 || y == 0 || x == g.nx - 1 || y == g.ny - 1);
@@ -152,7 +161,7 @@ __device__ __forceinline__ void mf3_column(const Mf3& g, int x, int y, int z0, i
     load_layer(z0 - 1, km);
     load_plane(z0 + 1, P[1]);  // z0 < z1 <= nz: at most the padding plane nz
     load_layer(z0, K[0]);
-    rnext = rc[z0 * PXY];
+    rnext = rc[0];
     layer_sums(km, sm);
     carry = cross_of(f, plane_layer(pm, km, sm)) + same_of(f, plane_layer(P[0], km, sm));
   }
@@ -165,7 +174,7 @@ __device__ __forceinline__ void mf3_column(const Mf3& g, int x, int y, int z0, i
     if (z + 1 < z1) {  // the next step's operands: plane z + 2 <= z1 <= nz, layer z + 1 <= nz - 1
       load_plane(z + 2, P[(PH + 2) % 3]);
       load_layer(z + 1, K[(PH + 1) % 2]);
-      rnext = rc[(z + 1) * PXY];
+      rnext = rc[(z + 1 - z0) * items];
     }
     float sl[5];
     layer_sums(kl, sl);
@@ -177,7 +186,7 @@ __device__ __forceinline__ void mf3_column(const Mf3& g, int x, int y, int z0, i
       zv = rv;  // unit row: z = r (the diagonal is 1), w = z
       wv = rv;
     }
-    wc[z * PXY] = wv;
+    wc[(z - z0) * items] = wv;
     gam = fmaf(rv, zv, gam);
     del = fmaf(zv, wv, del);
     rr = fmaf(rv, rv, rr);
@@ -203,12 +212,11 @@ template <bool DIR>
 __device__ __forceinline__ void mf3_apply_items(const Mf3& g, const float* __restrict__ kap, const float* zb,
                                                 const float* r, float* __restrict__ w, float& gam, float& del,
                                                 float& rr) {
-  const long long items = (long long)g.ncol * g.chunks;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long it = blockIdx.x * (long long)blockDim.x + threadIdx.x; it < items; it += stride) {
-    const int c = int(it % g.ncol), k = int(it / g.ncol);
+  const int stride = gridDim.x * blockDim.x;
+  for (int it = blockIdx.x * blockDim.x + threadIdx.x; it < g.items; it += stride) {
+    const int c = it % g.ncol, k = it / g.ncol;
     const int z0 = k * g.zlen, z1 = min(g.nz, z0 + g.zlen);
-    mf3_column<DIR>(g, c % g.nx, c / g.nx, z0, z1, kap, zb, r, w, gam, del, rr);
+    mf3_column<DIR>(g, c % g.nx, c / g.nx, z0, z1, kap, zb, r, w, it, gam, del, rr);
   }
 }
 
@@ -217,9 +225,8 @@ enum { MF3_CONTINUE = 0, MF3_INIT = 1, MF3_REPLACE = 2 };
 
 struct MfPArgs {
   Mf3 g;
-  long long n4;  // float4 groups of the padded vertex arrays
   const float* kap;
-  const float* dm;  // D_m: Jacobi inverse diagonal (or 1), 0 on Dirichlet rows and in the padding
+  const float* dm;  // D_m: Jacobi inverse diagonal (or 1), 0 on Dirichlet rows
   float* p;
   float* s;
   float* x32;
@@ -227,25 +234,72 @@ struct MfPArgs {
   float* w;
   float* zb;
   MfState* st;
-  double* part;  // 3 * gridDim.x doubles
-  unsigned int* bar;
-  unsigned long long wait_ns;
-  int start;  // MF3_INIT / MF3_REPLACE: the first pass is the operator alone
+  ExchangeView ex;  // the whole grid
+  int start;        // MF3_INIT / MF3_REPLACE: the first pass is the operator alone
+  int shared;       // how many of s, p, x32 live in shared memory during the launch
 };
 
 // The solver scalars live in shared memory (thread 0 updates them after each reduction), so the
 // registers go to the operator's planes.
 struct MfScalars {
   double alpha, beta, gamma, gamma_prev, alpha_prev, rr;
+  double inv_gamma, inv_alpha;  // of gamma_prev and alpha_prev of the next iteration
+  double enough;                // |r|^2 at which the launch ends: replacement due, or the tolerance
+  double total[3];
   float af, bf;  // alpha and beta as the update pass uses them (one conversion, by thread 0)
-  int iter, done, flag, brk;
+  int iter, max_iter, done, flag, brk;
 };
 
-template <bool DIR>
-__global__ void __launch_bounds__(MT, 1) k_mf3_persistent(MfPArgs a) {
-  __shared__ double red[3 * 32];
-  __shared__ double bc[3];
+// p = z + beta p, s = w + beta s, x32 += alpha p, r -= alpha s, zb = D_m r of the thread's rows (z = D r: D_m, or 1
+// where D_m is 0 on a Dirichlet row). s, p and x32 of plane t at [t * step], from shared or global memory.
+template <int SH>
+__device__ __forceinline__ void mf3_update_items(const MfPArgs& a, float af, float bf, float* smem) {
+  const int stride = gridDim.x * blockDim.x, items = a.g.items;
+  int sbase = threadIdx.x;
+  for (int it = blockIdx.x * blockDim.x + threadIdx.x; it < items; it += stride) {
+    const int c = it % a.g.ncol, k = it / a.g.ncol;
+    const int len = min(a.g.zlen, a.g.nz - k * a.g.zlen);
+    const int per = a.g.zlen * MT * ((items + stride - 1) / stride);  // of one array in shared memory
+    float* zc = a.zb + (c % a.g.nx + 1) + (long long)a.g.PX * (c / a.g.nx + 1) + a.g.PXY * (k * a.g.zlen + 1);
+    auto at = [&](int var, float* g, int t) -> float& { return var < SH ? smem[var * per + sbase + t * MT] : g[t * items + it]; };
+    constexpr int U = 4;
+    auto rows = [&](int t0, auto n) {
+      constexpr int N = decltype(n)::value;
+      float r[N], w[N], d[N], s[N], p[N], x[N];
+#pragma unroll
+      for (int u = 0; u < N; ++u) {
+        const int i = (t0 + u) * items + it;
+        r[u] = a.r[i];
+        w[u] = a.w[i];
+        d[u] = __ldg(a.dm + i);
+        s[u] = at(0, a.s, t0 + u);
+        p[u] = at(1, a.p, t0 + u);
+        x[u] = at(2, a.x32, t0 + u);
+      }
+#pragma unroll
+      for (int u = 0; u < N; ++u) {
+        const float zt = d[u] != 0.f ? d[u] * r[u] : r[u];
+        const float pn = fmaf(bf, p[u], zt), sn = fmaf(bf, s[u], w[u]);
+        const float rn = fmaf(-af, sn, r[u]);
+        at(0, a.s, t0 + u) = sn;
+        at(1, a.p, t0 + u) = pn;
+        at(2, a.x32, t0 + u) = fmaf(af, pn, x[u]);
+        a.r[(t0 + u) * items + it] = rn;
+        zc[(t0 + u) * a.g.PXY] = d[u] * rn;
+      }
+    };
+    int t = 0;
+    for (; t + U <= len; t += U) rows(t, Ph<U>{});
+    for (; t < len; ++t) rows(t, Ph<1>{});
+    sbase += a.g.zlen * MT;
+  }
+}
+
+template <bool DIR, int SH>
+__global__ void __launch_bounds__(MT, 1) k_mf3_persistent(const __grid_constant__ MfPArgs a) {
+  __shared__ ExchangeShared<256> sh;
   __shared__ MfScalars sc;
+  extern __shared__ __align__(16) float mf_smem[];
   MfState* st = a.st;
   if (mf_stopped(st)) return;
   if (threadIdx.x == 0) {
@@ -256,102 +310,88 @@ __global__ void __launch_bounds__(MT, 1) k_mf3_persistent(MfPArgs a) {
     sc.alpha_prev = st->alpha_prev;
     sc.rr = st->rr;
     sc.iter = st->iter;
-    sc.af = float(sc.alpha);
-    sc.bf = float(sc.beta);
+    sc.max_iter = st->max_iter;
+    sc.enough = fmax(st->drop * st->rr_ref, st->tol2 * st->rr0);
+    sc.inv_gamma = a.start == MF3_REPLACE ? 1.0 / sc.gamma_prev : 0.0;
+    sc.inv_alpha = a.start == MF3_REPLACE ? 1.0 / sc.alpha_prev : 0.0;
     sc.done = sc.flag = sc.brk = 0;
+    sh.fault = 0;
   }
+  // s, p and x32 of the thread's rows to shared memory
+  const int stride = gridDim.x * blockDim.x, items = a.g.items;
+  const int per = a.g.zlen * MT * ((items + stride - 1) / stride);
+  auto exchange_rows = [&](bool in) {
+    float* const g[3] = {a.s, a.p, a.x32};
+    int sbase = threadIdx.x;
+    for (int it = blockIdx.x * blockDim.x + threadIdx.x; it < items; it += stride, sbase += a.g.zlen * MT) {
+      const int len = min(a.g.zlen, a.g.nz - it / a.g.ncol * a.g.zlen);
+#pragma unroll
+      for (int v = 0; v < SH; ++v)
+        for (int t = 0; t < len; ++t) {
+          float& own = mf_smem[v * per + sbase + t * MT];
+          if (in) own = g[v][t * items + it];
+          else g[v][t * items + it] = own;
+        }
+    }
+  };
+  exchange_rows(true);
   __syncthreads();
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   unsigned int epoch = 0;
   int pass = a.start;
   while (true) {
     if (pass == MF3_CONTINUE) {
-      // p = z + beta p, s = w + beta s, x32 += alpha p, r -= alpha s, zb = D_m r (z = D r: D_m, or 1 where
-      // D_m is 0 on a Dirichlet row; 0 in the padding, where r is 0)
-      const float af = sc.af, bf = sc.bf;
-      // (the written arrays restrict: the next group's loads may be issued before this group's stores)
-      float4* __restrict__ p4 = reinterpret_cast<float4*>(a.p);
-      float4* __restrict__ s4 = reinterpret_cast<float4*>(a.s);
-      float4* __restrict__ x4 = reinterpret_cast<float4*>(a.x32);
-      float4* __restrict__ r4 = reinterpret_cast<float4*>(a.r);
-      const float4* w4 = reinterpret_cast<const float4*>(a.w);
-      const float4* d4 = reinterpret_cast<const float4*>(a.dm);
-      float4* __restrict__ z4 = reinterpret_cast<float4*>(a.zb);
-      for (long long i = t0; i < a.n4; i += stride) {
-        float4 pv = p4[i], sv = s4[i], xv = x4[i], rv = r4[i];
-        const float4 wv = w4[i], dv = __ldg(d4 + i);
-        float* pp = &pv.x;
-        float* ss = &sv.x;
-        float* xx = &xv.x;
-        float* rr4 = &rv.x;
-        const float* ww = &wv.x;
-        const float* dd = &dv.x;
-        float zn[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const float zt = dd[u] != 0.f ? dd[u] * rr4[u] : rr4[u];
-          pp[u] = fmaf(bf, pp[u], zt);
-          ss[u] = fmaf(bf, ss[u], ww[u]);
-          xx[u] = fmaf(af, pp[u], xx[u]);
-          rr4[u] = fmaf(-af, ss[u], rr4[u]);
-          zn[u] = dd[u] * rr4[u];
-        }
-        p4[i] = pv;
-        s4[i] = sv;
-        x4[i] = xv;
-        r4[i] = rv;
-        z4[i] = make_float4(zn[0], zn[1], zn[2], zn[3]);
-      }
-      if (!grid_barrier(a.bar, epoch, a.wait_ns)) break;
+      mf3_update_items<SH>(a, sc.af, sc.bf, mf_smem);
+      // (zb is read by the neighbours; the reciprocals of the next scalars are formed while thread 0 waits)
+      group_barrier(a.ex, epoch, sh, [&] {
+        sc.inv_gamma = 1.0 / sc.gamma;
+        sc.inv_alpha = 1.0 / sc.alpha;
+      });
+      if (sh.fault) break;
     }
     // w = A zb and the three dots
-    float gs = 0.f, ds = 0.f, rs = 0.f;
-    mf3_apply_items<DIR>(a.g, a.kap, a.zb, a.r, a.w, gs, ds, rs);
-    float vf[3] = {gs, ds, rs};
-    double v[3];
-    block_reduce_f32<3>(vf, v, red);
-    if (threadIdx.x == 0) {
-      a.part[blockIdx.x] = v[0];
-      a.part[gridDim.x + blockIdx.x] = v[1];
-      a.part[2 * gridDim.x + blockIdx.x] = v[2];
-    }
-    if (!grid_barrier(a.bar, epoch, a.wait_ns)) break;
-    grid_allreduce<3>(a.part, v, bc);
-    if (threadIdx.x == 0) {
-      const double gam = v[0], del = v[1], rrn = v[2];
-      if (pass == MF3_INIT) {
-        sc.gamma_prev = gam;
-        sc.beta = 0.0;
-        sc.alpha = gam / del;
-        sc.alpha_prev = sc.alpha;
-      } else {
-        if (pass == MF3_CONTINUE) {
-          sc.gamma_prev = sc.gamma;
+    float vf[3] = {0.f, 0.f, 0.f};
+    mf3_apply_items<DIR>(a.g, a.kap, a.zb, a.r, a.w, vf[0], vf[1], vf[2]);
+    const double t = group_exchange_f32<false>(a.ex, epoch, vf, sh);
+    if (threadIdx.x < 96) {
+      if ((threadIdx.x & 31) == 0) sc.total[threadIdx.x >> 5] = t;
+      asm volatile("bar.sync 1, 96;" ::: "memory");
+      if (threadIdx.x == 0) {
+        const double gam = sc.total[0], del = sc.total[1], rrn = sc.total[2];
+        if (pass == MF3_INIT) {
+          sc.gamma_prev = gam;
+          sc.beta = 0.0;
+          sc.alpha = gam / del;
           sc.alpha_prev = sc.alpha;
+        } else {
+          if (pass == MF3_CONTINUE) {
+            sc.gamma_prev = sc.gamma;
+            sc.alpha_prev = sc.alpha;
+          }
+          sc.beta = (pass == MF3_REPLACE && st->restarting) ? 0.0 : gam * sc.inv_gamma;
+          sc.alpha = gam / fma(-sc.beta * gam, sc.inv_alpha, del);
         }
-        sc.beta = (pass == MF3_REPLACE && st->restarting) ? 0.0 : gam / sc.gamma_prev;
-        sc.alpha = gam / (del - sc.beta * gam / sc.alpha_prev);
-      }
-      sc.gamma = gam;
-      sc.af = float(sc.alpha);
-      sc.bf = float(sc.beta);
-      if (!(del > 0.0) || !isfinite(sc.alpha) || !isfinite(rrn)) {
-        sc.brk = 1;
-        sc.done = 1;
-      } else if (pass == MF3_CONTINUE) {
-        sc.iter += 1;
-        sc.rr = rrn;
-        if (rrn <= st->drop * st->rr_ref || rrn <= st->tol2 * st->rr0 || sc.iter >= st->max_iter) {
-          sc.flag = 1;
+        sc.gamma = gam;
+        sc.af = float(sc.alpha);
+        sc.bf = float(sc.beta);
+        if (!(del > 0.0) || !isfinite(sc.alpha) || !isfinite(rrn)) {
+          sc.brk = 1;
           sc.done = 1;
+        } else if (pass == MF3_CONTINUE) {
+          sc.iter += 1;
+          sc.rr = rrn;
+          if (rrn <= sc.enough || sc.iter >= sc.max_iter) {
+            sc.flag = 1;
+            sc.done = 1;
+          }
         }
+        if (sh.fault) sc.done = 1;
       }
     }
     __syncthreads();
     if (sc.done) break;
     pass = MF3_CONTINUE;
   }
+  exchange_rows(false);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     st->alpha = sc.alpha;
     st->beta = sc.beta;
@@ -378,8 +418,8 @@ __global__ void k_mf3_cells(Mf3 g, const float* __restrict__ kin, float* __restr
   }
 }
 
-__device__ __forceinline__ bool on_boundary(const Mf3& g, long long v) {
-  const long long x = v % g.nx, y = (v / g.nx) % g.ny, z = v / ((long long)g.nx * g.ny);
+__device__ __forceinline__ bool on_boundary(const Mf3& g, int v) {
+  const int x = v % g.nx, y = (v / g.nx) % g.ny, z = v / g.ncol;
   return x == 0 || y == 0 || z == 0 || x == g.nx - 1 || y == g.ny - 1 || z == g.nz - 1;
 }
 
@@ -391,7 +431,7 @@ __global__ void k_mf3_diag(int n, Mf3 g, const int* __restrict__ rp, const int* 
     if (jacobi)
       for (int k = rp[i]; k < rp[i + 1]; ++k)
         if (col[k] == i) d = val[k];
-    dm[g.vidx(i)] = (dir && on_boundary(g, i)) ? 0.f : float(1.0 / d);
+    dm[g.pidx(i)] = (dir && on_boundary(g, i)) ? 0.f : float(1.0 / d);
   }
 }
 
@@ -410,9 +450,8 @@ __global__ void k_mf3_probe(int n, Mf3 g, int dir, double* __restrict__ v64, flo
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const double v = mf3_probe_value(i);
     v64[i] = v;
-    const long long ip = g.vidx(i);
-    r32[ip] = float(v);
-    zb[ip] = (dir && on_boundary(g, i)) ? 0.f : float(v);
+    r32[g.pidx(i)] = float(v);
+    zb[g.vidx(i)] = (dir && on_boundary(g, i)) ? 0.f : float(v);
   }
 }
 
@@ -432,7 +471,7 @@ __global__ void __launch_bounds__(TH) k_mf3_compare(int n, Mf3 g, const int* __r
   float md = 0.f, my = 0.f;
   for_rows_csr<G, PL, double>(n, rp, col, val, v64, [&](int row, bool leader, double y) {
     if (leader) {
-      md = fmaxf(md, float(fabs(y - double(w[g.vidx(row)]))));
+      md = fmaxf(md, float(fabs(y - double(w[g.pidx(row)]))));
       my = fmaxf(my, float(fabs(y)));
     }
   });
@@ -452,7 +491,7 @@ __global__ void __launch_bounds__(TH) k_mf3_compare_sell(SellView A, Mf3 g, cons
   float md = 0.f, my = 0.f;
   for_slices(A, v64, [&](int row, bool active, double y, double) {
     if (active) {
-      md = fmaxf(md, float(fabs(y - double(w[g.vidx(row)]))));
+      md = fmaxf(md, float(fabs(y - double(w[g.pidx(row)]))));
       my = fmaxf(my, float(fabs(y)));
     }
   });
@@ -478,9 +517,9 @@ __global__ void __launch_bounds__(TH) k_mf3_init(int n, Mf3 g, const int* __rest
     if (leader) {
       const double ri = b[row] - s;
       const float rf = float(ri);
-      const long long ip = g.vidx(row);
+      const int ip = g.pidx(row);
       r32[ip] = rf;
-      zb[ip] = dm[ip] * rf;
+      zb[g.vidx(row)] = dm[ip] * rf;
       a1 = fma(ri, ri, a1);
     }
   });
@@ -503,7 +542,7 @@ __global__ void __launch_bounds__(TH) k_mf3_accumulate(int n, Mf3 g, double* __r
                                                       const MfState* st, int force) {
   if (!force && (mf_stopped(st) || !entry_flag(&st->flag))) return;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const long long ip = g.vidx(i);
+    const int ip = g.pidx(i);
     x[i] += double(x32[ip]);
     x32[ip] = 0.f;
   }
@@ -524,9 +563,9 @@ __global__ void __launch_bounds__(TH) k_mf3_true_residual(int n, Mf3 g, const in
     if (leader) {
       const double ri = b[row] - s;
       const float rf = float(ri);
-      const long long ip = g.vidx(row);
+      const int ip = g.pidx(row);
       r32[ip] = rf;
-      zb[ip] = dm[ip] * rf;
+      zb[g.vidx(row)] = dm[ip] * rf;
       a1 = fma(ri, ri, a1);
     }
   });
@@ -563,9 +602,9 @@ __global__ void __launch_bounds__(TH) k_mf3_init_sell(SellView A, Mf3 g, const d
     if (active) {
       const double ri = b[row] - s;
       const float rf = float(ri);
-      const long long ip = g.vidx(row);
+      const int ip = g.pidx(row);
       r32[ip] = rf;
-      zb[ip] = dm[ip] * rf;
+      zb[g.vidx(row)] = dm[ip] * rf;
       a1 = fma(ri, ri, a1);
     }
   });
@@ -593,9 +632,9 @@ __global__ void __launch_bounds__(TH) k_mf3_true_residual_sell(SellView A, Mf3 g
     if (active) {
       const double ri = b[row] - s;
       const float rf = float(ri);
-      const long long ip = g.vidx(row);
+      const int ip = g.pidx(row);
       r32[ip] = rf;
-      zb[ip] = dm[ip] * rf;
+      zb[g.vidx(row)] = dm[ip] * rf;
       a1 = fma(ri, ri, a1);
     }
   });
@@ -653,8 +692,6 @@ gdt_status solve_mixed_mf(gdt_context ctx, gdt_matrix m, const double* b, double
   g.CPXY = (long long)g.CPX * (g.ny + 1);
   g.ncol = g.nx * g.ny;
   if (!xor_structure(m->mf_K, g.f)) return GDT_EUNSUPPORTED;
-  const long long nv = g.PXY * (g.nz + 2);
-  const long long ntot = (nv + 3) / 4 * 4;
   const long long ctot = g.CPXY * (g.nz + 1);
   const bool dir = m->mf_dirichlet != 0;
   const int vec_blocks = std::max(1, std::min(grid_blocks(n, TH), ctx->num_sms * 8));
@@ -662,21 +699,34 @@ gdt_status solve_mixed_mf(gdt_context ctx, gdt_matrix m, const double* b, double
   unsigned int* ticket = ctx->counters;
 
   // persistent launch shape: one block of MT threads per SM (co-resident: cooperative launch)
-  const void* fn = dir ? reinterpret_cast<const void*>(&k_mf3_persistent<true>)
-                       : reinterpret_cast<const void*>(&k_mf3_persistent<false>);
-  int dev = 0, coop = 0, per_sm = 0;
-  GDT_TRY_CUDA(ctx, cudaGetDevice(&dev));
-  GDT_TRY_CUDA(ctx, cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-  GDT_TRY_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, MT, 0));
-  if (!coop || per_sm < 1) return GDT_EUNSUPPORTED;
-  int blocks = ctx->num_sms;
+  int coop = 0, per_sm = 0, optin = 0;
+  GDT_TRY_CUDA(ctx, cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device));
+  GDT_TRY_CUDA(ctx, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+  if (!coop) return GDT_EUNSUPPORTED;
+  int blocks = std::min(ctx->num_sms, 256);
   if (ctx->persistent_blocks > 0) blocks = std::min(blocks, ctx->persistent_blocks);
-  if (3 * blocks > kScratchDoubles / 2) return GDT_EUNSUPPORTED;
   // (column, z chunk) items: about one per thread
   const long long threads = (long long)blocks * MT;
   g.chunks = int(std::max(1LL, std::min<long long>(g.nz, threads / g.ncol)));
   g.zlen = (g.nz + g.chunks - 1) / g.chunks;
   g.chunks = (g.nz + g.zlen - 1) / g.zlen;
+  if ((long long)g.ncol * g.chunks * g.zlen >= (1LL << 31)) return GDT_EUNSUPPORTED;
+  g.items = g.ncol * g.chunks;
+  // as many of s, p and x32 in shared memory as fit
+  const long long per = 4LL * g.zlen * MT * ((g.items + threads - 1) / threads);
+  const void* const fns[2][4] = {
+      {reinterpret_cast<const void*>(&k_mf3_persistent<false, 0>), reinterpret_cast<const void*>(&k_mf3_persistent<false, 1>),
+       reinterpret_cast<const void*>(&k_mf3_persistent<false, 2>), reinterpret_cast<const void*>(&k_mf3_persistent<false, 3>)},
+      {reinterpret_cast<const void*>(&k_mf3_persistent<true, 0>), reinterpret_cast<const void*>(&k_mf3_persistent<true, 1>),
+       reinterpret_cast<const void*>(&k_mf3_persistent<true, 2>), reinterpret_cast<const void*>(&k_mf3_persistent<true, 3>)}};
+  cudaFuncAttributes fa;
+  GDT_TRY_CUDA(ctx, cudaFuncGetAttributes(&fa, fns[dir][3]));
+  const int shared = int(std::min(3LL, (optin - (long long)fa.sharedSizeBytes) / per));
+  const void* fn = fns[dir][shared];
+  const size_t dyn = size_t(shared * per);
+  GDT_TRY_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(dyn)));
+  GDT_TRY_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, MT, dyn));
+  if (per_sm < 1) return GDT_EUNSUPPORTED;
 
   std::vector<void*> allocs;
   struct Freer {
@@ -692,13 +742,13 @@ gdt_status solve_mixed_mf(gdt_context ctx, gdt_matrix m, const double* b, double
     allocs.push_back(p);
     return reinterpret_cast<void*>((reinterpret_cast<uintptr_t>(p) + 255) & ~uintptr_t(255));
   };
-  const size_t vb = sizeof(float) * ntot;
+  const size_t vb = sizeof(float) * size_t(g.items) * g.zlen, zbytes = sizeof(float) * size_t(g.PXY) * (g.nz + 2);
   float* p = (float*)alloc(vb);
   float* sv = (float*)alloc(vb);
   float* x32 = (float*)alloc(vb);
   float* r32 = (float*)alloc(vb);
   float* w = (float*)alloc(vb);
-  float* zb = (float*)alloc(vb);
+  float* zb = (float*)alloc(zbytes);
   float* dm = (float*)alloc(vb);
   float* kap = (float*)alloc(sizeof(float) * ctot);
   double* v64 = (double*)alloc(sizeof(double) * n);
@@ -706,7 +756,8 @@ gdt_status solve_mixed_mf(gdt_context ctx, gdt_matrix m, const double* b, double
   MfState* st = (MfState*)alloc(sizeof(MfState));
   if (!p || !sv || !x32 || !r32 || !w || !zb || !dm || !kap || !v64 || !err || !st)
     return fail(ctx, GDT_ENOMEM, "mixed solver vectors");
-  for (float* v : {p, sv, x32, r32, w, zb, dm}) GDT_TRY_CUDA(ctx, cudaMemsetAsync(v, 0, vb, s));
+  for (float* v : {p, sv, x32}) GDT_TRY_CUDA(ctx, cudaMemsetAsync(v, 0, vb, s));
+  GDT_TRY_CUDA(ctx, cudaMemsetAsync(zb, 0, zbytes, s));
   GDT_TRY_CUDA(ctx, cudaMemsetAsync(kap, 0, sizeof(float) * ctot, s));
   GDT_TRY_CUDA(ctx, cudaMemsetAsync(err, 0, 2 * sizeof(unsigned int), s));
   MfState init{};
@@ -745,7 +796,6 @@ gdt_status solve_mixed_mf(gdt_context ctx, gdt_matrix m, const double* b, double
     std::memcpy(&ed, &herr[0], sizeof(float));
     std::memcpy(&ey, &herr[1], sizeof(float));
     if (!(ey > 0.f) || !std::isfinite(ed) || ed > 1e-4f * ey) return GDT_EUNSUPPORTED;
-    for (float* v : {r32, zb, w}) GDT_TRY_CUDA(ctx, cudaMemsetAsync(v, 0, vb, s));
   }
   const int sblocks_init =
       sell ? sell_blocks(SA.nslices, ctx->num_sms, reinterpret_cast<const void*>(&k_mf3_init_sell)) : 0;
@@ -762,7 +812,6 @@ gdt_status solve_mixed_mf(gdt_context ctx, gdt_matrix m, const double* b, double
 
   MfPArgs a{};
   a.g = g;
-  a.n4 = ntot / 4;
   a.kap = kap;
   a.dm = dm;
   a.p = p;
@@ -772,9 +821,16 @@ gdt_status solve_mixed_mf(gdt_context ctx, gdt_matrix m, const double* b, double
   a.w = w;
   a.zb = zb;
   a.st = st;
-  a.part = ctx->scratch;
-  a.bar = reinterpret_cast<unsigned int*>(ctx->scratch + kScratchDoubles / 2);
-  a.wait_ns = ctx->persistent_wait_ns > 0 ? (unsigned long long)ctx->persistent_wait_ns : kBarrierNs;
+  // fault flag and packets in the upper half of the scratch (kernels of the setup use its start)
+  unsigned long long* const words = reinterpret_cast<unsigned long long*>(ctx->scratch + kScratchDoubles / 2);
+  const size_t packets = size_t(2 * kSlot) * blocks;
+  static_assert(2 * kSlot * 256 + 16 <= kScratchDoubles / 2, "the packets fit the scratch");
+  a.ex.fault = reinterpret_cast<unsigned int*>(words);
+  a.ex.slots = words + 16;
+  a.ex.first = 0;
+  a.ex.count = blocks;
+  a.ex.wait_ns = ctx->persistent_wait_ns > 0 ? (unsigned long long)ctx->persistent_wait_ns : kBarrierNs;
+  a.shared = shared;
   MfState fin{};
   unsigned int fault = 0;
   int cycles = 0;
@@ -784,15 +840,14 @@ gdt_status solve_mixed_mf(gdt_context ctx, gdt_matrix m, const double* b, double
   // cleared once per solve: a barrier wait that runs out in any cycle stays visible, and the group's
   // remaining launches leave at their first barrier.
   constexpr int kCyclesPerCheck = 4;
-  GDT_TRY_CUDA(ctx, cudaMemsetAsync(a.bar + kBarFault, 0, sizeof(unsigned int), s));
+  GDT_TRY_CUDA(ctx, cudaMemsetAsync(a.ex.fault, 0, sizeof(unsigned int), s));
   while (cycles < 100000) {
     for (int k = 0; k < kCyclesPerCheck && cycles < 100000; ++k, ++cycles) {
       a.start = cycles == 0 ? MF3_INIT : MF3_REPLACE;
-      GDT_TRY_CUDA(ctx, cudaMemsetAsync(a.bar, 0, sizeof(unsigned long long), s));
-      GDT_TRY_CUDA(ctx, cudaMemsetAsync(a.bar + kBarGen, 0, sizeof(unsigned int), s));
+      GDT_TRY_CUDA(ctx, cudaMemsetAsync(a.ex.slots, 0, sizeof(unsigned long long) * packets, s));
       void* args[] = {&a};
       timing_begin(ctx, s, GDT_TIMING_MIXED_PERSISTENT);
-      const cudaError_t le = cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(MT), args, 0, s);
+      const cudaError_t le = cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(MT), args, dyn, s);
       timing_end(ctx, s);
       GDT_TRY_CUDA(ctx, le);
       ctx->launches++;
@@ -809,7 +864,7 @@ gdt_status solve_mixed_mf(gdt_context ctx, gdt_matrix m, const double* b, double
       ctx->launches += 2;
     }
     GDT_TRY_CUDA(ctx, cudaMemcpyAsync(&fin, st, sizeof(MfState), cudaMemcpyDeviceToHost, s));
-    GDT_TRY_CUDA(ctx, cudaMemcpyAsync(&fault, a.bar + kBarFault, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
+    GDT_TRY_CUDA(ctx, cudaMemcpyAsync(&fault, a.ex.fault, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
     GDT_TRY_CUDA(ctx, cudaStreamSynchronize(s));
     if (ctx->timing) timing_harvest(ctx);
     if (fault) return fail(ctx, GDT_ECUDA, "persistent mixed solver: a grid barrier wait ran out");
