@@ -49,10 +49,43 @@ constexpr double kReplaceDrop2 = 1e-2;
 struct MfState {
   double alpha, beta, gamma, gamma_prev, alpha_prev;
   double rr, rr0, rr_ref, tol2, drop;
-  int iter, max_iter, converged, flag, breakdown, updates, restarting, replaced_iter;
+  double aim;  // |r|^2 at which the iterated residual ends the solve
+  int iter, max_iter, converged, flag, breakdown, updates, restarting, replaced_iter, misses, fresh;
 };
 
 __device__ __forceinline__ bool mf_stopped(const MfState* st) { return entry_flag(&st->converged) != 0; }
+
+// After a replacement, rr the square of the true residual. Its difference to the iterated one is the rounding of
+// x64, about the same after every replacement, so where that is not small beside the tolerance the
+// iterated residual aims lower, by 1.5 of it and at most to half the tolerance. A true residual that
+// misses the tolerance all the same restarts the direction once (the recurrence for alpha does not
+// survive a replacement as large as the residual itself: at 128^3 and a tolerance 1.3 times the floor the
+// iteration stagnated without) and aims for half of that. Otherwise a cycle that gained less than 2x on the
+// true residual means that the FP32 operator is too far from the FP64 one for the sequence to continue;
+// from then on each replacement restarts the direction and waits for a 1000x drop (restarted FP64
+// refinement around FP32 CG).
+__device__ __forceinline__ void mf3_replaced(MfState* st, double rr) {
+  const double tol = st->tol2 * st->rr0;
+  const bool missed = rr > tol && st->rr <= st->aim && !st->restarting && st->misses < 3;
+  st->misses += missed ? 1 : 0;
+  if (!missed && !st->restarting && rr > 0.25 * st->rr_ref) {
+    st->restarting = 1;
+    st->drop = 1e-6;
+  }
+  st->fresh = missed || st->restarting;
+  const double cut = st->misses == 0 ? 1.0 : st->misses == 1 ? 0.25 : st->misses == 2 ? 0.0625 : 0.015625;
+  st->aim = cut * fmax(0.25 * tol, tol - 1.5 * fmax(rr - st->rr, 0.0));
+  st->rr_ref = rr;
+  st->rr = rr;
+  st->flag = 0;
+  st->updates += 1;
+  st->replaced_iter = st->iter;
+  if (rr <= st->tol2 * st->rr0 || st->iter >= st->max_iter) st->converged = 1;
+  if (!isfinite(rr)) {
+    st->breakdown = 1;
+    st->converged = 1;
+  }
+}
 
 // Layouts. The operator's input zb: vertex (x, y, z), -1 <= x <= nx, at (x + 1) + PX (y + 1) + PXY (z + 1); the
 // coefficients: cell (cx, cy, cz), -1 <= cx <= nx - 1, at (cx + 1) + CPX (cy + 1) + CPXY (cz + 1). Everything
@@ -311,7 +344,8 @@ __global__ void __launch_bounds__(MT, 1) k_mf3_persistent(const __grid_constant_
     sc.rr = st->rr;
     sc.iter = st->iter;
     sc.max_iter = st->max_iter;
-    sc.enough = fmax(st->drop * st->rr_ref, st->tol2 * st->rr0);
+    // a replacement less than 4x above the tolerance would be followed by another one at it
+    sc.enough = st->drop * st->rr_ref > 16.0 * st->aim ? st->drop * st->rr_ref : st->aim;
     sc.inv_gamma = a.start == MF3_REPLACE ? 1.0 / sc.gamma_prev : 0.0;
     sc.inv_alpha = a.start == MF3_REPLACE ? 1.0 / sc.alpha_prev : 0.0;
     sc.done = sc.flag = sc.brk = 0;
@@ -367,7 +401,7 @@ __global__ void __launch_bounds__(MT, 1) k_mf3_persistent(const __grid_constant_
             sc.gamma_prev = sc.gamma;
             sc.alpha_prev = sc.alpha;
           }
-          sc.beta = (pass == MF3_REPLACE && st->restarting) ? 0.0 : gam * sc.inv_gamma;
+          sc.beta = (pass == MF3_REPLACE && st->fresh) ? 0.0 : gam * sc.inv_gamma;
           sc.alpha = gam / fma(-sc.beta * gam, sc.inv_alpha, del);
         }
         sc.gamma = gam;
@@ -528,6 +562,9 @@ __global__ void __launch_bounds__(TH) k_mf3_init(int n, Mf3 g, const int* __rest
     st->rr = st->rr0 = st->rr_ref = v[0];
     st->drop = kReplaceDrop2;
     st->restarting = 0;
+    st->aim = st->tol2 * v[0];
+    st->misses = 0;
+    st->fresh = 0;
     st->replaced_iter = -1;
     st->iter = 0;
     st->flag = 0;
@@ -571,23 +608,7 @@ __global__ void __launch_bounds__(TH) k_mf3_true_residual(int n, Mf3 g, const in
   });
   double v[1] = {a1};
   if (grid_reduce<1>(v, partials, ticket) && threadIdx.x == 0) {
-    // stagnation guard: a cycle that gained less than 2x on the true residual means the FP32 operator
-    // is too far from the FP64 one for the sequence to continue; from then on each replacement
-    // restarts the direction and waits for a 1000x drop (restarted FP64 refinement around FP32 CG)
-    if (!st->restarting && v[0] > 0.25 * st->rr_ref) {
-      st->restarting = 1;
-      st->drop = 1e-6;
-    }
-    st->rr_ref = v[0];
-    st->rr = v[0];
-    st->flag = 0;
-    st->updates += 1;
-    st->replaced_iter = st->iter;
-    if (v[0] <= st->tol2 * st->rr0 || st->iter >= st->max_iter) st->converged = 1;
-    if (!isfinite(v[0])) {
-      st->breakdown = 1;
-      st->converged = 1;
-    }
+    mf3_replaced(st, v[0]);
   }
 }
 
@@ -613,6 +634,9 @@ __global__ void __launch_bounds__(TH) k_mf3_init_sell(SellView A, Mf3 g, const d
     st->rr = st->rr0 = st->rr_ref = v[0];
     st->drop = kReplaceDrop2;
     st->restarting = 0;
+    st->aim = st->tol2 * v[0];
+    st->misses = 0;
+    st->fresh = 0;
     st->replaced_iter = -1;
     st->iter = 0;
     st->flag = 0;
@@ -640,20 +664,7 @@ __global__ void __launch_bounds__(TH) k_mf3_true_residual_sell(SellView A, Mf3 g
   });
   double v[1] = {a1};
   if (grid_reduce<1>(v, partials, ticket) && threadIdx.x == 0) {
-    if (!st->restarting && v[0] > 0.25 * st->rr_ref) {
-      st->restarting = 1;
-      st->drop = 1e-6;
-    }
-    st->rr_ref = v[0];
-    st->rr = v[0];
-    st->flag = 0;
-    st->updates += 1;
-    st->replaced_iter = st->iter;
-    if (v[0] <= st->tol2 * st->rr0 || st->iter >= st->max_iter) st->converged = 1;
-    if (!isfinite(v[0])) {
-      st->breakdown = 1;
-      st->converged = 1;
-    }
+    mf3_replaced(st, v[0]);
   }
 }
 
