@@ -113,6 +113,10 @@ struct gdt_matrix_s {
   long long val_version = 0;    // bumped by every entry point that may change the values
   long long sell_version = -1;  // val_version the SELL copy was filled at
   int use_sell = 0;             // plain SpMV and the graph-form CG SpMV read the SELL copy (tuned or pinned)
+  // products with changed values read the CSR arrays until what the copy would have saved has paid its fill
+  int csr_products = 0;         // how many (0: fill at once), timed by the tuner
+  int csr_done = 0;             // products with the values of csr_version so far
+  long long csr_version = -1;
   float mf_K[64] = {};
   int mf_valid = 0;      // the values are exactly that assembly (cleared by any other value change)
   int mf_dirichlet = 0;  // with Dirichlet unit rows and columns
@@ -125,8 +129,6 @@ constexpr int kScratchDoubles = 1 << 16;
 constexpr int kCounters = 64;
 
 gdt_status fail(gdt_context ctx, gdt_status s, const std::string& msg);
-// keeps the element coefficients of a 3D Q1 Laplace assembly for the matrix-free FP32 operator
-gdt_status mf_capture(gdt_context ctx, gdt_matrix m, const gdt_diffusion_desc* d);
 gdt_status check_launch(gdt_context ctx, const char* what);
 
 #define GDT_TRY_CUDA(ctx, call)                                                                   \

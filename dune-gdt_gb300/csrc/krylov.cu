@@ -754,18 +754,6 @@ __device__ __forceinline__ void pcg_publish(const PcgArgs& a, unsigned int& epoc
   if (threadIdx.x < 64 && (threadIdx.x & 31) == 0) sh.last[threadIdx.x >> 5] = total;
 }
 
-// s += v[J] p[J] + ... + v[cnt - 1] p[cnt - 1] (cnt warp-uniform). A predicated-off FP64 instruction takes its 64 cycles
-// like any other (measured: a masked second row doubled a pass), hence nested branches, not masks.
-template <int J, int CH>
-__device__ __forceinline__ void fma_chain(int cnt, const double (&v)[CH], const double (&p)[CH], double& s) {
-  if constexpr (J < CH) {
-    if (cnt > J) {
-      s = fma(v[J], p[J], s);
-      fma_chain<J + 1>(cnt, v, p, s);
-    }
-  }
-}
-
 // sum of a row's products, entries t of the lane's row at v[32 t], c[32 t]; w is warp-uniform. All loads of
 // CH entries are issued before their FMAs. One accumulator: with 16 or more warps on the SM each
 // warp's turn at the FP64 pipe comes after the FMA's latency, and a second one would cost an add.

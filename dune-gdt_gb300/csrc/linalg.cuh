@@ -129,17 +129,33 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// Asynchronous double-buffered warp staging: each warp owns 32 consecutive rows per step. While it
-// reduces the current slice from one shared-memory buffer, the next slice (values and indices,
-// rounded out to 16-byte boundaries; the CSR arrays carry padding) is already being copied into the
-// other buffer with cp.async. Lane i reduces row r0 + i: one lane per row, so the FP64 instructions
-// per row are the row's FMAs only (no shuffle reductions). Rows of at most CAP entries.
+// s += v[J] p[J] + ... + v[cnt - 1] p[cnt - 1] (cnt warp-uniform). A predicated-off FP64 instruction takes its 64 cycles
+// like any other (measured: a masked second row doubled a pass), hence nested branches, not masks.
+template <int J, int CH, class T>
+__device__ __forceinline__ void fma_chain(int cnt, const T (&v)[CH], const T (&p)[CH], T& s) {
+  if constexpr (J < CH) {
+    if (cnt > J) {
+      s = fma(v[J], p[J], s);
+      fma_chain<J + 1>(cnt, v, p, s);
+    }
+  }
+}
+
+// Asynchronous warp staging: a warp owns 32 consecutive rows per step and copies their contiguous slice of the
+// values and indices (rounded out to 16-byte boundaries; the CSR arrays carry padding) to its buffer with
+// cp.async; lane i then reduces row r0 + i. One lane per row, so the FP64 instructions of a row are its FMAs
+// only (G lanes per row add log2 G shuffled sums to 27 / G FMAs each), and the gathers of nine are in flight. One
+// buffer per warp: 20 warps per SM hide the copies and the gathers behind each other's FMAs, where two
+// buffers leave room for 10 warps (128^3 Q1: 250 us with two, two sums and the gathers behind
+// branches, 151 like this; 97 x 102 x 91 rows 109 and 70; P1 113 x 101 x 106 rows 109 and 56). One sum
+// instead of three, or the next nine gathers ahead of the products, measured the same or slower.
+// Rows of at most CAP entries.
 template <class T, int CAP>
 struct AsyncWindow {
   static constexpr int VE = 16 / sizeof(T);            // values per 16-byte chunk
-  static constexpr int VCAP = 32 * CAP + 2 * VE;       // values per buffer (slack for alignment)
-  static constexpr int CCAP = 32 * CAP + 8;            // indices per buffer
-  static constexpr size_t bytes_per_warp = 2 * (VCAP * sizeof(T) + CCAP * sizeof(int));
+  static constexpr int VCAP = 32 * CAP + 2 * VE;       // values (slack for alignment)
+  static constexpr int CCAP = 32 * CAP + 8;            // indices
+  static constexpr size_t bytes_per_warp = VCAP * sizeof(T) + CCAP * sizeof(int);
 };
 
 template <class T, int CAP, bool HASW = false, class Body>
@@ -149,58 +165,53 @@ __device__ __forceinline__ void for_rows_async(int n, const int* __restrict__ rp
   using W = AsyncWindow<T, CAP>;
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-  unsigned char* const base = gdt_dyn_smem + warp * W::bytes_per_warp;
-  auto vbuf = [&](int b) { return reinterpret_cast<T*>(base + b * (W::VCAP * sizeof(T))); };
-  auto cbuf = [&](int b) {
-    return reinterpret_cast<int*>(base + 2 * W::VCAP * sizeof(T) + b * (W::CCAP * sizeof(int)));
-  };
+  T* const vbuf = reinterpret_cast<T*>(gdt_dyn_smem + warp * W::bytes_per_warp);
+  int* const cbuf = reinterpret_cast<int*>(vbuf + W::VCAP);
   const int step = gridDim.x * wpb * 32;
-  // stage the slice of rows [r, r+32) into buffer b; returns this lane's row bounds and the slice's
-  // aligned (value, index) start offsets. Warp-uniform: every lane calls it.
-  auto stage = [&](int r, int b, int& rbeg, int& rend, int& vb, int& cb) {
-    const int row = r + lane;
-    rbeg = row < n ? rp[row] : 0;
-    rend = row < n ? rp[row + 1] : 0;
-    const int last = (n - 1 - r) < 31 ? (n - 1 - r) : 31;
-    const int beg = __shfl_sync(0xffffffffu, rbeg, 0);
-    const int end = __shfl_sync(0xffffffffu, rend, last);
-    vb = beg & ~(W::VE - 1);
-    cb = beg & ~3;
-    const int nv = (end - vb + W::VE - 1) / W::VE, nc = (end - cb + 3) / 4;
-    T* dv = vbuf(b);
-    int* dc = cbuf(b);
-    for (int k = lane; k < nv; k += 32) cp_async16(dv + k * W::VE, val + vb + k * W::VE);
-    for (int k = lane; k < nc; k += 32) cp_async16(dc + k * 4, col + cb + k * 4);
-    cp_async_commit();
-  };
   int r0 = (blockIdx.x * wpb + warp) * 32;
-  int rb = 0, re = 0, vb = 0, cb = 0, cur = 0;
-  if (r0 < n) stage(r0, 0, rb, re, vb, cb);
-  for (; r0 < n; r0 += step, cur ^= 1) {
-    const bool more = r0 + step < n;
-    int rb2 = 0, re2 = 0, vb2 = 0, cb2 = 0;
-    if (more) {
-      stage(r0 + step, cur ^ 1, rb2, re2, vb2, cb2);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
+  int rb = r0 + lane < n ? rp[r0 + lane] : 0, re = r0 + lane < n ? rp[r0 + lane + 1] : 0;
+  for (; r0 < n; r0 += step) {
     const int row = r0 + lane;
     const bool active = row < n;
+    const int last = (n - 1 - r0) < 31 ? (n - 1 - r0) : 31;
+    const int beg = __shfl_sync(0xffffffffu, rb, 0);
+    const int end = __shfl_sync(0xffffffffu, re, last);
+    const int vb = beg & ~(W::VE - 1), cb = beg & ~3;
+    const int nv = (end - vb + W::VE - 1) / W::VE, nc = (end - cb + 3) / 4;
+    for (int k = lane; k < nc; k += 32) cp_async16(cbuf + k * 4, col + cb + k * 4);
+    for (int k = lane; k < nv; k += 32) cp_async16(vbuf + k * W::VE, val + vb + k * W::VE);
+    cp_async_commit();
+    // the next slice's row bounds while this one is copied
+    const int next = row + step;
+    const int rb2 = next < n ? rp[next] : 0, re2 = next < n ? rp[next + 1] : 0;
     const T wr = (HASW && active) ? w[row] : T(0);
+    cp_async_wait<0>();
     __syncwarp();
-    const T* wv = vbuf(cur) + (rb - vb);
-    const int* wc = cbuf(cur) + (rb - cb);
-    const int len = re - rb;
-    T s0 = T(0), s1 = T(0);
+    const T* wv = vbuf + (rb - vb);
+    const int* wc = cbuf + (rb - cb);
+    const int len = re - rb, width = __reduce_max_sync(0xffffffffu, len);
+    T s0 = T(0), s1 = T(0), s2 = T(0);
+    int t = 0;
+    for (; t + 9 <= width; t += 9) {
+      T v[9], g[9];
 #pragma unroll
-    for (int j = 0; j < CAP; j += 2) {
-      if (j < len) s0 = fma(wv[j], __ldg(x + wc[j]), s0);
-      if (j + 1 < len) s1 = fma(wv[j + 1], __ldg(x + wc[j + 1]), s1);
+      for (int j = 0; j < 9; ++j) {
+        const bool in = t + j < len;
+        v[j] = in ? wv[t + j] : T(0);
+        g[j] = in ? __ldg(x + wc[t + j]) : T(0);
+      }
+#pragma unroll
+      for (int j = 0; j < 9; j += 3) {
+        s0 = fma(v[j], g[j], s0);
+        s1 = fma(v[j + 1], g[j + 1], s1);
+        s2 = fma(v[j + 2], g[j + 2], s2);
+      }
     }
-    row_body<HASW>(body, row, active, s0 + s1, wr);
-    __syncwarp();  // the buffer just read is refilled by the next stage
-    rb = rb2, re = re2, vb = vb2, cb = cb2;
+    for (; t < width; ++t)
+      if (t < len) s0 = fma(wv[t], __ldg(x + wc[t]), s0);
+    row_body<HASW>(body, row, active, (s0 + s1) + s2, wr);
+    __syncwarp();  // the buffer just read is refilled by the next step
+    rb = rb2, re = re2;
   }
 }
 
@@ -220,8 +231,9 @@ struct SellView {
 // Warp-uniform loop over the slices, one warp per slice (grid-stride): body(row, active, s, wr) runs
 // in every lane with s = (A x)[row]; with HASW, wr = w[row] is loaded before the row's gathers (the
 // dot partner of a fused reduction), else 0. Entries are consumed 9 at a time (the 27 of a 3D Q1
-// row are three full groups), all 9 value/column loads issued before the first FMA, then one at a
-// time for the rest of the slice's width.
+// row are three full groups), all 9 value/column loads issued before the first FMA, then up to 8 for
+// the rest of the slice's width (one at a time each pays the latency of its gather: 60 us for the
+// 125-entry rows of 28^3 Q2 cubes, 41 like this). The bits are those of the asynchronous CSR schedule.
 template <bool HASW = false, class Body>
 __device__ __forceinline__ void for_slices(const SellView& A, const double* __restrict__ x, Body body,
                                            const double* __restrict__ w = nullptr) {
@@ -251,7 +263,18 @@ __device__ __forceinline__ void for_slices(const SellView& A, const double* __re
         s2 = fma(vv[j + 2], __ldg(x + cc[j + 2]), s2);
       }
     }
-    for (; t < md.y; ++t) s0 = fma(ld_stream(v + t * 32), __ldg(x + ld_stream(c + t * 32)), s0);
+    if (t < md.y) {
+      double vv[8], xv[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        vv[j] = xv[j] = 0.0;
+        if (t + j < md.y) {
+          vv[j] = ld_stream(v + (t + j) * 32);
+          xv[j] = __ldg(x + ld_stream(c + (t + j) * 32));
+        }
+      }
+      fma_chain<0>(md.y - t, vv, xv, s0);
+    }
     body(row, active, (s0 + s1) + s2, wr);
   }
 }
@@ -284,6 +307,7 @@ __device__ __forceinline__ void for_rows_csr_w(int n, const int* __restrict__ rp
 
 // the schedule table: index -> (G, PL)
 constexpr int kSchedules = 8;
+constexpr int kAsyncSchedule = 7;
 __host__ __device__ constexpr int sched_G(int s) { return s == 0 ? 4 : s == 1 ? 8 : s == 2 ? 16 : s == 3 ? 32 : 0; }
 __host__ __device__ constexpr int sched_PL(int s) {
   return s == 4 ? 8 : s == 5 ? 16 : s == 6 ? 32 : s == 7 ? -28 : 0;

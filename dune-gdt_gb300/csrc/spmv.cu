@@ -2,10 +2,10 @@
 // form, and the SpMV schedule autotuner.
 //
 // Schedules (linalg.cuh): vector-CSR with G in {4, 8, 16, 32} lanes per row, register-pipelined
-// warp staging with PL in {8, 16, 32} entries per lane, cp.async double-buffered warp staging for
+// warp staging with PL in {8, 16, 32} entries per lane, cp.async warp staging for
 // rows of at most 28 entries, and (index 8) the SELL-32 copy of the matrix read one lane per row.
 // The first SpMV-type call on a matrix times every schedule valid for its longest row with CUDA
-// events (FP64, on a non-trivial probe vector, three launches each, after one warm-up) and keeps the
+// events (FP64, on a non-trivial probe vector, three launches each, after a warm-up) and keeps the
 // fastest CSR schedule for all CSR kernels of that matrix (plain, fused dot, residual,
 // mixed-precision residual); when the SELL-32 schedule is faster still, the plain SpMV and the
 // graph-form CG SpMV read the SELL copy instead.
@@ -239,15 +239,22 @@ gdt_status tune_spmv(gdt_context ctx, gdt_matrix m, double* times_ms) {
   cudaEventCreate(&e1);
   float best = FLT_MAX;
   int best_sched = m->spmv_sched;
-  auto time3 = [&](auto launch, float& ms) {
-    launch();
+  auto timed = [&](auto launch, int reps, float& ms) {
     cudaEventRecord(e0, s);
-    for (int r = 0; r < 3; ++r) launch();
+    for (int r = 0; r < reps; ++r) launch();
     cudaEventRecord(e1, s);
     cudaEventSynchronize(e1);
     ms = 0.f;
-    ctx->launches += 4;
+    ctx->launches += reps;
     return cudaGetLastError() == cudaSuccess && cudaEventElapsedTime(&ms, e0, e1) == cudaSuccess;
+  };
+  // three launches after one to warm up; unless the caller wants all the times, not of schedules that
+  // take more than twice as long as the best so far
+  auto time3 = [&](auto launch, float& ms) {
+    launch();
+    ctx->launches++;
+    if (!times_ms && (!timed(launch, 1, ms) || 3.f * ms > 2.f * best)) return false;
+    return timed(launch, 3, ms);
   };
   for (int sched = 0; sched < kSchedules; ++sched) {
     if (!schedule_valid(sched, m->max_row)) continue;
@@ -261,11 +268,17 @@ gdt_status tune_spmv(gdt_context ctx, gdt_matrix m, double* times_ms) {
   }
   // the SELL-32 copy, when there is room for it
   bool sell_best = false;
+  m->csr_products = 0;
   if (sell_prepare(ctx, m, s, false) == GDT_OK) {
-    float ms = 0.f;
+    float ms = 0.f, fill = 0.f;
     const bool ok = time3([&] { launch_sell_spmv(m, x, y, ctx->num_sms, s); }, ms);
     if (ok && times_ms) times_ms[kSellSchedule] = ms / 3.0;
     sell_best = ok && ms < best;
+    // Changed values need a new copy, which costs about three products (96 x 101 x 90 Q1: 171 us beside
+    // 53 us with it and 70 us without). So the first products with them read the CSR arrays, as many as it takes
+    // the copy to save its fill; only where both give the same bits (one lane per row, sums in one order).
+    if (sell_best && best_sched == kAsyncSchedule && timed([&] { sell_prepare(ctx, m, s, true); }, 1, fill))
+      m->csr_products = int(std::min(3.f * fill / (best - ms), 1000.f));
   }
   cudaGetLastError();
   cudaEventDestroy(e0);
@@ -282,9 +295,17 @@ gdt_status tune_spmv(gdt_context ctx, gdt_matrix m, double* times_ms) {
 
 gdt_status spmv(gdt_context ctx, gdt_matrix m, const double* x, double* y) {
   GDT_CHECK(ctx, tune_spmv(ctx, m));
-  if (m->use_sell && sell_prepare(ctx, m, ctx->stream, false) != GDT_OK) m->use_sell = 0;
+  bool sell = m->use_sell;
+  if (sell && m->sell_version != m->val_version && m->csr_products > 0) {
+    if (m->csr_version != m->val_version) {
+      m->csr_version = m->val_version;
+      m->csr_done = 0;
+    }
+    sell = m->csr_done++ >= m->csr_products;
+  }
+  if (sell && sell_prepare(ctx, m, ctx->stream, false) != GDT_OK) m->use_sell = sell = false;
   timing_begin(ctx, ctx->stream, GDT_TIMING_SPMV_FP64);
-  if (m->use_sell) launch_sell_spmv(m, x, y, ctx->num_sms, ctx->stream);
+  if (sell) launch_sell_spmv(m, x, y, ctx->num_sms, ctx->stream);
   else launch_spmv<double>(m->spmv_sched, int(m->rows), m->rp, m->col, m->val, x, y, ctx->num_sms, ctx->stream);
   timing_end(ctx, ctx->stream);
   return check_launch(ctx, "spmv");
@@ -309,6 +330,7 @@ extern "C" gdt_status gdt_matrix_set_schedule(gdt_matrix m, int schedule) {
   if (schedule == gdt::kSellSchedule) {
     // the CSR kernels (residuals, mixed-precision checks) keep their schedule
     m->use_sell = 1;
+    m->csr_products = 0;
   } else {
     if (!gdt::schedule_valid(schedule, m->max_row)) return GDT_EINVAL;
     m->spmv_sched = schedule;
