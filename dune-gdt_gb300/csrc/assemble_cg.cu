@@ -108,12 +108,12 @@ __device__ __forceinline__ bool on_boundary(const GridDesc& g, const long long* 
 
 // Row v of the assembled operator from its gathered stencil acc (slots of the 3^d neighbourhood) and
 // load b: Dirichlet unit row / zero columns with the lifting of given boundary values, then the
-// right-hand side entry and the CSR row (slots in ascending column order)
+// right-hand side entry and the row's values to out (slots in ascending column order)
 template <int DIM, bool SIMPLEX>
 __device__ __forceinline__ void finish_row(const GridDesc& g, long long v, const long long (&vi)[3],
-                                           const double (&acc)[pow3(DIM)], double b, const int* __restrict__ rp,
-                                           double* __restrict__ val, double* __restrict__ rhs, int dirichlet,
-                                           const double* __restrict__ gD, double gD_const) {
+                                           const double (&acc)[pow3(DIM)], double b, double* __restrict__ out,
+                                           double* __restrict__ rhs, int dirichlet, const double* __restrict__ gD,
+                                           double gD_const) {
   constexpr int NS = pow3(DIM);
   const bool bnd = dirichlet && on_boundary(g, vi, DIM);
   // Dirichlet values g: b_v = g_v on a boundary row; elsewhere the zeroed columns move to the right-hand
@@ -134,8 +134,7 @@ __device__ __forceinline__ void finish_row(const GridDesc& g, long long v, const
     }
   }
   if (rhs) rhs[v] = bnd ? (lift ? (gD ? gD[v] : gD_const) : 0.0) : b;
-  if (!val) return;
-  long long pos = rp[v];
+  if (!out) return;
 #pragma unroll
   for (int k = 0; k < NS; ++k) {
     if (!slot_in_stencil(DIM, SIMPLEX, k)) continue;
@@ -152,7 +151,7 @@ __device__ __forceinline__ void finish_row(const GridDesc& g, long long v, const
       if (bnd) value = (k == center_slot(DIM)) ? 1.0 : 0.0;  // unit_row
       else if (on_boundary(g, w, DIM)) value = 0.0;          // unit_col
     }
-    val[pos++] = value;
+    *out++ = value;
   }
 }
 
@@ -198,7 +197,124 @@ __global__ void __launch_bounds__(256) assemble_cg_rows(GridDesc g, const int* _
       }
     }
   }
-  finish_row<DIM, SIMPLEX>(g, v, vi, acc, b, rp, val, rhs, dirichlet, gD, gD_const);
+  finish_row<DIM, SIMPLEX>(g, v, vi, acc, b, val ? val + rp[v] : nullptr, rhs, dirichlet, gD, gD_const);
+}
+
+// The same rows for 3D cubes. K[i][j] depends on the axes in which corners i and j differ only (f[i ^ j]), so an
+// entry of row v is f of its offset times the sum of kappa over the cells that both vertices belong to, and the
+// nine entries towards the plane above are those of the row above towards this plane. A thread walks a chunk of
+// zlen planes of a vertex column: 33 FP64 operations and 5 for the load per row instead of 72 (an FP64
+// instruction takes a quarter of an SM for 64 cycles: 106 us of the 145 us of 97 x 102 x 91 rows). The sums
+// associate by axis, the same from both ends of an entry, so the matrix is symmetric to the bit. A warp's 32
+// columns are 32 consecutive rows, hence one range of the CSR values: it is put together in shared memory and
+// stored side by side (the rows themselves start 216 bytes apart). kappa_out: FP32 copy of the coefficients.
+constexpr int QT = 128;
+
+__global__ void __launch_bounds__(QT, 4) assemble_q1_columns(GridDesc g, const int* __restrict__ rp,
+                                                             double* __restrict__ val, double* __restrict__ rhs,
+                                                             const LocalTables tab, const double* __restrict__ kappa,
+                                                             double kappa_const, const double* __restrict__ force,
+                                                             double force_const, int dirichlet,
+                                                             const double* __restrict__ gD, double gD_const,
+                                                             float* __restrict__ kappa_out, int zlen) {
+  __shared__ double stage[QT / 32][32 * 27];
+  const int lane = threadIdx.x & 31;
+  const int nx = int(g.vn[0]), ny = int(g.vn[1]), nz = int(g.vn[2]), ncol = nx * ny;
+  const int warp_col = blockIdx.x * QT + (threadIdx.x & ~31);
+  if (warp_col >= ncol) return;
+  const int c = warp_col + lane;
+  const bool active = c < ncol;
+  const int x = active ? c % nx : 0, y = active ? c / nx : 0;
+  const int z0 = blockIdx.y * zlen, z1 = min(nz, z0 + zlen);
+  const long long cxy = (long long)g.n[0] * g.n[1];
+  double f[8];
+#pragma unroll
+  for (int t = 0; t < 8; ++t) f[t] = tab.K[t];
+  // the cells (x - 1 + (j & 1), y - 1 + (j >> 1)) around the column
+  bool in[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int cx = x - 1 + (j & 1), cy = y - 1 + (j >> 1);
+    in[j] = active && cx >= 0 && cx < nx - 1 && cy >= 0 && cy < ny - 1;
+  }
+  const long long cell0 = (x - 1) + (long long)g.n[0] * (y - 1);
+  auto load_layer = [&](int cz, double(&k)[4], double& q) {
+    const bool inside = cz >= 0 && cz < nz - 1;
+    double p[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const long long e = cell0 + (j & 1) + (j >> 1) * (long long)g.n[0] + cz * cxy;
+      k[j] = inside && in[j] ? (kappa ? __ldg(kappa + e) : kappa_const) : 0.0;
+      p[j] = rhs && inside && in[j] ? (force ? __ldg(force + e) : force_const) : 0.0;
+    }
+    q = rhs ? (p[0] + p[1]) + (p[2] + p[3]) : 0.0;
+  };
+  // sums over a layer's cells: its two x rows, its two y rows, all four; and its nine entries towards the other plane
+  struct Layer {
+    double k[4], row[2], colsum[2], all;
+  };
+  auto sums = [](Layer& l) {
+    l.row[0] = l.k[0] + l.k[1];
+    l.row[1] = l.k[2] + l.k[3];
+    l.colsum[0] = l.k[0] + l.k[2];
+    l.colsum[1] = l.k[1] + l.k[3];
+    l.all = l.row[0] + l.row[1];
+  };
+  auto across = [&](const Layer& l, double* a) {
+    a[0] = f[7] * l.k[0];
+    a[1] = f[6] * l.row[0];
+    a[2] = f[7] * l.k[1];
+    a[3] = f[5] * l.colsum[0];
+    a[4] = f[4] * l.all;
+    a[5] = f[5] * l.colsum[1];
+    a[6] = f[7] * l.k[2];
+    a[7] = f[6] * l.row[1];
+    a[8] = f[7] * l.k[3];
+  };
+  Layer lo, hi;
+  double qlo, qhi, acc[27];
+  load_layer(z0 - 1, lo.k, qlo);
+  load_layer(z0, hi.k, qhi);
+  sums(lo);
+  across(lo, acc);
+  for (int z = z0; z < z1; ++z) {
+    double next[4], qnext;  // in flight during this row
+    load_layer(z + 1, next, qnext);
+    const int v0 = z * ncol + warp_col, v = v0 + lane;
+    const int rows = min(32, ncol - warp_col);
+    const int beg = rp ? __ldg(rp + v0) : 0, own = rp ? __ldg(rp + min(v, v0 + rows - 1)) : 0;
+    const int end = rp ? __ldg(rp + v0 + rows) : 0;
+    if (kappa_out && in[3] && z < nz - 1) kappa_out[cell0 + 1 + g.n[0] + z * cxy] = float(hi.k[3]);
+    sums(hi);
+    across(hi, acc + 18);
+    acc[9] = f[3] * (lo.k[0] + hi.k[0]);
+    acc[10] = f[2] * (lo.row[0] + hi.row[0]);
+    acc[11] = f[3] * (lo.k[1] + hi.k[1]);
+    acc[12] = f[1] * (lo.colsum[0] + hi.colsum[0]);
+    acc[13] = f[0] * (lo.all + hi.all);
+    acc[14] = f[1] * (lo.colsum[1] + hi.colsum[1]);
+    acc[15] = f[3] * (lo.k[2] + hi.k[2]);
+    acc[16] = f[2] * (lo.row[1] + hi.row[1]);
+    acc[17] = f[3] * (lo.k[3] + hi.k[3]);
+    double* const st = stage[threadIdx.x >> 5];
+    if (active) {
+      const long long vi[3] = {x, y, z};
+      finish_row<3, false>(g, v, vi, acc, rhs ? tab.B[0] * (qlo + qhi) : 0.0, val ? st + (own - beg) : nullptr, rhs,
+                           dirichlet, gD, gD_const);
+    }
+    if (val) {
+      __syncwarp();
+      for (int k = lane; k < end - beg; k += 32) val[beg + k] = st[k];
+      __syncwarp();
+    }
+    lo = hi;
+    qlo = qhi;
+    qhi = qnext;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) hi.k[j] = next[j];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) acc[k] = acc[18 + k];
+  }
 }
 
 // Mapped grids (vertex coordinates g.xv) in two passes, so that each element's geometry is formed once:
@@ -614,7 +730,7 @@ __global__ void __launch_bounds__(256) assemble_cg_rows_tabled(GridDesc g, const
     }
     if (rhs) b += tb[(SIMPLEX ? cv : 0) * nc + cell];
   }
-  finish_row<DIM, SIMPLEX>(g, v, vi, acc, b, rp, val, rhs, dirichlet, gD, gD_const);
+  finish_row<DIM, SIMPLEX>(g, v, vi, acc, b, val ? val + rp[v] : nullptr, rhs, dirichlet, gD, gD_const);
 }
 
 // DirichletConstraints::apply(M, V) as a separate pass over an assembled matrix: unit rows for
@@ -695,25 +811,28 @@ LocalTables make_tables(const GridDesc& g) {
 
 }  // namespace
 
-__global__ void k_mf_kappa(long long n, const double* __restrict__ kappa, double kc, float* __restrict__ out) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    out[i] = float(kappa ? kappa[i] : kc);
-}
-
-gdt_status mf_capture(gdt_context ctx, gdt_matrix m, const gdt_diffusion_desc* d) {
+// the reference element's stiffness for the matrix-free FP32 operator; the coefficients are written by the assembly
+gdt_status mf_prepare(gdt_context ctx, gdt_matrix m, const gdt_diffusion_desc* d, const LocalTables& tab) {
   const GridDesc& g = m->test.g;
-  m->mf_valid = 0;
-  if (g.dim != 3 || g.simplex || m->test.order != 1 || m->test.kind != GDT_SPACE_CG) return GDT_OK;
   if (!m->mf_kappa) GDT_TRY_CUDA(ctx, cudaMalloc(&m->mf_kappa, sizeof(float) * g.nelem));
-  const int bl = std::max(1, std::min(grid_blocks(g.nelem, 256), ctx->num_sms * 8));
-  k_mf_kappa<<<bl, 256, 0, ctx->stream>>>(g.nelem, d->kappa, d->kappa_const, m->mf_kappa);
-  const LocalTables tab = make_tables(g);
   for (int li = 0; li < 8; ++li)
     for (int lj = 0; lj < 8; ++lj)
       m->mf_K[local_corner(3, false, 0, li) * 8 + local_corner(3, false, 0, lj)] = float(tab.K[li * kMaxLoc + lj]);
   m->mf_dirichlet = d->dirichlet ? 1 : 0;
-  m->mf_valid = 1;
-  return check_launch(ctx, "mf_capture");
+  return GDT_OK;
+}
+
+// 3D cubes: rows of a column per thread, few enough for eight blocks of an SM to have work
+gdt_status launch_q1_columns(gdt_context ctx, const GridDesc& g, const int* rp, double* val, double* rhs,
+                             const LocalTables& tab, const gdt_diffusion_desc* d, const double* gD, double gD_const,
+                             float* kappa_out) {
+  const long long ncol = g.vn[0] * g.vn[1];
+  // (a chunk repeats the sums of one layer, 14 operations; longer ones leave SMs idle on small grids)
+  const int zlen = int(std::max((g.vn[2] + 65534) / 65535, std::max(1LL, std::min(8LL, g.nvert / (1024LL * ctx->num_sms)))));
+  const dim3 grid(grid_blocks(ncol, QT), unsigned((g.vn[2] + zlen - 1) / zlen));
+  assemble_q1_columns<<<grid, QT, 0, ctx->stream>>>(g, rp, val, rhs, tab, d->kappa, d->kappa_const, d->force,
+                                                    d->force_const, d->dirichlet, gD, gD_const, kappa_out, zlen);
+  return check_launch(ctx, "assemble_q1_columns");
 }
 
 // mapped grids: the cube tables (stiffness and/or load), then the row gather over them
@@ -755,6 +874,14 @@ gdt_status assemble_cg(gdt_context ctx, gdt_matrix m, const gdt_diffusion_desc* 
     return assemble_cg_mapped(ctx, g, m->rp, m->val, d, rhs, d->dirichlet_values, d->dirichlet_value_const);
   }
   const LocalTables tab = make_tables(g);
+  m->mf_valid = 0;
+  if (g.dim == 3 && !g.simplex) {
+    GDT_CHECK(ctx, mf_prepare(ctx, m, d, tab));
+    GDT_CHECK(ctx, launch_q1_columns(ctx, g, m->rp, m->val, rhs, tab, d, d->dirichlet_values, d->dirichlet_value_const,
+                                     m->mf_kappa));
+    m->mf_valid = 1;
+    return GDT_OK;
+  }
   const int th = 256;
   const int bl = grid_blocks(g.nvert, th);
   cudaStream_t s = ctx->stream;
@@ -764,17 +891,16 @@ gdt_status assemble_cg(gdt_context ctx, gdt_matrix m, const gdt_diffusion_desc* 
   if (g.dim == 1) GDT_LAUNCH_ASM(1, false);
   else if (g.dim == 2 && !g.simplex) GDT_LAUNCH_ASM(2, false);
   else if (g.dim == 2) GDT_LAUNCH_ASM(2, true);
-  else if (!g.simplex) GDT_LAUNCH_ASM(3, false);
   else GDT_LAUNCH_ASM(3, true);
 #undef GDT_LAUNCH_ASM
-  GDT_CHECK(ctx, check_launch(ctx, "assemble_cg_rows"));
-  return mf_capture(ctx, m, d);
+  return check_launch(ctx, "assemble_cg_rows");
 }
 
 gdt_status assemble_cg_rhs(gdt_context ctx, const gdt_space_s& sp, const gdt_diffusion_desc* d, double* rhs) {
   const GridDesc& g = sp.g;
   if (g.xv) return assemble_cg_mapped(ctx, g, nullptr, nullptr, d, rhs, nullptr, 0.0);
   const LocalTables tab = make_tables(g);
+  if (g.dim == 3 && !g.simplex) return launch_q1_columns(ctx, g, nullptr, nullptr, rhs, tab, d, nullptr, 0.0, nullptr);
   const int th = 256;
   const int bl = grid_blocks(g.nvert, th);
   cudaStream_t s = ctx->stream;
@@ -784,7 +910,6 @@ gdt_status assemble_cg_rhs(gdt_context ctx, const gdt_space_s& sp, const gdt_dif
   if (g.dim == 1) GDT_LAUNCH_RHS(1, false);
   else if (g.dim == 2 && !g.simplex) GDT_LAUNCH_RHS(2, false);
   else if (g.dim == 2) GDT_LAUNCH_RHS(2, true);
-  else if (!g.simplex) GDT_LAUNCH_RHS(3, false);
   else GDT_LAUNCH_RHS(3, true);
 #undef GDT_LAUNCH_RHS
   return check_launch(ctx, "assemble_cg_rhs");
