@@ -203,11 +203,13 @@ __global__ void __launch_bounds__(256) assemble_cg_rows(GridDesc g, const int* _
 // The same rows for 3D cubes. K[i][j] depends on the axes in which corners i and j differ only (f[i ^ j]), so an
 // entry of row v is f of its offset times the sum of kappa over the cells that both vertices belong to, and the
 // nine entries towards the plane above are those of the row above towards this plane. A thread walks a chunk of
-// zlen planes of a vertex column: 33 FP64 operations and 5 for the load per row instead of 72 (an FP64
-// instruction takes a quarter of an SM for 64 cycles: 106 us of the 145 us of 97 x 102 x 91 rows). The sums
+// zlen planes of a vertex column: 37 FP64 operations per row instead of 72 (an FP64 instruction takes a
+// quarter of an SM for 64 cycles: 106 us of the 145 us that 97 x 102 x 91 rows took; now 69 of 86). The sums
 // associate by axis, the same from both ends of an entry, so the matrix is symmetric to the bit. A warp's 32
 // columns are 32 consecutive rows, hence one range of the CSR values: it is put together in shared memory and
-// stored side by side (the rows themselves start 216 bytes apart). kappa_out: FP32 copy of the coefficients.
+// stored side by side (the rows themselves start 216 bytes apart). Which neighbours are there is kept as bits
+// per column (64-bit comparisons per entry were 30 us), and each nine entries are stored as they are formed
+// (all 27 at once took 128 registers and 115 us). kappa_out: FP32 copy of the coefficients.
 constexpr int QT = 128;
 
 __global__ void __launch_bounds__(QT, 4) assemble_q1_columns(GridDesc g, const int* __restrict__ rp,
@@ -237,6 +239,14 @@ __global__ void __launch_bounds__(QT, 4) assemble_q1_columns(GridDesc g, const i
     const int cx = x - 1 + (j & 1), cy = y - 1 + (j >> 1);
     in[j] = active && cx >= 0 && cx < nx - 1 && cy >= 0 && cy < ny - 1;
   }
+  // the columns around it (and itself, bit 4): there in the grid, and on its boundary
+  unsigned there = 0, zero = 0;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) {
+    const int xn = x + k % 3 - 1, yn = y + k / 3 - 1;
+    if (active && xn >= 0 && xn < nx && yn >= 0 && yn < ny) there |= 1u << k;
+    if (dirichlet && (xn == 0 || xn == nx - 1 || yn == 0 || yn == ny - 1)) zero |= 1u << k;
+  }
   const long long cell0 = (x - 1) + (long long)g.n[0] * (y - 1);
   auto load_layer = [&](int cz, double(&k)[4], double& q) {
     const bool inside = cz >= 0 && cz < nz - 1;
@@ -260,7 +270,7 @@ __global__ void __launch_bounds__(QT, 4) assemble_q1_columns(GridDesc g, const i
     l.colsum[1] = l.k[1] + l.k[3];
     l.all = l.row[0] + l.row[1];
   };
-  auto across = [&](const Layer& l, double* a) {
+  auto across = [&](const Layer& l, double(&a)[9]) {
     a[0] = f[7] * l.k[0];
     a[1] = f[6] * l.row[0];
     a[2] = f[7] * l.k[1];
@@ -271,12 +281,14 @@ __global__ void __launch_bounds__(QT, 4) assemble_q1_columns(GridDesc g, const i
     a[7] = f[6] * l.row[1];
     a[8] = f[7] * l.k[3];
   };
+  const bool lift = rhs && dirichlet && (gD || gD_const != 0.0);
+  double* const st = stage[threadIdx.x >> 5];
   Layer lo, hi;
-  double qlo, qhi, acc[27];
+  double qlo, qhi, low[9];
   load_layer(z0 - 1, lo.k, qlo);
   load_layer(z0, hi.k, qhi);
   sums(lo);
-  across(lo, acc);
+  across(lo, low);
   for (int z = z0; z < z1; ++z) {
     double next[4], qnext;  // in flight during this row
     load_layer(z + 1, next, qnext);
@@ -285,23 +297,41 @@ __global__ void __launch_bounds__(QT, 4) assemble_q1_columns(GridDesc g, const i
     const int beg = rp ? __ldg(rp + v0) : 0, own = rp ? __ldg(rp + min(v, v0 + rows - 1)) : 0;
     const int end = rp ? __ldg(rp + v0 + rows) : 0;
     if (kappa_out && in[3] && z < nz - 1) kappa_out[cell0 + 1 + g.n[0] + z * cxy] = float(hi.k[3]);
+    const bool bnd = dirichlet && ((zero >> 4 & 1) || z == 0 || z == nz - 1);
+    double b = tab.B[0] * (qlo + qhi);
+    double* out = st + (own - beg);
+    // the row's nine entries towards plane z + p: unit row, zero columns; with Dirichlet values g the zeroed columns
+    // move to the right-hand side
+    auto emit = [&](int p, const double(&a)[9]) {
+      const int zn = z + p;
+      const unsigned stored = zn >= 0 && zn < nz ? there : 0u;
+      const unsigned drop = bnd || (dirichlet && (zn == 0 || zn == nz - 1)) ? 511u : zero;
+      if (lift && !bnd) {
+#pragma unroll
+        for (int k = 0; k < 9; ++k)
+          if (stored & drop & 1u << k) b -= a[k] * (gD ? gD[v + k % 3 - 1 + (k / 3 - 1) * nx + p * ncol] : gD_const);
+      }
+      if (!val) return;
+#pragma unroll
+      for (int k = 0; k < 9; ++k)
+        if (stored >> k & 1) *out++ = drop >> k & 1 ? (bnd && k == 4 && p == 0 ? 1.0 : 0.0) : a[k];
+    };
+    emit(-1, low);
     sums(hi);
-    across(hi, acc + 18);
-    acc[9] = f[3] * (lo.k[0] + hi.k[0]);
-    acc[10] = f[2] * (lo.row[0] + hi.row[0]);
-    acc[11] = f[3] * (lo.k[1] + hi.k[1]);
-    acc[12] = f[1] * (lo.colsum[0] + hi.colsum[0]);
-    acc[13] = f[0] * (lo.all + hi.all);
-    acc[14] = f[1] * (lo.colsum[1] + hi.colsum[1]);
-    acc[15] = f[3] * (lo.k[2] + hi.k[2]);
-    acc[16] = f[2] * (lo.row[1] + hi.row[1]);
-    acc[17] = f[3] * (lo.k[3] + hi.k[3]);
-    double* const st = stage[threadIdx.x >> 5];
-    if (active) {
-      const long long vi[3] = {x, y, z};
-      finish_row<3, false>(g, v, vi, acc, rhs ? tab.B[0] * (qlo + qhi) : 0.0, val ? st + (own - beg) : nullptr, rhs,
-                           dirichlet, gD, gD_const);
-    }
+    double mid[9];
+    mid[0] = f[3] * (lo.k[0] + hi.k[0]);
+    mid[1] = f[2] * (lo.row[0] + hi.row[0]);
+    mid[2] = f[3] * (lo.k[1] + hi.k[1]);
+    mid[3] = f[1] * (lo.colsum[0] + hi.colsum[0]);
+    mid[4] = f[0] * (lo.all + hi.all);
+    mid[5] = f[1] * (lo.colsum[1] + hi.colsum[1]);
+    mid[6] = f[3] * (lo.k[2] + hi.k[2]);
+    mid[7] = f[2] * (lo.row[1] + hi.row[1]);
+    mid[8] = f[3] * (lo.k[3] + hi.k[3]);
+    emit(0, mid);
+    across(hi, low);
+    emit(1, low);
+    if (rhs && active) rhs[v] = bnd ? (lift ? (gD ? gD[v] : gD_const) : 0.0) : b;
     if (val) {
       __syncwarp();
       for (int k = lane; k < end - beg; k += 32) val[beg + k] = st[k];
@@ -312,8 +342,6 @@ __global__ void __launch_bounds__(QT, 4) assemble_q1_columns(GridDesc g, const i
     qhi = qnext;
 #pragma unroll
     for (int j = 0; j < 4; ++j) hi.k[j] = next[j];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) acc[k] = acc[18 + k];
   }
 }
 
@@ -822,13 +850,13 @@ gdt_status mf_prepare(gdt_context ctx, gdt_matrix m, const gdt_diffusion_desc* d
   return GDT_OK;
 }
 
-// 3D cubes: rows of a column per thread, few enough for eight blocks of an SM to have work
 gdt_status launch_q1_columns(gdt_context ctx, const GridDesc& g, const int* rp, double* val, double* rhs,
                              const LocalTables& tab, const gdt_diffusion_desc* d, const double* gD, double gD_const,
                              float* kappa_out) {
   const long long ncol = g.vn[0] * g.vn[1];
-  // (a chunk repeats the sums of one layer, 14 operations; longer ones leave SMs idle on small grids)
-  const int zlen = int(std::max((g.vn[2] + 65534) / 65535, std::max(1LL, std::min(8LL, g.nvert / (1024LL * ctx->num_sms)))));
+  // a chunk repeats the sums of one layer, 20 operations; longer ones leave SMs idle on small grids (97 x 102 x 91
+  // rows: 113, 111, 117 and 130 us with 4, 6, 8 and 16 planes; 40 x 38 x 41: 17 us with one, 27 with 6)
+  const int zlen = int(std::max((g.vn[2] + 65534) / 65535, std::max(1LL, std::min(6LL, g.nvert / (1024LL * ctx->num_sms)))));
   const dim3 grid(grid_blocks(ncol, QT), unsigned((g.vn[2] + zlen - 1) / zlen));
   assemble_q1_columns<<<grid, QT, 0, ctx->stream>>>(g, rp, val, rhs, tab, d->kappa, d->kappa_const, d->force,
                                                     d->force_const, d->dirichlet, gD, gD_const, kappa_out, zlen);
