@@ -110,6 +110,8 @@ struct gdt_matrix_s {
   int* sell_col = nullptr;
   double* sell_val = nullptr;
   long long sell_len = 0;
+  std::vector<int> sell_off;    // the offsets on the host, sell_len last
+  bool sell_padded = false;     // found too full of padding for the persistent CG
   long long val_version = 0;    // bumped by every entry point that may change the values
   long long sell_version = -1;  // val_version the SELL copy was filled at
   int use_sell = 0;             // plain SpMV and the graph-form CG SpMV read the SELL copy (tuned or pinned)
@@ -184,6 +186,8 @@ gdt_status tune_spmv(gdt_context ctx, gdt_matrix m, double* times_ms = nullptr);
 // SELL-32 copy of m: slice table built once per pattern (GDT_EUNSUPPORTED when there is no room or the
 // offsets do not fit 32 bits), values and columns copied when the values changed or `refill` is set
 gdt_status sell_prepare(gdt_context ctx, gdt_matrix m, cudaStream_t s, bool refill);
+// its slice table and memory alone
+gdt_status sell_table(gdt_context ctx, gdt_matrix m, cudaStream_t s);
 // the copy without the zero values, for solves whose vectors are finite by their own checks (a product
 // keeps them: 0 * inf is not 0): width (device, one per 32-row slice) receives the entries per row
 gdt_status sell_prepare_nonzero(gdt_context ctx, gdt_matrix m, cudaStream_t s, int* width);

@@ -663,7 +663,6 @@ void ilu_apply(gdt_context ctx, gdt_matrix m, const Ilu& f, const double* r, dou
 // between the sums and read with plain loads, which the fences of the exchanges order.
 struct PcgArgs {
   int n;
-  int nslices;
   const int2* meta;   // SELL-32 (offset, width) per slice
   const int* width;   // entries per row of the slice after dropping zeros
   const int* col;     // SELL-32 columns
@@ -677,6 +676,8 @@ struct PcgArgs {
   ExchangeView ex;    // the whole grid
   int cap;            // matrix entries a block may keep in shared memory (resident form)
   int stream;         // the matrix exceeds L2: mark its lines evict-first
+  int units;          // the most units of a block (streaming form by units)
+  int first[257];     // the block's slices: first[block] .. first[block + 1] - 1
 };
 
 // The scalars of the iteration, kept by thread 0 of every block (the same bits in all of them).
@@ -809,8 +810,7 @@ __global__ void __launch_bounds__(RT, 1) k_pcg_resident(const __grid_constant__ 
   constexpr int CH = R <= 8 ? 16 : 9;  // entries in flight per row, as the registers allow
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (entry_flag(&a.st->converged)) return;
-  const int s0 = int((long long)a.nslices * blockIdx.x / gridDim.x);
-  const int ns = int((long long)a.nslices * (blockIdx.x + 1) / gridDim.x) - s0;
+  const int s0 = a.first[blockIdx.x], ns = a.first[blockIdx.x + 1] - s0;
   const int warps = min(ns, RT / 32);  // that have rows
   if (threadIdx.x == 0) {
     sh.ex.fault = 0;
@@ -912,50 +912,159 @@ __global__ void __launch_bounds__(RT, 1) k_pcg_resident(const __grid_constant__ 
 
 // The streaming form, for systems whose rows do not fit the registers of the grid: the same iteration with the
 // vectors in memory (each block the same contiguous rows in both passes).
+// SPLIT: slices of long rows in units of at most kUnit entries per row, each summed by any warp into shared memory, so
+// that a few dozen slices of 125 entries are neither 14 gathers in a row for one warp nor uneven shares
+// for the others (28^3 Q2 cubes: 69 us an iteration by slices, 52 by units, 48 with the
+// gathers ahead).
 constexpr int PT = 1024;  // threads per block (one block per SM)
+constexpr int kUnit = 36;
 
+__host__ __device__ constexpr int pcg_units(int width) { return width <= kUnit ? 1 : (width + kUnit - 1) / kUnit; }
+
+// The sums of a warp's segments (entries t < w of the lane's row at src + 32 t; next(src, w) gives them one after the
+// other, warp-uniform): begin() where a segment starts, done(sum) where it ends. Groups of nine entries in three
+// buffers: the entries are loaded three steps of three before their products and the vector is gathered one step
+// before, across the ends of segments, so that neither latency is waited for.
+template <class Next, class Begin, class Done>
+__device__ __forceinline__ void pcg_segments(const PcgArgs& a, unsigned long long pol, Next next, Begin begin, Done done) {
+  const int lane = threadIdx.x & 31;
+  int src, w, nsrc = 0, nw = 0;
+  if (!next(src, w)) return;
+  bool more = next(nsrc, nw);
+  double v[3][3], g[3][3];
+  int c[3][3];
+  auto load = [&](int j, int base, int left) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const bool in = 3 * j + i < left;  // warp-uniform
+      v[j][i] = in ? ld_matrix(a.val + base + lane + 32 * (3 * j + i), pol) : 0.0;
+      c[j][i] = in ? ld_matrix(a.col + base + lane + 32 * (3 * j + i), pol) : 0;
+    }
+  };
+  auto gather = [&](int j) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) g[j][i] = a.p[c[j][i]];
+  };
+#pragma unroll
+  for (int j = 0; j < 3; ++j) load(j, src, w);
+  gather(0);
+  begin();
+  double s = 0.0;
+  for (int t = 0;;) {
+    const bool last = t + 9 >= w;
+    const int base = last ? nsrc : src + 32 * (t + 9), left = last ? (more ? nw : 0) : w - t - 9;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      gather((j + 1) % 3);
+      fma_chain<0>(w - t - 3 * j, v[j], g[j], s);
+      load(j, base, left);
+    }
+    if (last) {
+      done(s);
+      if (!more) break;
+      src = nsrc;
+      w = nw;
+      t = 0;
+      s = 0.0;
+      more = next(nsrc, nw);
+      begin();
+    } else {
+      t += 9;
+    }
+  }
+}
+
+template <bool SPLIT>
 __global__ void __launch_bounds__(PT, 1) k_pcg_stream(const __grid_constant__ PcgArgs a) {
   __shared__ PcgShared<PT> sh;
+  extern __shared__ __align__(16) unsigned char pcg_smem[];
+  double* const part = reinterpret_cast<double*>(pcg_smem);          // [unit][lane]
+  int2* const unit = reinterpret_cast<int2*>(part + 32 * a.units);   // first entry, entries per row
+  int* const begin = reinterpret_cast<int*>(unit + a.units);         // first unit of the block's slices
   if (entry_flag(&a.st->converged)) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int s0 = int((long long)a.nslices * blockIdx.x / gridDim.x);
-  const int s1 = int((long long)a.nslices * (blockIdx.x + 1) / gridDim.x);
+  const int s0 = a.first[blockIdx.x], s1 = a.first[blockIdx.x + 1];
   const int row1 = min(a.n, s1 * 32);
   const unsigned long long pol = matrix_policy(a.stream);
   if (threadIdx.x == 0) {
     sh.ex.fault = 0;
     sh.k.load(a.st);
   }
+  if (SPLIT) {
+    for (int k = threadIdx.x; k < s1 - s0; k += PT) begin[k + 1] = pcg_units(a.width[s0 + k]);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      begin[0] = 0;
+      for (int k = 0; k < s1 - s0; ++k) begin[k + 1] += begin[k];
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < s1 - s0; k += PT) {
+      const int w = a.width[s0 + k], n = pcg_units(w), each = (w + n - 1) / n, src = a.meta[s0 + k].x;
+      for (int u = 0; u < n; ++u) unit[begin[k] + u] = make_int2(src + 32 * each * u, min(each, w - each * u));
+    }
+    __syncthreads();
+  }
   unsigned int epoch = 0;
   while (true) {
     double v3[3] = {0.0, 0.0, 0.0};
-    for (int slice = s0 + warp; slice < s1; slice += PT / 32) {
+    if (SPLIT) {
+      int u = warp, out = warp;
+      pcg_segments(
+          a, pol,
+          [&](int& src, int& w) {
+            if (u >= begin[s1 - s0]) return false;
+            src = unit[u].x;
+            w = unit[u].y;
+            u += PT / 32;
+            return true;
+          },
+          [] {},
+          [&](double s) {
+            part[32 * out + lane] = s;
+            out += PT / 32;
+          });
+      __syncthreads();
+    }
+    // q of the slice's rows and their share of the sums
+    double pr = 0.0, rr = 0.0, dr = 0.0;
+    int slice = s0 + warp;
+    auto begin_row = [&] {
       const int row = slice * 32 + lane;
       const bool in = row < a.n;
-      const double pr = in ? a.p[row] : 0.0, rr = in ? a.r[row] : 0.0, dr = in ? __ldg(a.dinv + row) : 0.0;
-      const int src = __ldg(&a.meta[slice].x) + lane, w = __ldg(a.width + slice);
-      const double* gv = a.val + src;
-      const int* gc = a.col + src;
-      double s = 0.0;
-#pragma unroll 1
-      for (int t0 = 0; t0 < w; t0 += 9) {
-        double vv[9];
-        int cc[9];
-#pragma unroll
-        for (int j = 0; j < 9; ++j) {
-          const bool on = t0 + j < w;  // warp-uniform
-          vv[j] = on ? ld_matrix(gv + 32 * (t0 + j), pol) : 0.0;
-          cc[j] = on ? ld_matrix(gc + 32 * (t0 + j), pol) : 0;
-        }
-#pragma unroll
-        for (int j = 0; j < 9; ++j)
-          if (t0 + j < w) s = fma(vv[j], a.p[cc[j]], s);
-      }
-      if (in) a.q[row] = s;
+      pr = in ? a.p[row] : 0.0;
+      rr = in ? a.r[row] : 0.0;
+      dr = in ? __ldg(a.dinv + row) : 0.0;
+    };
+    auto end_row = [&](double s) {
+      const int row = slice * 32 + lane;
+      if (row < a.n) a.q[row] = s;
       const double ds = dr * s;
       v3[0] = fma(pr, s, v3[0]);
       v3[1] = fma(rr, ds, v3[1]);
       v3[2] = fma(s, ds, v3[2]);
+      slice += PT / 32;
+    };
+    if (SPLIT) {
+      while (slice < s1) {
+        begin_row();
+        const int u1 = begin[slice - s0 + 1];
+        int u = begin[slice - s0];
+        double s = part[32 * u + lane];
+        for (++u; u < u1; ++u) s += part[32 * u + lane];
+        end_row(s);
+      }
+    } else {
+      int ahead = slice;
+      pcg_segments(
+          a, pol,
+          [&](int& src, int& w) {
+            if (ahead >= s1) return false;
+            src = __ldg(&a.meta[ahead].x);
+            w = __ldg(a.width + ahead);
+            ahead += PT / 32;
+            return true;
+          },
+          begin_row, end_row);
     }
     if (!pcg_step(a, epoch, v3, PT / 32, sh)) break;
     const double alpha = sh.k.alpha, beta = sh.k.beta;
@@ -995,11 +1104,42 @@ __global__ void __launch_bounds__(PT, 1) k_pcg_stream(const __grid_constant__ Pc
 // Rows of at most 32 entries (the SELL-32 SpMV's limit). Per iteration, before (three counter barriers, shuffle
 // reductions, scalars in every thread) and now: 4,225 rows of Q1 squares 25.5 and 5.6 us; 68,921 of an
 // unstructured tetrahedral mesh 31.2 and 9.6; 98,304 of SWIPDG 26.0 and 9.9; 155,480 of P1 tetrahedra 29.7
-// and 11.5; 2,146,689 of 128^3 Q1 (streaming, 727.7 MB of matrix) 209 and 179. The graph form takes
+// and 11.5; 2,146,689 of 128^3 Q1 (streaming, 727.7 MB of matrix) 209 and 154
+// (178 before the gathers went ahead of the products). The graph form takes
 // 51.7 us for 393,216 rows of SWIPDG and 264 us for 128^3: AUTO takes this form wherever it applies.
+// Longer rows too where the form is left to the library (28^3 Q2 cubes, 185,193 rows of up to 125 entries: 60 us in
+// the graph form, 48 here; 15,625 rows 37 and 21); a caller who asks for the persistent form gets it for rows of at most 32.
 bool persistent_applies(gdt_context ctx, gdt_matrix m) {
   if (ctx->timing || ctx->solver_launch == GDT_SOLVER_LAUNCH_GRAPH) return false;
-  return m->max_row >= 1 && m->max_row <= 32 && m->rows >= 1;
+  return m->max_row >= 1 && m->rows >= 1 &&
+         (m->max_row <= 32 ||
+          (ctx->solver_launch == GDT_SOLVER_LAUNCH_AUTO && m->max_row <= 512 && !m->sell_padded));
+}
+
+// The slices of every block: equally many, unless rows of different lengths are numbered one kind after the other
+// (Q2: vertices, edges, faces, cells), where that leaves blocks with twice the average work; then equal
+// shares of entries + 10 per row (the vector operations). Returns the most slices of a block.
+int pcg_partition(gdt_matrix m, int blocks, int* first) {
+  const int n = int(m->sell_off.size()) - 1;
+  const auto work = [&](int s) { return m->sell_off[s] + 320LL * s; };
+  long long most = 0;
+  for (int b = 0; b <= blocks; ++b) {
+    first[b] = int((long long)n * b / blocks);
+    if (b > 0) most = std::max(most, work(first[b]) - work(first[b - 1]));
+  }
+  if (10 * most * blocks > 12 * work(n))
+    for (int b = 1; b < blocks; ++b) {
+      int lo = first[b - 1], hi = n;  // the first slice with at least b shares before it
+      while (lo < hi) {
+        const int mid = (lo + hi) / 2;
+        if (work(mid) * blocks < work(n) * b) lo = mid + 1;
+        else hi = mid;
+      }
+      first[b] = lo;
+    }
+  int slices = 0;
+  for (int b = 0; b < blocks; ++b) slices = std::max(slices, first[b + 1] - first[b]);
+  return slices;
 }
 
 // Runs the iterations after residual_init; the caller reads the final state from st. Returns
@@ -1020,20 +1160,49 @@ gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, d
   blocks = std::max(1, std::min(blocks, (nslices + 3) / 4));
   // slices per warp of the resident form; where a block has more rows than its registers hold, the
   // streaming form
-  const int per_warp = ((nslices + blocks - 1) / blocks + RT / 32 - 1) / (RT / 32);
+  GDT_CHECK(ctx, sell_table(ctx, m, s));
+  if (m->max_row > 32 && m->sell_len - m->nnz > m->nnz / 2 + 32768) {  // padding is work
+    m->sell_padded = true;
+    if (!m->use_sell) sell_free(m);
+    return GDT_EUNSUPPORTED;
+  }
+  PcgArgs a;
+  const int slices = pcg_partition(m, blocks, a.first);
+  const int per_warp = (slices + RT / 32 - 1) / (RT / 32);
   const void* fn = per_warp <= 1   ? reinterpret_cast<const void*>(&k_pcg_resident<1>)
                    : per_warp <= 2 ? reinterpret_cast<const void*>(&k_pcg_resident<2>)
                    : per_warp <= 4 ? reinterpret_cast<const void*>(&k_pcg_resident<4>)
                    : per_warp <= 8 ? reinterpret_cast<const void*>(&k_pcg_resident<8>)
                    : per_warp <= RMAX ? reinterpret_cast<const void*>(&k_pcg_resident<RMAX>)
-                                      : reinterpret_cast<const void*>(&k_pcg_stream);
-  const int threads = per_warp <= RMAX ? RT : PT;
+                                      : reinterpret_cast<const void*>(&k_pcg_stream<false>);
+  int threads = per_warp <= RMAX ? RT : PT;
   int cap = 0;
   size_t dyn = 0;
-  if (per_warp <= RMAX) {
+  a.units = 0;
+  // long rows: eight warps cannot hide the latency of what does not stay in shared memory (20^3 Q2 cubes, four slices a
+  // warp: 25 us an iteration resident, 33 streaming by slices; 24^3, eight: 48 resident, 38 streaming by units)
+  if (m->max_row > 32 && per_warp > 4) {
+    fn = reinterpret_cast<const void*>(&k_pcg_stream<false>);
+    threads = PT;
+    int most = 0;
+    for (int b = 0; b < blocks; ++b) {
+      int units = 0;
+      for (int k = a.first[b]; k < a.first[b + 1]; ++k) units += pcg_units((m->sell_off[k + 1] - m->sell_off[k]) / 32);
+      most = std::max(most, units);
+    }
+    cudaFuncAttributes fa;
+    GDT_TRY_CUDA(ctx, cudaFuncGetAttributes(&fa, reinterpret_cast<const void*>(&k_pcg_stream<true>)));
+    const size_t bytes = 264ull * most + 4ull * (slices + 1);
+    if (bytes + fa.sharedSizeBytes <= size_t(optin)) {  // (with more there are enough slices for every warp)
+      fn = reinterpret_cast<const void*>(&k_pcg_stream<true>);
+      a.units = most;
+      dyn = bytes;
+      GDT_TRY_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(dyn)));
+    }
+  } else if (per_warp <= RMAX) {
     cudaFuncAttributes fa;
     GDT_TRY_CUDA(ctx, cudaFuncGetAttributes(&fa, fn));
-    const long long want = 32LL * m->max_row * ((nslices + blocks - 1) / blocks);
+    const long long want = 32LL * m->max_row * slices;
     const long long room = (optin - (long long)fa.sharedSizeBytes) / 12 / 32 * 32;
     cap = int(std::max(0LL, std::min(want, room)));
     dyn = size_t(cap) * 12;
@@ -1046,9 +1215,7 @@ gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, d
     const gdt_status ss = sell_prepare_nonzero(ctx, m, s, width);
     if (ss != GDT_OK) return ss;
   }
-  PcgArgs a;
   a.n = int(m->rows);
-  a.nslices = nslices;
   a.meta = reinterpret_cast<const int2*>(m->sell_meta);
   a.width = width;
   a.col = m->sell_col;

@@ -103,11 +103,12 @@ void sell_free(gdt_matrix m) {
   m->sell_meta = m->sell_col = nullptr;
   m->sell_val = nullptr;
   m->sell_len = 0;
+  m->sell_off.clear();
   m->sell_version = -1;
 }
 
 // the slice table of the pattern and room for the copy (its values are filled by the callers below)
-static gdt_status sell_table(gdt_context ctx, gdt_matrix m, cudaStream_t s) {
+gdt_status sell_table(gdt_context ctx, gdt_matrix m, cudaStream_t s) {
   const int n = int(m->rows);
   const int nslices = (n + 31) / 32;
   const int blocks = (nslices * 32 + 255) / 256;
@@ -151,6 +152,9 @@ static gdt_status sell_table(gdt_context ctx, gdt_matrix m, cudaStream_t s) {
     m->sell_col = dcol;
     m->sell_val = dval;
     m->sell_len = off;
+    m->sell_off.resize(nslices + 1);
+    for (int i = 0; i < nslices; ++i) m->sell_off[i] = meta[2 * i];
+    m->sell_off[nslices] = int(off);
     m->sell_version = -1;
   }
   return GDT_OK;

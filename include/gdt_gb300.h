@@ -112,8 +112,8 @@ gdt_status gdt_measure_l2_bandwidth(gdt_context ctx, double* gbs);
  * captured in CUDA graphs. PERSISTENT: one cooperative launch runs every iteration, with grid
  * barriers between the steps and a SELL-32 copy of the matrix; it takes matrices whose rows hold at
  * most 32 entries. AUTO (default): PERSISTENT wherever it applies (it was faster both for systems
- * that stay in L2 and for ones streamed from HBM), GRAPH otherwise or where no cooperative launch or
- * no room for the copy is available. Timing mode always runs GRAPH's kernels launched one by one. */
+ * that stay in L2 and for ones streamed from HBM) and for rows of up to 512 entries that the copy pads by less
+ * than half, GRAPH otherwise or where no cooperative launch or no room for the copy is available. Timing mode always runs GRAPH's kernels launched one by one. */
 #define GDT_SOLVER_LAUNCH_AUTO 0
 #define GDT_SOLVER_LAUNCH_GRAPH 1
 #define GDT_SOLVER_LAUNCH_PERSISTENT 2
