@@ -111,6 +111,7 @@ struct gdt_matrix_s {
   double* sell_val = nullptr;
   long long sell_len = 0;
   std::vector<int> sell_off;    // the offsets on the host, sell_len last
+  int sell_band = 0;            // largest |column - row| of the pattern
   bool sell_padded = false;     // found too full of padding for the persistent CG
   long long val_version = 0;    // bumped by every entry point that may change the values
   long long sell_version = -1;  // val_version the SELL copy was filled at
@@ -190,7 +191,8 @@ gdt_status sell_prepare(gdt_context ctx, gdt_matrix m, cudaStream_t s, bool refi
 gdt_status sell_table(gdt_context ctx, gdt_matrix m, cudaStream_t s);
 // the copy without the zero values, for solves whose vectors are finite by their own checks (a product
 // keeps them: 0 * inf is not 0): width (device, one per 32-row slice) receives the entries per row
-gdt_status sell_prepare_nonzero(gdt_context ctx, gdt_matrix m, cudaStream_t s, int* width);
+// with `narrow` (sell_band of at most 32767) the columns are stored as 16-bit differences to the row
+gdt_status sell_prepare_nonzero(gdt_context ctx, gdt_matrix m, cudaStream_t s, int* width, bool narrow = false);
 void sell_free(gdt_matrix m);
 // index of the SELL-32 schedule in gdt_matrix_tune / gdt_matrix_set_schedule
 constexpr int kSellSchedule = 8;

@@ -676,6 +676,7 @@ struct PcgArgs {
   ExchangeView ex;    // the whole grid
   int cap;            // matrix entries a block may keep in shared memory (resident form)
   int stream;         // the matrix exceeds L2: mark its lines evict-first
+  int qshared;        // the streaming form keeps q in shared memory
   int units;          // the most units of a block (streaming form by units)
   int first[257];     // the block's slices: first[block] .. first[block + 1] - 1
 };
@@ -786,6 +787,11 @@ __device__ __forceinline__ unsigned long long matrix_policy(int stream) {
 __device__ __forceinline__ double ld_matrix(const double* a, unsigned long long pol) {
   double v;
   asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(a), "l"(pol));
+  return v;
+}
+__device__ __forceinline__ int ld_matrix(const short* a, unsigned long long pol) {
+  short v;
+  asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.s16 %0, [%1], %2;" : "=h"(v) : "l"(a), "l"(pol));
   return v;
 }
 __device__ __forceinline__ int ld_matrix(const int* a, unsigned long long pol) {
@@ -921,16 +927,16 @@ constexpr int kUnit = 36;
 
 __host__ __device__ constexpr int pcg_units(int width) { return width <= kUnit ? 1 : (width + kUnit - 1) / kUnit; }
 
-// The sums of a warp's segments (entries t < w of the lane's row at src + 32 t; next(src, w) gives them one after the
-// other, warp-uniform): begin() where a segment starts, done(sum) where it ends. Groups of nine entries in three
+// The sums of a warp's segments (entries t < w of the lane's row at src + 32 t, columns counted from `row`, 0 unless they
+// are 16-bit differences; next(src, w, row) gives them one after the other): begin() where a segment starts, done(sum) where it ends. Groups of nine entries in three
 // buffers: the entries are loaded three steps of three before their products and the vector is gathered one step
 // before, across the ends of segments, so that neither latency is waited for.
-template <class Next, class Begin, class Done>
+template <class Col, class Next, class Begin, class Done>
 __device__ __forceinline__ void pcg_segments(const PcgArgs& a, unsigned long long pol, Next next, Begin begin, Done done) {
   const int lane = threadIdx.x & 31;
-  int src, w, nsrc = 0, nw = 0;
-  if (!next(src, w)) return;
-  bool more = next(nsrc, nw);
+  int src, w, row, nsrc = 0, nw = 0, nrow = 0;
+  if (!next(src, w, row)) return;
+  bool more = next(nsrc, nw, nrow);
   double v[3][3], g[3][3];
   int c[3][3];
   auto load = [&](int j, int base, int left) {
@@ -938,16 +944,16 @@ __device__ __forceinline__ void pcg_segments(const PcgArgs& a, unsigned long lon
     for (int i = 0; i < 3; ++i) {
       const bool in = 3 * j + i < left;  // warp-uniform
       v[j][i] = in ? ld_matrix(a.val + base + lane + 32 * (3 * j + i), pol) : 0.0;
-      c[j][i] = in ? ld_matrix(a.col + base + lane + 32 * (3 * j + i), pol) : 0;
+      c[j][i] = in ? ld_matrix(reinterpret_cast<const Col*>(a.col) + base + lane + 32 * (3 * j + i), pol) : 0;
     }
   };
-  auto gather = [&](int j) {
+  auto gather = [&](int j, int from) {
 #pragma unroll
-    for (int i = 0; i < 3; ++i) g[j][i] = a.p[c[j][i]];
+    for (int i = 0; i < 3; ++i) g[j][i] = a.p[from + c[j][i]];
   };
 #pragma unroll
   for (int j = 0; j < 3; ++j) load(j, src, w);
-  gather(0);
+  gather(0, row);
   begin();
   double s = 0.0;
   for (int t = 0;;) {
@@ -955,7 +961,7 @@ __device__ __forceinline__ void pcg_segments(const PcgArgs& a, unsigned long lon
     const int base = last ? nsrc : src + 32 * (t + 9), left = last ? (more ? nw : 0) : w - t - 9;
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
-      gather((j + 1) % 3);
+      gather((j + 1) % 3, j == 2 && last ? nrow : row);
       fma_chain<0>(w - t - 3 * j, v[j], g[j], s);
       load(j, base, left);
     }
@@ -964,9 +970,10 @@ __device__ __forceinline__ void pcg_segments(const PcgArgs& a, unsigned long lon
       if (!more) break;
       src = nsrc;
       w = nw;
+      row = nrow;
       t = 0;
       s = 0.0;
-      more = next(nsrc, nw);
+      more = next(nsrc, nw, nrow);
       begin();
     } else {
       t += 9;
@@ -974,7 +981,7 @@ __device__ __forceinline__ void pcg_segments(const PcgArgs& a, unsigned long lon
   }
 }
 
-template <bool SPLIT>
+template <bool SPLIT, class Col>
 __global__ void __launch_bounds__(PT, 1) k_pcg_stream(const __grid_constant__ PcgArgs a) {
   __shared__ PcgShared<PT> sh;
   extern __shared__ __align__(16) unsigned char pcg_smem[];
@@ -985,6 +992,7 @@ __global__ void __launch_bounds__(PT, 1) k_pcg_stream(const __grid_constant__ Pc
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int s0 = a.first[blockIdx.x], s1 = a.first[blockIdx.x + 1];
   const int row1 = min(a.n, s1 * 32);
+  double* const q = !SPLIT && a.qshared ? reinterpret_cast<double*>(pcg_smem) : a.q + 32LL * s0;  // of row 32 s0 on
   const unsigned long long pol = matrix_policy(a.stream);
   if (threadIdx.x == 0) {
     sh.ex.fault = 0;
@@ -1009,9 +1017,10 @@ __global__ void __launch_bounds__(PT, 1) k_pcg_stream(const __grid_constant__ Pc
     double v3[3] = {0.0, 0.0, 0.0};
     if (SPLIT) {
       int u = warp, out = warp;
-      pcg_segments(
+      pcg_segments<Col>(
           a, pol,
-          [&](int& src, int& w) {
+          [&](int& src, int& w, int& row) {
+            row = 0;
             if (u >= begin[s1 - s0]) return false;
             src = unit[u].x;
             w = unit[u].y;
@@ -1037,7 +1046,7 @@ __global__ void __launch_bounds__(PT, 1) k_pcg_stream(const __grid_constant__ Pc
     };
     auto end_row = [&](double s) {
       const int row = slice * 32 + lane;
-      if (row < a.n) a.q[row] = s;
+      if (row < a.n) q[row - 32 * s0] = s;
       const double ds = dr * s;
       v3[0] = fma(pr, s, v3[0]);
       v3[1] = fma(rr, ds, v3[1]);
@@ -1055,10 +1064,11 @@ __global__ void __launch_bounds__(PT, 1) k_pcg_stream(const __grid_constant__ Pc
       }
     } else {
       int ahead = slice;
-      pcg_segments(
+      pcg_segments<Col>(
           a, pol,
-          [&](int& src, int& w) {
+          [&](int& src, int& w, int& row) {
             if (ahead >= s1) return false;
+            row = sizeof(Col) == 2 ? min(ahead * 32 + lane, a.n - 1) : 0;  // (in bounds where there is no row)
             src = __ldg(&a.meta[ahead].x);
             w = __ldg(a.width + ahead);
             ahead += PT / 32;
@@ -1077,7 +1087,7 @@ __global__ void __launch_bounds__(PT, 1) k_pcg_stream(const __grid_constant__ Pc
         const int i = i0 + u * PT;
         const bool in = i < row1;
         pv[u] = in ? a.p[i] : 0.0;
-        qv[u] = in ? a.q[i] : 0.0;
+        qv[u] = in ? q[i - 32 * s0] : 0.0;
         xv[u] = in ? a.x[i] : 0.0;
         rv[u] = in ? a.r[i] : 0.0;
         dv[u] = in ? __ldg(a.dinv + i) : 0.0;
@@ -1104,8 +1114,8 @@ __global__ void __launch_bounds__(PT, 1) k_pcg_stream(const __grid_constant__ Pc
 // Rows of at most 32 entries (the SELL-32 SpMV's limit). Per iteration, before (three counter barriers, shuffle
 // reductions, scalars in every thread) and now: 4,225 rows of Q1 squares 25.5 and 5.6 us; 68,921 of an
 // unstructured tetrahedral mesh 31.2 and 9.6; 98,304 of SWIPDG 26.0 and 9.9; 155,480 of P1 tetrahedra 29.7
-// and 11.5; 2,146,689 of 128^3 Q1 (streaming, 727.7 MB of matrix) 209 and 154
-// (178 before the gathers went ahead of the products). The graph form takes
+// and 11.5; 2,146,689 of 128^3 Q1 (streaming, 727.7 MB of matrix) 209 and 146
+// (178 before the gathers went ahead of the products, 154 with 32-bit columns). The graph form takes
 // 51.7 us for 393,216 rows of SWIPDG and 264 us for 128^3: AUTO takes this form wherever it applies.
 // Longer rows too where the form is left to the library (28^3 Q2 cubes, 185,193 rows of up to 125 entries: 60 us in
 // the graph form, 48 here; 15,625 rows 37 and 21); a caller who asks for the persistent form gets it for rows of at most 32.
@@ -1174,7 +1184,7 @@ gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, d
                    : per_warp <= 4 ? reinterpret_cast<const void*>(&k_pcg_resident<4>)
                    : per_warp <= 8 ? reinterpret_cast<const void*>(&k_pcg_resident<8>)
                    : per_warp <= RMAX ? reinterpret_cast<const void*>(&k_pcg_resident<RMAX>)
-                                      : reinterpret_cast<const void*>(&k_pcg_stream<false>);
+                                      : reinterpret_cast<const void*>(&k_pcg_stream<false, int>);
   int threads = per_warp <= RMAX ? RT : PT;
   int cap = 0;
   size_t dyn = 0;
@@ -1182,7 +1192,7 @@ gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, d
   // long rows: eight warps cannot hide the latency of what does not stay in shared memory (20^3 Q2 cubes, four slices a
   // warp: 25 us an iteration resident, 33 streaming by slices; 24^3, eight: 48 resident, 38 streaming by units)
   if (m->max_row > 32 && per_warp > 4) {
-    fn = reinterpret_cast<const void*>(&k_pcg_stream<false>);
+    fn = reinterpret_cast<const void*>(&k_pcg_stream<false, int>);
     threads = PT;
     int most = 0;
     for (int b = 0; b < blocks; ++b) {
@@ -1191,10 +1201,10 @@ gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, d
       most = std::max(most, units);
     }
     cudaFuncAttributes fa;
-    GDT_TRY_CUDA(ctx, cudaFuncGetAttributes(&fa, reinterpret_cast<const void*>(&k_pcg_stream<true>)));
+    GDT_TRY_CUDA(ctx, cudaFuncGetAttributes(&fa, reinterpret_cast<const void*>(&k_pcg_stream<true, int>)));
     const size_t bytes = 264ull * most + 4ull * (slices + 1);
     if (bytes + fa.sharedSizeBytes <= size_t(optin)) {  // (with more there are enough slices for every warp)
-      fn = reinterpret_cast<const void*>(&k_pcg_stream<true>);
+      fn = reinterpret_cast<const void*>(&k_pcg_stream<true, int>);
       a.units = most;
       dyn = bytes;
       GDT_TRY_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(dyn)));
@@ -1208,11 +1218,26 @@ gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, d
     dyn = size_t(cap) * 12;
     GDT_TRY_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(dyn)));
   }
+  // streaming by slices: the columns as 16-bit differences where they fit (10 bytes an entry instead of 12), q in shared
+  // memory where it fits. 128^3 Q1: 165 us an iteration, 160 and 161 with one of them, 156 with both; 91^3
+  // rows, which L2 holds better: 63 and 62.
+  const bool narrow = fn == reinterpret_cast<const void*>(&k_pcg_stream<false, int>) && m->sell_band <= 32767;
+  if (narrow) fn = reinterpret_cast<const void*>(&k_pcg_stream<false, short>);
+  a.qshared = 0;
+  if (threads == PT && a.units == 0) {
+    cudaFuncAttributes fa;
+    GDT_TRY_CUDA(ctx, cudaFuncGetAttributes(&fa, fn));
+    if (256ull * slices + fa.sharedSizeBytes <= size_t(optin)) {
+      a.qshared = 1;
+      dyn = 256ull * slices;
+      GDT_TRY_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(dyn)));
+    }
+  }
   GDT_TRY_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, dyn));
   if (per_sm < 1) return GDT_EUNSUPPORTED;
   {
     // the values are copied at every solve: the caller may have written them through the CSR pointer
-    const gdt_status ss = sell_prepare_nonzero(ctx, m, s, width);
+    const gdt_status ss = sell_prepare_nonzero(ctx, m, s, width, narrow);
     if (ss != GDT_OK) return ss;
   }
   a.n = int(m->rows);

@@ -41,14 +41,21 @@ template void launch_spmv<float>(int, int, const int*, const int*, const float*,
                                  cudaStream_t);
 
 // ------------------------------------------------------------------------------ SELL-32 ---
-// widths: one warp per slice, the longest row of its 32
-__global__ void k_sell_width(int n, int nslices, const int* __restrict__ rp, int* __restrict__ width) {
+// widths: one warp per slice, the longest row of its 32; and the largest |column - row| to band
+__global__ void k_sell_width(int n, int nslices, const int* __restrict__ rp, const int* __restrict__ col,
+                             int* __restrict__ width, int* __restrict__ band) {
   const int slice = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (slice >= nslices) return;
   const int row = slice * 32 + (threadIdx.x & 31);
   const int len = row < n ? rp[row + 1] - rp[row] : 0;
   const int w = __reduce_max_sync(0xffffffffu, len);
-  if ((threadIdx.x & 31) == 0) width[slice] = w;
+  int far = 0;
+  for (int t = 0; t < len; ++t) far = max(far, abs(col[rp[row] + t] - row));
+  far = __reduce_max_sync(0xffffffffu, far);
+  if ((threadIdx.x & 31) == 0) {
+    width[slice] = w;
+    atomicMax(band, far);
+  }
 }
 
 // values and columns from the CSR arrays; padding entries are 0 * x[row] (row 0 past the end)
@@ -70,27 +77,29 @@ __global__ void k_sell_fill(int n, int nslices, const int* __restrict__ rp, cons
 
 // the same with the zero values left out: width[slice] = the most nonzeros of a row of the slice; a row's
 // entries beyond its own nonzeros (and beyond width) are padding, those beyond width are not written
+template <class Col>
 __global__ void k_sell_fill_nonzero(int n, int nslices, const int* __restrict__ rp, const int* __restrict__ col,
                                     const double* __restrict__ val, const int2* __restrict__ meta,
-                                    int* __restrict__ scol, double* __restrict__ sval, int* __restrict__ width) {
+                                    Col* __restrict__ scol, double* __restrict__ sval, int* __restrict__ width) {
   const int slice = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (slice >= nslices) return;
   const int lane = threadIdx.x & 31;
   const int row = slice * 32 + lane;
   const long long base = (long long)meta[slice].x + lane;
+  const int zero = sizeof(Col) == 2 ? row : 0;
   const int beg = row < n ? rp[row] : 0, end = row < n ? rp[row + 1] : 0;
   int t = 0;
   for (int k = beg; k < end; ++k) {
     const double v = val[k];
     if (v != 0.0) {
-      scol[base + 32LL * t] = col[k];
+      scol[base + 32LL * t] = Col(col[k] - zero);
       sval[base + 32LL * t] = v;
       ++t;
     }
   }
   const int w = __reduce_max_sync(0xffffffffu, t);
   for (; t < w; ++t) {
-    scol[base + 32LL * t] = row < n ? row : 0;
+    scol[base + 32LL * t] = Col(row < n ? row - zero : 0);
     sval[base + 32LL * t] = 0.0;
   }
   if (lane == 0) width[slice] = w;
@@ -114,14 +123,16 @@ gdt_status sell_table(gdt_context ctx, gdt_matrix m, cudaStream_t s) {
   const int blocks = (nslices * 32 + 255) / 256;
   if (!m->sell_meta) {
     int* width = nullptr;
-    if (cudaMalloc(&width, sizeof(int) * nslices) != cudaSuccess) {
+    if (cudaMalloc(&width, sizeof(int) * (nslices + 1)) != cudaSuccess) {
       cudaGetLastError();
       return GDT_EUNSUPPORTED;
     }
-    k_sell_width<<<blocks, 256, 0, s>>>(n, nslices, m->rp, width);
+    std::vector<int> w(nslices + 1);
+    cudaError_t e = cudaMemsetAsync(width + nslices, 0, sizeof(int), s);
+    k_sell_width<<<blocks, 256, 0, s>>>(n, nslices, m->rp, m->col, width, width + nslices);
     ctx->launches++;
-    std::vector<int> w(nslices);
-    cudaError_t e = cudaMemcpyAsync(w.data(), width, sizeof(int) * nslices, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(w.data(), width, sizeof(int) * (nslices + 1), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     cudaFree(width);
     if (e != cudaSuccess) return fail(ctx, GDT_ECUDA, std::string("sell widths: ") + cudaGetErrorString(e));
@@ -152,6 +163,7 @@ gdt_status sell_table(gdt_context ctx, gdt_matrix m, cudaStream_t s) {
     m->sell_col = dcol;
     m->sell_val = dval;
     m->sell_len = off;
+    m->sell_band = w[nslices];
     m->sell_off.resize(nslices + 1);
     for (int i = 0; i < nslices; ++i) m->sell_off[i] = meta[2 * i];
     m->sell_off[nslices] = int(off);
@@ -173,13 +185,18 @@ gdt_status sell_prepare(gdt_context ctx, gdt_matrix m, cudaStream_t s, bool refi
   return GDT_OK;
 }
 
-gdt_status sell_prepare_nonzero(gdt_context ctx, gdt_matrix m, cudaStream_t s, int* width) {
+gdt_status sell_prepare_nonzero(gdt_context ctx, gdt_matrix m, cudaStream_t s, int* width, bool narrow) {
   const gdt_status st = sell_table(ctx, m, s);
   if (st != GDT_OK) return st;
   const int n = int(m->rows), nslices = (n + 31) / 32;
   m->sell_version = -1;  // not the full copy: the next reader of that one refills it
-  k_sell_fill_nonzero<<<(nslices * 32 + 255) / 256, 256, 0, s>>>(
-      n, nslices, m->rp, m->col, m->val, reinterpret_cast<const int2*>(m->sell_meta), m->sell_col, m->sell_val, width);
+  const int blocks = (nslices * 32 + 255) / 256;
+  const int2* meta = reinterpret_cast<const int2*>(m->sell_meta);
+  if (narrow)
+    k_sell_fill_nonzero<<<blocks, 256, 0, s>>>(n, nslices, m->rp, m->col, m->val, meta,
+                                               reinterpret_cast<short*>(m->sell_col), m->sell_val, width);
+  else
+    k_sell_fill_nonzero<<<blocks, 256, 0, s>>>(n, nslices, m->rp, m->col, m->val, meta, m->sell_col, m->sell_val, width);
   return check_launch(ctx, "sell fill");
 }
 
