@@ -870,8 +870,8 @@ gdt_status assemble_cg_mapped(gdt_context ctx, const GridDesc& g, const int* rp,
   cudaStream_t s = ctx->stream;
   double* tm = nullptr;
   double* tb = nullptr;
-  if ((val && cudaMallocAsync(&tm, sizeof(double) * size_t(np) * g.ncells, s) != cudaSuccess) ||
-      (rhs && cudaMallocAsync(&tb, sizeof(double) * size_t(nb) * g.ncells, s) != cudaSuccess)) {
+  if ((val && pool_malloc(ctx, &tm, sizeof(double) * size_t(np) * g.ncells, s) != cudaSuccess) ||
+      (rhs && pool_malloc(ctx, &tb, sizeof(double) * size_t(nb) * g.ncells, s) != cudaSuccess)) {
     cudaGetLastError();
     if (tm) cudaFreeAsync(tm, s);
     return fail(ctx, GDT_ENOMEM, "mapped assembly tables");

@@ -91,6 +91,17 @@ gdt_status gdt_context_create(int device, void* stream, gdt_context* out) {
     gdt_context_destroy(ctx);
     return GDT_ECUDA;
   }
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = device;
+  if (cudaMemPoolCreate(&ctx->pool, &props) == cudaSuccess) {
+    unsigned long long keep = kPoolBytes;
+    cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  } else {
+    ctx->pool = nullptr;  // the device's default pool
+    cudaGetLastError();
+  }
   *out = ctx;
   return GDT_OK;
 }
@@ -146,6 +157,8 @@ gdt_status gdt_context_destroy(gdt_context ctx) {
   if (ctx->scratch) cudaFree(ctx->scratch);
   if (ctx->counters) cudaFree(ctx->counters);
   if (ctx->host_pinned) cudaFreeHost(ctx->host_pinned);
+  if (ctx->own) cudaStreamDestroy(ctx->own);
+  if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
   delete ctx;
   return GDT_OK;
 }

@@ -30,7 +30,7 @@ struct ExchangeView {
 template <int T>
 struct ExchangeShared {
   double part[3][T];
-  double packet[3][T];  // of block first + b at [..][b]
+  double packet[3][T];  // of block first + b at [..][b]; cluster_exchange: [epoch & 1][3][16], written by the blocks
   double own[3];
   int fault;  // set by the caller to 0 before the first exchange
 };
@@ -147,6 +147,40 @@ __device__ __forceinline__ double group_exchange_f32(const ExchangeView& ex, uns
     if (warp == 0 && lane >= (int)(blockDim.x >> 5)) sh.part[k][lane] = 0.0;
   }
   return exchange_stored<RELEASE, NV>(ex, epoch, 1, sh);
+}
+
+// group_exchange for the blocks of one cluster (at most 16, the grid): the block sums go to the other blocks' shared
+// memory, and the cluster's barrier, which releases the writes of all threads, is the only wait (the
+// hardware's: the blocks of a cluster run together, and all take the same decisions from the same bits).
+template <int NV, int T>
+__device__ __forceinline__ double cluster_exchange(unsigned int& epoch, const double (&v)[NV], int warps,
+                                                   ExchangeShared<T>& sh) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  static_assert(3 * T >= 2 * 3 * 16, "two buffers");
+  ++epoch;
+  double* const remote = &sh.packet[0][0] + 16 * (3 * (epoch & 1) + warp);
+  if (warp < warps) {
+#pragma unroll
+    for (int k = 0; k < NV; ++k) sh.part[k][threadIdx.x] = v[k];
+  }
+  __syncthreads();
+  if (warp < NV) {
+    const double b = sum_strided(sh.part[warp] + lane, warps);
+    const unsigned int here = static_cast<unsigned int>(__cvta_generic_to_shared(remote + blockIdx.x));
+    unsigned int there;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(here), "r"(min(lane, int(gridDim.x) - 1)));
+    if (lane < (int)gridDim.x) asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(there), "d"(b) : "memory");
+    __syncwarp();
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  double b = 0.0;
+  if (warp < NV) {
+    b = lane < (int)gridDim.x ? remote[lane] : 0.0;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) b += __shfl_xor_sync(0xffffffffu, b, o);
+    b = __shfl_sync(0xffffffffu, b, 0);
+  }
+  return b;
 }
 
 // The barrier alone, releasing the block's writes; thread 0 runs `meanwhile` between its arrival and its wait.

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdint>
 #include <memory>
 #include <string>
@@ -47,6 +48,8 @@ struct GridDesc {
 struct gdt_context_s {
   int device = 0;
   cudaStream_t stream = nullptr;
+  std::atomic<cudaStream_t> own{nullptr};  // blocking stream for a solve on the legacy stream, left by the last one
+  cudaMemPool_t pool = nullptr;   // temporary memory; keeps at most kPoolBytes between calls
   std::string last_error;
   long long launches = 0;
   // small device scratch for reductions and solver scalars
@@ -129,6 +132,28 @@ struct gdt_matrix_s {
 namespace gdt {
 
 constexpr int kScratchDoubles = 1 << 16;
+// The default pool gives everything back at every synchronisation: a small solve spent 360 us outside its iterations,
+// most of it on mapping its vectors anew and on a stream of its own; with both kept 138 us.
+constexpr unsigned long long kPoolBytes = 256ull << 20;
+
+// Lets a launch of fn ask for all the dynamic shared memory there is: room = what is left beside its static memory. Always
+// the same limit, since a launch of another thread may come between this and its own.
+inline cudaError_t allow_shared(gdt_context ctx, const void* fn, long long* room) {
+  int optin = 0;
+  cudaFuncAttributes fa;
+  cudaError_t e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, fn);
+  if (e != cudaSuccess) return e;
+  *room = optin - (long long)fa.sharedSizeBytes;
+  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(*room));
+}
+
+// temporary memory in the order of stream s, freed with cudaFreeAsync
+template <class T>
+inline cudaError_t pool_malloc(gdt_context ctx, T** p, size_t bytes, cudaStream_t s) {
+  if (!ctx->pool) return cudaMallocAsync(reinterpret_cast<void**>(p), bytes, s);
+  return cudaMallocFromPoolAsync(reinterpret_cast<void**>(p), bytes, ctx->pool, s);
+}
 constexpr int kCounters = 64;
 
 gdt_status fail(gdt_context ctx, gdt_status s, const std::string& msg);

@@ -603,10 +603,10 @@ gdt_status ilu_setup(gdt_context ctx, gdt_matrix m, Ilu& f, cudaStream_t s) {
   std::vector<int> lo, uo;
   level_sets(n, rp, col, false, lo, f.loff);
   level_sets(n, rp, col, true, uo, f.uoff);
-  GDT_TRY_CUDA(ctx, cudaMallocAsync(&f.lu, sizeof(double) * m->nnz, s));
-  GDT_TRY_CUDA(ctx, cudaMallocAsync(&f.diag, sizeof(int) * n, s));
-  GDT_TRY_CUDA(ctx, cudaMallocAsync(&f.lorder, sizeof(int) * n, s));
-  GDT_TRY_CUDA(ctx, cudaMallocAsync(&f.uorder, sizeof(int) * n, s));
+  GDT_TRY_CUDA(ctx, pool_malloc(ctx, &f.lu, sizeof(double) * m->nnz, s));
+  GDT_TRY_CUDA(ctx, pool_malloc(ctx, &f.diag, sizeof(int) * n, s));
+  GDT_TRY_CUDA(ctx, pool_malloc(ctx, &f.lorder, sizeof(int) * n, s));
+  GDT_TRY_CUDA(ctx, pool_malloc(ctx, &f.uorder, sizeof(int) * n, s));
   GDT_TRY_CUDA(ctx, cudaMemcpyAsync(f.lorder, lo.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s));
   GDT_TRY_CUDA(ctx, cudaMemcpyAsync(f.uorder, uo.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s));
   GDT_TRY_CUDA(ctx, cudaMemcpyAsync(f.lu, m->val, sizeof(double) * m->nnz, cudaMemcpyDeviceToDevice, s));
@@ -718,11 +718,13 @@ struct PcgShared {
 // v = (p.q, z.q, q.D^-1 q) over the rows of the thread: alpha and beta in sh.k; false when done. The stopping test
 // of the iteration before is made here too: its sums (sh.last) are formed while the other warps
 // already multiply, so a solve ends with one product it does not use.
-template <int T>
+template <bool CLUSTER, int T>
 __device__ __forceinline__ bool pcg_step(const PcgArgs& a, unsigned int& epoch, const double (&v)[3], int warps,
                                          PcgShared<T>& sh) {
   const bool first = epoch == 0;
-  const double total = group_exchange<false>(a.ex, epoch, v, warps, sh.ex);
+  double total;
+  if constexpr (CLUSTER) total = cluster_exchange(epoch, v, warps, sh.ex);
+  else total = group_exchange<false>(a.ex, epoch, v, warps, sh.ex);
   if (threadIdx.x < 96) {
     const double inv = threadIdx.x == 0 ? 1.0 / total : 0.0;
     if ((threadIdx.x & 31) == 0) sh.total[threadIdx.x >> 5] = total;
@@ -749,10 +751,12 @@ __device__ __forceinline__ bool pcg_step(const PcgArgs& a, unsigned int& epoch, 
 }
 
 // v = (r.z, r.r) of the updated residual; p is visible to every block from here on
-template <int T>
+template <bool CLUSTER, int T>
 __device__ __forceinline__ void pcg_publish(const PcgArgs& a, unsigned int& epoch, const double (&v)[2], int warps,
                                             PcgShared<T>& sh) {
-  const double total = group_exchange<true>(a.ex, epoch, v, warps, sh.ex);
+  double total;
+  if constexpr (CLUSTER) total = cluster_exchange(epoch, v, warps, sh.ex);
+  else total = group_exchange<true>(a.ex, epoch, v, warps, sh.ex);
   if (threadIdx.x < 64 && (threadIdx.x & 31) == 0) sh.last[threadIdx.x >> 5] = total;
 }
 
@@ -803,10 +807,13 @@ __device__ __forceinline__ int ld_matrix(const int* a, unsigned long long pol) {
 // The resident form: one block of RT threads per SM, a contiguous range of slices per block, R slices per
 // warp, everything a row needs in registers. Two warps per scheduler keep the FP64 pipe busy (a dependent
 // FMA can issue as soon as the pipe is free), and each warp more would add its 32 values to every block sum.
+// CLUSTER: the grid is one cluster of at most 16 blocks, and the sums go through their shared memory.
 constexpr int RT = 256;
 constexpr int RMAX = 16;
+constexpr int kClusterSlices = 160;
+static_assert(kClusterSlices <= 2 * 16 * RT / 32, "two slices per warp");
 
-template <int R>
+template <int R, bool CLUSTER>
 __global__ void __launch_bounds__(RT, 1) k_pcg_resident(const __grid_constant__ PcgArgs a) {
   __shared__ PcgShared<RT> sh;
   __shared__ int s_off[RT / 32 * R + 1];
@@ -842,6 +849,8 @@ __global__ void __launch_bounds__(RT, 1) k_pcg_resident(const __grid_constant__ 
   }
   __syncthreads();
   const unsigned long long pol = matrix_policy(a.stream);
+  // (no block writes to the shared memory of one that has not started)
+  if (CLUSTER) asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   double x[R], r[R], p[R], d[R];
 #pragma unroll
   for (int k = 0; k < R; ++k) {
@@ -888,7 +897,7 @@ __global__ void __launch_bounds__(RT, 1) k_pcg_resident(const __grid_constant__ 
         v3[1] = fma(r[i], dq, v3[1]);
         v3[2] = fma(q[i], dq, v3[2]);
       }
-    if (!pcg_step(a, epoch, v3, warps, sh)) break;
+    if (!pcg_step<CLUSTER>(a, epoch, v3, warps, sh)) break;
     const double alpha = sh.k.alpha, beta = sh.k.beta;
     double v[2] = {0.0, 0.0};
 #pragma unroll
@@ -905,7 +914,7 @@ __global__ void __launch_bounds__(RT, 1) k_pcg_resident(const __grid_constant__ 
         v[1] = fma(r[i], r[i], v[1]);
       }
     }
-    pcg_publish(a, epoch, v, warps, sh);
+    pcg_publish<CLUSTER>(a, epoch, v, warps, sh);
   }
 #pragma unroll
   for (int i = 0; i < R; ++i) {
@@ -1076,7 +1085,7 @@ __global__ void __launch_bounds__(PT, 1) k_pcg_stream(const __grid_constant__ Pc
           },
           begin_row, end_row);
     }
-    if (!pcg_step(a, epoch, v3, PT / 32, sh)) break;
+    if (!pcg_step<false>(a, epoch, v3, PT / 32, sh)) break;
     const double alpha = sh.k.alpha, beta = sh.k.beta;
     double v[2] = {0.0, 0.0};
     // (two rows per thread and pass, all their loads issued before the first store)
@@ -1106,7 +1115,7 @@ __global__ void __launch_bounds__(PT, 1) k_pcg_stream(const __grid_constant__ Pc
         }
       }
     }
-    pcg_publish(a, epoch, v, PT / 32, sh);
+    pcg_publish<false>(a, epoch, v, PT / 32, sh);
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) sh.k.store(a.st);
 }
@@ -1129,7 +1138,7 @@ bool persistent_applies(gdt_context ctx, gdt_matrix m) {
 // The slices of every block: equally many, unless rows of different lengths are numbered one kind after the other
 // (Q2: vertices, edges, faces, cells), where that leaves blocks with twice the average work; then equal
 // shares of entries + 10 per row (the vector operations). Returns the most slices of a block.
-int pcg_partition(gdt_matrix m, int blocks, int* first) {
+int pcg_partition(gdt_matrix m, int blocks, bool by_work, int* first) {
   const int n = int(m->sell_off.size()) - 1;
   const auto work = [&](int s) { return m->sell_off[s] + 320LL * s; };
   long long most = 0;
@@ -1137,7 +1146,7 @@ int pcg_partition(gdt_matrix m, int blocks, int* first) {
     first[b] = int((long long)n * b / blocks);
     if (b > 0) most = std::max(most, work(first[b]) - work(first[b - 1]));
   }
-  if (10 * most * blocks > 12 * work(n))
+  if (by_work && 10 * most * blocks > 12 * work(n))
     for (int b = 1; b < blocks; ++b) {
       int lo = first[b - 1], hi = n;  // the first slice with at least b shares before it
       while (lo < hi) {
@@ -1157,10 +1166,10 @@ int pcg_partition(gdt_matrix m, int blocks, int* first) {
 // (the caller then runs the graph form).
 gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, double* p, double* q, int* width,
                           const double* dinv, KState* st, cudaStream_t s) {
-  int dev = 0, coop = 0, per_sm = 0, optin = 0;
+  int dev = 0, coop = 0, per_sm = 0;
+  long long room = 0;
   GDT_TRY_CUDA(ctx, cudaGetDevice(&dev));
   GDT_TRY_CUDA(ctx, cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-  GDT_TRY_CUDA(ctx, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   if (!coop) return GDT_EUNSUPPORTED;  // the caller runs the graph form
   int blocks = std::min(ctx->num_sms, RT);  // one block per SM
   if (ctx->persistent_blocks > 0) blocks = std::min(blocks, ctx->persistent_blocks);
@@ -1168,6 +1177,12 @@ gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, d
   // four slices, one per scheduler, before the next block: 4,225 rows in 34 blocks of four warps take 5.6 us
   // an iteration, in 133 blocks of one warp 6.0 us
   blocks = std::max(1, std::min(blocks, (nslices + 3) / 4));
+  // Small systems on one cluster, unless the caller has set limits, which are the grid's. Per iteration on the grid and
+  // on a cluster: 20 slices of Q1 squares 4.6 and 3.5 us, 133 5.55 and 5.25, 259 5.6 and 6.3; 42 slices
+  // of Q1 cubes 6.3 and 4.7, 106 6.4 and 5.6, 215 6.6 and 8.1 (16 SMs' FP64 pipes).
+  const bool cluster = ctx->persistent_blocks == 0 && ctx->persistent_wait_ns == 0 && m->max_row <= 32 &&
+                       nslices <= kClusterSlices;
+  if (cluster) blocks = std::min(16, std::max(1, nslices / 4));
   // slices per warp of the resident form; where a block has more rows than its registers hold, the
   // streaming form
   GDT_CHECK(ctx, sell_table(ctx, m, s));
@@ -1177,14 +1192,17 @@ gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, d
     return GDT_EUNSUPPORTED;
   }
   PcgArgs a;
-  const int slices = pcg_partition(m, blocks, a.first);
+  const int slices = pcg_partition(m, blocks, !cluster, a.first);
   const int per_warp = (slices + RT / 32 - 1) / (RT / 32);
-  const void* fn = per_warp <= 1   ? reinterpret_cast<const void*>(&k_pcg_resident<1>)
-                   : per_warp <= 2 ? reinterpret_cast<const void*>(&k_pcg_resident<2>)
-                   : per_warp <= 4 ? reinterpret_cast<const void*>(&k_pcg_resident<4>)
-                   : per_warp <= 8 ? reinterpret_cast<const void*>(&k_pcg_resident<8>)
-                   : per_warp <= RMAX ? reinterpret_cast<const void*>(&k_pcg_resident<RMAX>)
+  const void* fn = per_warp <= 1   ? reinterpret_cast<const void*>(&k_pcg_resident<1, false>)
+                   : per_warp <= 2 ? reinterpret_cast<const void*>(&k_pcg_resident<2, false>)
+                   : per_warp <= 4 ? reinterpret_cast<const void*>(&k_pcg_resident<4, false>)
+                   : per_warp <= 8 ? reinterpret_cast<const void*>(&k_pcg_resident<8, false>)
+                   : per_warp <= RMAX ? reinterpret_cast<const void*>(&k_pcg_resident<RMAX, false>)
                                       : reinterpret_cast<const void*>(&k_pcg_stream<false, int>);
+  if (cluster)
+    fn = per_warp <= 1 ? reinterpret_cast<const void*>(&k_pcg_resident<1, true>)
+                       : reinterpret_cast<const void*>(&k_pcg_resident<2, true>);
   int threads = per_warp <= RMAX ? RT : PT;
   int cap = 0;
   size_t dyn = 0;
@@ -1200,23 +1218,20 @@ gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, d
       for (int k = a.first[b]; k < a.first[b + 1]; ++k) units += pcg_units((m->sell_off[k + 1] - m->sell_off[k]) / 32);
       most = std::max(most, units);
     }
-    cudaFuncAttributes fa;
-    GDT_TRY_CUDA(ctx, cudaFuncGetAttributes(&fa, reinterpret_cast<const void*>(&k_pcg_stream<true, int>)));
-    const size_t bytes = 264ull * most + 4ull * (slices + 1);
-    if (bytes + fa.sharedSizeBytes <= size_t(optin)) {  // (with more there are enough slices for every warp)
+    GDT_TRY_CUDA(ctx, allow_shared(ctx, reinterpret_cast<const void*>(&k_pcg_stream<true, int>), &room));
+    const long long bytes = 264LL * most + 4LL * (slices + 1);
+    if (bytes <= room) {  // (with more there are enough slices for every warp)
       fn = reinterpret_cast<const void*>(&k_pcg_stream<true, int>);
       a.units = most;
-      dyn = bytes;
-      GDT_TRY_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(dyn)));
+      dyn = size_t(bytes);
     }
   } else if (per_warp <= RMAX) {
-    cudaFuncAttributes fa;
-    GDT_TRY_CUDA(ctx, cudaFuncGetAttributes(&fa, fn));
-    const long long want = 32LL * m->max_row * slices;
-    const long long room = (optin - (long long)fa.sharedSizeBytes) / 12 / 32 * 32;
-    cap = int(std::max(0LL, std::min(want, room)));
+    GDT_TRY_CUDA(ctx, allow_shared(ctx, fn, &room));
+    long long want = 0;  // no more than the block with the most entries has: the rest is L1 for the gathers
+    for (int b = 0; b < blocks; ++b)
+      want = std::max(want, (long long)m->sell_off[a.first[b + 1]] - m->sell_off[a.first[b]]);
+    cap = int(std::max(0LL, std::min(want, room / 12 / 32 * 32)));
     dyn = size_t(cap) * 12;
-    GDT_TRY_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(dyn)));
   }
   // streaming by slices: the columns as 16-bit differences where they fit (10 bytes an entry instead of 12), q in shared
   // memory where it fits. 128^3 Q1: 165 us an iteration, 160 and 161 with one of them, 156 with both; 91^3
@@ -1225,15 +1240,31 @@ gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, d
   if (narrow) fn = reinterpret_cast<const void*>(&k_pcg_stream<false, short>);
   a.qshared = 0;
   if (threads == PT && a.units == 0) {
-    cudaFuncAttributes fa;
-    GDT_TRY_CUDA(ctx, cudaFuncGetAttributes(&fa, fn));
-    if (256ull * slices + fa.sharedSizeBytes <= size_t(optin)) {
+    GDT_TRY_CUDA(ctx, allow_shared(ctx, fn, &room));
+    if (256LL * slices <= room) {
       a.qshared = 1;
-      dyn = 256ull * slices;
-      GDT_TRY_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(dyn)));
+      dyn = size_t(256) * slices;
     }
   }
-  GDT_TRY_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, dyn));
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = dyn;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  if (cluster) {
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = blocks;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    GDT_TRY_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    GDT_TRY_CUDA(ctx, cudaOccupancyMaxActiveClusters(&per_sm, fn, &cfg));
+  } else {
+    attr.id = cudaLaunchAttributeCooperative;
+    attr.val.cooperative = 1;
+    GDT_TRY_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, dyn));
+  }
   if (per_sm < 1) return GDT_EUNSUPPORTED;
   {
     // the values are copied at every solve: the caller may have written them through the CSR pointer
@@ -1264,7 +1295,7 @@ gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, d
   a.stream = 12LL * m->sell_len > (64LL << 20);
   GDT_TRY_CUDA(ctx, cudaMemsetAsync(words, 0, sizeof(unsigned long long) * (packets + 16), s));
   void* args[] = {&a};
-  const cudaError_t le = cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(threads), args, dyn, s);
+  const cudaError_t le = cudaLaunchKernelExC(&cfg, fn, args);
   if (le == cudaErrorCooperativeLaunchTooLarge) {  // fewer SMs available than the device has
     cudaGetLastError();
     return GDT_EUNSUPPORTED;
@@ -1304,12 +1335,12 @@ gdt_status tune_cg(gdt_context ctx, gdt_matrix m, const Launch& L0, cudaStream_t
   const size_t vb = sizeof(double) * std::max(n, 1);
   double *x = nullptr, *r = nullptr, *p = nullptr, *q = nullptr, *d = nullptr;
   KState* st = nullptr;
-  GDT_TRY_CUDA(ctx, cudaMallocAsync(&x, vb, s));
-  GDT_TRY_CUDA(ctx, cudaMallocAsync(&r, vb, s));
-  GDT_TRY_CUDA(ctx, cudaMallocAsync(&p, vb, s));
-  GDT_TRY_CUDA(ctx, cudaMallocAsync(&q, vb, s));
-  GDT_TRY_CUDA(ctx, cudaMallocAsync(&d, vb, s));
-  GDT_TRY_CUDA(ctx, cudaMallocAsync(&st, sizeof(KState), s));
+  GDT_TRY_CUDA(ctx, pool_malloc(ctx, &x, vb, s));
+  GDT_TRY_CUDA(ctx, pool_malloc(ctx, &r, vb, s));
+  GDT_TRY_CUDA(ctx, pool_malloc(ctx, &p, vb, s));
+  GDT_TRY_CUDA(ctx, pool_malloc(ctx, &q, vb, s));
+  GDT_TRY_CUDA(ctx, pool_malloc(ctx, &d, vb, s));
+  GDT_TRY_CUDA(ctx, pool_malloc(ctx, &st, sizeof(KState), s));
   const int pair_blocks = std::max(1, std::min(grid_blocks((n + 1) / 2, TH), ctx->num_sms * 8));
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
@@ -1372,18 +1403,20 @@ gdt_status solve(gdt_context ctx, gdt_matrix m, const double* b, double* x, cons
   cudaStream_t s = ctx->stream;
   cudaStream_t own = nullptr;
   if (s == nullptr) {  // the legacy stream cannot be captured; use a blocking stream ordered with it
-    GDT_TRY_CUDA(ctx, cudaStreamCreate(&own));
+    own = ctx->own.exchange(nullptr);  // (a solve of another thread in the meantime makes its own)
+    if (!own) GDT_TRY_CUDA(ctx, cudaStreamCreate(&own));
     s = own;
   }
   struct Cleanup {
+    gdt_context ctx;
     cudaStream_t st;
     ~Cleanup() {
-      if (st) {
-        cudaStreamSynchronize(st);
-        cudaStreamDestroy(st);
-      }
+      if (!st) return;
+      cudaStreamSynchronize(st);
+      cudaStream_t none = nullptr;
+      if (!ctx->own.compare_exchange_strong(none, st)) cudaStreamDestroy(st);
     }
-  } cleanup{own};
+  } cleanup{ctx, own};
   const int n = int(m->rows);
   ctx->last_solver_launch = 0;
   Launch L;
@@ -1420,7 +1453,7 @@ gdt_status solve(gdt_context ctx, gdt_matrix m, const double* b, double* x, cons
     return solve_mixed_stencil(ctx, m, b, x, o, info, s);
   }
   KState* st = nullptr;
-  GDT_TRY_CUDA(ctx, cudaMallocAsync(&st, sizeof(KState), s));
+  GDT_TRY_CUDA(ctx, pool_malloc(ctx, &st, sizeof(KState), s));
   KState init{};
   init.tol2 = o->tol * o->tol;
   init.max_iter = o->max_iter;
@@ -1428,7 +1461,7 @@ gdt_status solve(gdt_context ctx, gdt_matrix m, const double* b, double* x, cons
   allocs.push_back(st);
   auto alloc = [&](size_t bytes) -> void* {
     void* p = nullptr;
-    if (cudaMallocAsync(&p, bytes, s) != cudaSuccess) return nullptr;
+    if (pool_malloc(ctx, &p, bytes, s) != cudaSuccess) return nullptr;
     allocs.push_back(p);
     return p;
   };

@@ -636,9 +636,9 @@ gdt_status mesh_element_error(gdt_context ctx, const gdt_space_s& sp, int norm, 
         if (q) cudaFreeAsync(q, s);
     }
   } freer{{}, st};
-  GDT_TRY_CUDA(ctx, cudaMallocAsync(&dphi, sizeof(double) * phi.size(), st));
+  GDT_TRY_CUDA(ctx, pool_malloc(ctx, &dphi, sizeof(double) * phi.size(), st));
   freer.p[0] = dphi;
-  GDT_TRY_CUDA(ctx, cudaMallocAsync(&dw, sizeof(double) * Q.w.size(), st));
+  GDT_TRY_CUDA(ctx, pool_malloc(ctx, &dw, sizeof(double) * Q.w.size(), st));
   freer.p[1] = dw;
   GDT_TRY_CUDA(ctx, cudaMemcpyAsync(dphi, phi.data(), sizeof(double) * phi.size(), cudaMemcpyHostToDevice, st));
   GDT_TRY_CUDA(ctx, cudaMemcpyAsync(dw, Q.w.data(), sizeof(double) * Q.w.size(), cudaMemcpyHostToDevice, st));
@@ -648,11 +648,11 @@ gdt_status mesh_element_error(gdt_context ctx, const gdt_space_s& sp, int norm, 
   else k_mesh_element_error<3><<<bl, 128, 0, st>>>(g, dg, Q.nq, norm, dphi, dw, u, ref, eta2);
   GDT_CHECK(ctx, check_launch(ctx, "mesh element error"));
   if (total) {
-    GDT_TRY_CUDA(ctx, cudaMallocAsync(&sum, sizeof(double), st));
+    GDT_TRY_CUDA(ctx, pool_malloc(ctx, &sum, sizeof(double), st));
     freer.p[2] = sum;
     size_t tb = 0;
     cub::DeviceReduce::Sum(nullptr, tb, eta2, sum, int(g.nelem), st);
-    GDT_TRY_CUDA(ctx, cudaMallocAsync(&tmp, std::max<size_t>(tb, 16), st));
+    GDT_TRY_CUDA(ctx, pool_malloc(ctx, &tmp, std::max<size_t>(tb, 16), st));
     freer.p[3] = tmp;
     cub::DeviceReduce::Sum(tmp, tb, eta2, sum, int(g.nelem), st);
     double h = 0.0;

@@ -846,7 +846,7 @@ gdt_status solve_mixed_stencil(gdt_context ctx, gdt_matrix m, const double* b, d
   // every array starts on a 256-byte boundary (16-byte vector accesses, TMA base addresses)
   auto alloc = [&](size_t bytes) -> void* {
     void* p = nullptr;
-    if (cudaMallocAsync(&p, bytes + 256, s) != cudaSuccess) return nullptr;
+    if (pool_malloc(ctx, &p, bytes + 256, s) != cudaSuccess) return nullptr;
     allocs.push_back(p);
     return reinterpret_cast<void*>((reinterpret_cast<uintptr_t>(p) + 255) & ~uintptr_t(255));
   };

@@ -710,9 +710,8 @@ gdt_status solve_mixed_mf(gdt_context ctx, gdt_matrix m, const double* b, double
   unsigned int* ticket = ctx->counters;
 
   // persistent launch shape: one block of MT threads per SM (co-resident: cooperative launch)
-  int coop = 0, per_sm = 0, optin = 0;
+  int coop = 0, per_sm = 0;
   GDT_TRY_CUDA(ctx, cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device));
-  GDT_TRY_CUDA(ctx, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
   if (!coop) return GDT_EUNSUPPORTED;
   int blocks = std::min(ctx->num_sms, 256);
   if (ctx->persistent_blocks > 0) blocks = std::min(blocks, ctx->persistent_blocks);
@@ -730,12 +729,12 @@ gdt_status solve_mixed_mf(gdt_context ctx, gdt_matrix m, const double* b, double
        reinterpret_cast<const void*>(&k_mf3_persistent<false, 2>), reinterpret_cast<const void*>(&k_mf3_persistent<false, 3>)},
       {reinterpret_cast<const void*>(&k_mf3_persistent<true, 0>), reinterpret_cast<const void*>(&k_mf3_persistent<true, 1>),
        reinterpret_cast<const void*>(&k_mf3_persistent<true, 2>), reinterpret_cast<const void*>(&k_mf3_persistent<true, 3>)}};
-  cudaFuncAttributes fa;
-  GDT_TRY_CUDA(ctx, cudaFuncGetAttributes(&fa, fns[dir][3]));
-  const int shared = int(std::min(3LL, (optin - (long long)fa.sharedSizeBytes) / per));
+  long long room = 0;
+  GDT_TRY_CUDA(ctx, allow_shared(ctx, fns[dir][3], &room));  // (all have the same static memory)
+  const int shared = int(std::min(3LL, room / per));
   const void* fn = fns[dir][shared];
   const size_t dyn = size_t(shared * per);
-  GDT_TRY_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(dyn)));
+  GDT_TRY_CUDA(ctx, allow_shared(ctx, fn, &room));
   GDT_TRY_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, MT, dyn));
   if (per_sm < 1) return GDT_EUNSUPPORTED;
 
@@ -749,7 +748,7 @@ gdt_status solve_mixed_mf(gdt_context ctx, gdt_matrix m, const double* b, double
   } freer{&allocs, s};
   auto alloc = [&](size_t bytes) -> void* {
     void* p = nullptr;
-    if (cudaMallocAsync(&p, bytes + 256, s) != cudaSuccess) return nullptr;
+    if (pool_malloc(ctx, &p, bytes + 256, s) != cudaSuccess) return nullptr;
     allocs.push_back(p);
     return reinterpret_cast<void*>((reinterpret_cast<uintptr_t>(p) + 255) & ~uintptr_t(255));
   };

@@ -359,9 +359,8 @@ gdt_status solve_mixed_resident(gdt_context ctx, gdt_matrix m, const double* b, 
                                 gdt_solve_info* info, cudaStream_t s) {
   const int n = int(m->rows);
   const GridDesc& g = m->test.g;
-  int coop = 0, optin = 0;
+  int coop = 0;
   GDT_TRY_CUDA(ctx, cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device));
-  GDT_TRY_CUDA(ctx, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
   if (!coop) return GDT_EUNSUPPORTED;
   int blocks = std::min(ctx->num_sms, MT);
   if (ctx->persistent_blocks > 0) blocks = std::min(blocks, ctx->persistent_blocks);
@@ -401,14 +400,12 @@ gdt_status solve_mixed_resident(gdt_context ctx, gdt_matrix m, const double* b, 
     const gdt_status ss = sell_prepare(ctx, m, s, true);
     if (ss != GDT_OK) return ss;
   }
-  cudaFuncAttributes fa;
-  GDT_TRY_CUDA(ctx, cudaFuncGetAttributes(&fa, fn));
-  const long long room = (optin - (long long)fa.sharedSizeBytes) / 4 / 32 * 32;
+  long long room = 0;
+  GDT_TRY_CUDA(ctx, allow_shared(ctx, fn, &room));
   const long long want = 32LL * a.slots.count * ((nslices + blocks - 1) / blocks);
-  a.cap = int(std::max(0LL, std::min(want, room)));
+  a.cap = int(std::max(0LL, std::min(want, room / 4 / 32 * 32)));
   const size_t dyn = size_t(a.cap) * 4;
   int per_sm = 0;
-  GDT_TRY_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(dyn)));
   GDT_TRY_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, MT, dyn));
   if (per_sm < 1) return GDT_EUNSUPPORTED;
   a.n = n;
@@ -428,10 +425,10 @@ gdt_status solve_mixed_resident(gdt_context ctx, gdt_matrix m, const double* b, 
     }
   } buf;
   buf.s = s;
-  if (cudaMallocAsync(&buf.p[0], sizeof(float) * a.ld * a.slots.count, s) != cudaSuccess ||
-      cudaMallocAsync(&buf.p[1], sizeof(float) * plen, s) != cudaSuccess ||
-      cudaMallocAsync(&buf.p[2], sizeof(RState), s) != cudaSuccess ||
-      cudaMallocAsync(&buf.p[3], sizeof(int), s) != cudaSuccess) {
+  if (pool_malloc(ctx, &buf.p[0], sizeof(float) * a.ld * a.slots.count, s) != cudaSuccess ||
+      pool_malloc(ctx, &buf.p[1], sizeof(float) * plen, s) != cudaSuccess ||
+      pool_malloc(ctx, &buf.p[2], sizeof(RState), s) != cudaSuccess ||
+      pool_malloc(ctx, &buf.p[3], sizeof(int), s) != cudaSuccess) {
     cudaGetLastError();
     return fail(ctx, GDT_ENOMEM, "mixed solver vectors");
   }

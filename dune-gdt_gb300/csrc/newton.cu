@@ -62,10 +62,10 @@ gdt_status newton_solve(gdt_context ctx, gdt_matrix m, const double* range, doub
         if (*q) cudaFreeAsync(*q, s);
     }
   } freer{{&r, &u, &cand, &rr}, s};
-  GDT_TRY_CUDA(ctx, cudaMallocAsync(&r, vb, s));
-  GDT_TRY_CUDA(ctx, cudaMallocAsync(&u, vb, s));
-  GDT_TRY_CUDA(ctx, cudaMallocAsync(&cand, vb, s));
-  GDT_TRY_CUDA(ctx, cudaMallocAsync(&rr, sizeof(double), s));
+  GDT_TRY_CUDA(ctx, pool_malloc(ctx, &r, vb, s));
+  GDT_TRY_CUDA(ctx, pool_malloc(ctx, &u, vb, s));
+  GDT_TRY_CUDA(ctx, pool_malloc(ctx, &cand, vb, s));
+  GDT_TRY_CUDA(ctx, pool_malloc(ctx, &rr, sizeof(double), s));
   // ||range - A y||_2, with r = range - A y left on the device
   auto defect = [&](const double* y, double& norm) -> gdt_status {
 #define GDT_NEWTON_DEFECT(GG, PP)                                                                             \

@@ -252,8 +252,8 @@ gdt_status tune_spmv(gdt_context ctx, gdt_matrix m, double* times_ms) {
   const int n = int(m->rows);
   cudaStream_t s = ctx->stream;
   double *x = nullptr, *y = nullptr;
-  GDT_TRY_CUDA(ctx, cudaMallocAsync(&x, sizeof(double) * std::max(n, 1), s));
-  GDT_TRY_CUDA(ctx, cudaMallocAsync(&y, sizeof(double) * std::max(n, 1), s));
+  GDT_TRY_CUDA(ctx, pool_malloc(ctx, &x, sizeof(double) * std::max(n, 1), s));
+  GDT_TRY_CUDA(ctx, pool_malloc(ctx, &y, sizeof(double) * std::max(n, 1), s));
   k_probe_vector<<<std::max(1, std::min(grid_blocks(n, 256), ctx->num_sms * 8)), 256, 0, s>>>(n, x);
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
