@@ -102,10 +102,10 @@ def hbm_peak():
 # the 128^3 workload, from single-pass ncu captures:
 #   ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum,gpu__time_duration.sum --clock-control none \
 #       -k regex:k_mf3_persistent -c 60 python bench.py --headline-only --no-cpu-baseline --steps 1 --warmup 0
-#   (mean of the 11 launches of one solve: 75.9 MB read + 67.7 MB written)
+#   (mean of the 11 launches of one solve: 60.9 MB read + 0.3 MB written)
 #   ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum --clock-control none -k regex:sell_spmv_kernel -s 3 -c 1 \
 #       python bench.py --headline-only --no-cpu-baseline --steps 1 --warmup 0 --spmv-schedule sell32
-MIXED_TRAFFIC_PER_LAUNCH_128 = 143.6e6
+MIXED_TRAFFIC_PER_LAUNCH_128 = 61.2e6
 SELL_TRAFFIC_PER_SPMV_128 = 706.5e6 + 4.1e6
 
 
@@ -365,7 +365,7 @@ def run_gdt(args):
         # per cell); one launch runs the iterations of one residual-replacement cycle
         its = max(int(info32.get("iterations", 0)), 1)
         classes = {"mixed_persistent": ("k_mf3_persistent: matrix-free FP32 CG iterations (update + Q1 operator, "
-                                        "two grid barriers each)", (56 * ndof + 4 * grid.num_elements), its)}
+                                        "one grid barrier and one exchange of the sums each)", (56 * ndof + 4 * grid.num_elements), its)}
     elif inner == "matrix_free":
         # Chronopoulos-Gear iteration: operator w = A z with r.z, z.w, r.r (coefficients, z, own r read,
         # w written); one vector update p, s, x, r, z (z, p, w, s, x, r, 1/diag read; p, s, x, r, z written)
@@ -457,8 +457,8 @@ def run_gdt(args):
                                      "launch), mean of the 11 launches of one solve at 128^3",
                      "l2": l2_roof,
                      "note": ("the inner iteration's working set (FP32 vectors and coefficients, ~70 MB) stays in "
-                              "the 129 MB L2, so the achieved rate is measured against HBM but served mostly from "
-                              "L2") if inner == "matrix_free" else None},
+                              "shared memory and the 129 MB L2, so the achieved rate is measured against HBM but "
+                              "served mostly from those") if inner == "matrix_free" else None},
         "roofline_by_kernel": by_kernel,
         "inner_operator": inner,
         "clocks": clk,
@@ -595,13 +595,12 @@ def batched_metrics(args, gdt, cpu=True, world=1, steps=None, warmup=None):
                                                                 "events, scaled by the class counts)"},
         "speedup_batched_mixed_vs_plain_fp64": t_plain / ms_mixed,
         "speedup_batched_fp64_vs_plain_fp64": t_plain / ms_fp64,
-        "roofline": {"bound": "hbm (the large problems; cluster-barrier latency for the small ones)",
-                     "kernel": "batch_kernel (FP64)",
+        "roofline": {"bound": "hbm and the FP64 pipe (12 operations per DoF and iteration)",
+                     "kernel": "batch_team_kernel (FP64)",
                      "achieved": bytes_fp64 / (ms_fp64 / 1e3) / 1e9, "peak": hbm, "unit": "GB/s",
                      "frac": bytes_fp64 / (ms_fp64 / 1e3) / 1e9 / hbm, "peak_source": hbm_src,
                      "bytes": "13 FP64 words per DoF and CG iteration (7 stencil values, 6 vector accesses), "
-                              "summed over this GPU's problems' iterations; the three passes of an iteration "
-                              "move about 20 words (vectors re-read by the update and direction passes)",
+                              "summed over this GPU's problems' iterations",
                      "traffic": None},
         "scaling": ("strong: the problems split across the ranks by DoF weight" if world > 1
                     else "one GPU solves all problems"),
@@ -670,11 +669,11 @@ def bumps(n, seed, count=32):
 
 
 # FP64 instructions executed per cell and SSP-RK2 step of the LF Burgers stage kernels, from ncu's
-# InstructionStats (fused + non-fused FP64 warp instructions x 32 / cells) on 2048^2 periodic cells:
-#   ncu --section InstructionStats --clock-control none -k regex:fv2d_tile -s 4 -c 2 \
+# sm__inst_executed_pipe_fp64.sum (warp instructions x 32 / cells) on 2048^2 periodic cells:
+#   ncu --metrics sm__inst_executed_pipe_fp64.sum --clock-control none -k regex:fv2d_tile -s 4 -c 2 \
 #       python bench.py --config fv --fv-n 2048 --fv-steps 2 --steps 1 --warmup 0 --no-cpu-baseline
-# stage 1: (401,408 + 954,368) x 32 / 4,194,304 = 10.34; stage 2: (684,032 + 1,085,440) x 32 / 4,194,304 = 13.50
-FV_FP64_INSTR_PER_CELL_STEP = 10.344 + 13.500
+# stage 1: 1,118,208 x 32 / 4,194,304 = 8.53; stage 2: 1,499,136 x 32 / 4,194,304 = 11.44
+FV_FP64_INSTR_PER_CELL_STEP = 8.531 + 11.438
 
 # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) of one SSP-RK2 step of the stage kernels
 # on the bench's 4096^2 state (one pass per launch, both stages of one step):
@@ -1152,13 +1151,13 @@ def run_swipdg(args):
                                 "iterations": {"persistent": it_persistent, "graph": it_graph}},
         "gradient_vs_central_differences": {"max_rel_error_h1e-6": fd_err[1e-6], "max_rel_error_h1e-4": fd_err[1e-4],
                                             "elements": int(args.dg_fd), "relative_to": "max |gradient|"},
-        "roofline": {"bound": "hbm", "kernel": "k_pcg_persistent: all CG iterations in one cooperative launch",
+        "roofline": {"bound": "hbm", "kernel": "k_pcg_resident: all CG iterations in one cooperative launch",
                      "achieved": bytes_it / (it_ms_persistent / 1e3) / 1e9, "peak": hbm, "unit": "GB/s",
                      "frac": bytes_it / (it_ms_persistent / 1e3) / 1e9 / hbm, "bytes_per_iteration": bytes_it,
                      "ms_per_iteration": it_ms_persistent, "peak_source": hbm_src, "traffic": None,
                      "note": "the 64 MB system stays in the 129 MB L2 across iterations, so HBM is not the bound: "
-                             "the FP64 pipe (about 21 FP64 operations per row and iteration, 12 in the SpMV) and "
-                             "the three grid barriers and reductions of an iteration are"},
+                             "the FP64 pipe (22 FP64 operations per row and iteration, 12 in the SpMV) and the "
+                             "two exchanges of an iteration are"},
         "clocks": clk,
     }
     print(json.dumps(line), flush=True)

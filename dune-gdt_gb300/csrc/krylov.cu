@@ -8,8 +8,8 @@
 // fixed summation order: deterministic), so an iteration issues no host synchronisation. Iterations
 // are captured into a CUDA graph in chunks of `check_every`; the host reads the converged flag once
 // per chunk, and kernels of iterations past convergence return immediately. FP64 CG with Jacobi or
-// no preconditioner on rows of at most 32 entries instead runs all its iterations in one persistent
-// cooperative launch (k_pcg_persistent below).
+// no preconditioner instead runs all its iterations, where persistent_applies, in one persistent
+// launch (k_pcg_resident, k_pcg_stream below).
 // Mixed precision: FP32 inner CG (FP32 CSR values, FP32 vectors, FP32 Jacobi) inside FP64
 // iterative refinement with an FP64 residual r = b - A x from the FP64 matrix.
 #include <cfloat>

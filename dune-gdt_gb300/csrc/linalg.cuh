@@ -285,7 +285,7 @@ SellView sell_view(gdt_matrix m);
 int sell_blocks(long long nslices, int num_sms, const void* kernel);
 
 // SpMV schedules: PL == 0 -> vector-CSR with G lanes per row; PL > 0 -> pipelined warp staging with
-// PL entries per lane; PL < 0 -> asynchronous double-buffered staging for rows of at most -PL
+// PL entries per lane; PL < 0 -> asynchronous staging for rows of at most -PL
 // entries. Chosen per matrix by the autotuner.
 template <int G, int PL, class T, class Body>
 __device__ __forceinline__ void for_rows_csr(int n, const int* __restrict__ rp, const int* __restrict__ col,

@@ -11,18 +11,20 @@
 // kappa over the cells that hold both vertices, and these sums come from the 2 x 2 coefficients of the
 // cell layers below and above v: per layer two row sums in each direction and their total, and the
 // four below + above pair sums. w_v = sum_t f[t] G_t, G_t the kappa-sum-weighted sum of z over the
-// neighbours of type t: 35 FMAs and 14 adds per row, where the element form takes 72. All FP32
-// vectors live on a zero-padded vertex layout (one layer of zero vertices around the grid), the
+// neighbours of type t: 35 FMAs and 14 adds per row, where the element form takes 72. The operator's
+// input lives on a zero-padded vertex layout (one layer of zero vertices around the grid), the
 // coefficients on a zero-padded cell layout, so no load is predicated. Dirichlet rows (unit rows,
 // zero columns) are the rows of boundary vertices: the operator's input is zb = D_m r with D_m = 0
 // there (their columns drop out) and the row itself is w_v = z_v = r_v.
 //
 // Iteration: p = z + beta p, s = w + beta s, x32 += alpha p, r -= alpha s, z = D r; w = A z;
-// gamma = r.z, delta = z.w, rr = r.r -> beta, alpha. In the persistent kernel the update is one
-// grid-stride pass over the padded arrays (the padding stays zero), then a grid barrier, then the
-// operator over vertex columns (a thread owns a column and a chunk of z planes and keeps three planes
-// of z and two layers of coefficients in registers), three partial sums per block, a second barrier,
-// and every block sums the partials in block order (bit-identical scalars in every block). The kernel
+// gamma = r.z, delta = z.w, rr = r.r -> beta, alpha. In the persistent kernel a thread owns a vertex
+// column's chunk of z planes for the whole launch. It updates its rows (s, p and x32 in shared memory
+// where they fit; r and w are its own, only zb is read by others), and after a grid barrier applies
+// the operator to them with three planes of z and two layers of coefficients in registers; the
+// exchange of the three sums is the second barrier, and every block adds the packets in block order
+// (bit-identical scalars in every block). 128^3: 26.8 us per iteration with the update as a pass over
+// padded arrays, two release barriers and a sum after the second, 20.5 like this. The kernel
 // returns when a residual replacement is due (the iterated residual dropped 10x), the tolerance or
 // max_iter is reached, or on breakdown; the host then runs the FP64 reliable update (x64 += x32,
 // r = b - A x64 from the FP64 CSR matrix, stagnation guard) and launches it again, starting with the
@@ -37,10 +39,9 @@ namespace gdt {
 namespace {
 
 constexpr int TH = 256;
-// threads per block of the persistent kernel (one block per SM): 768 at 80 registers (the column's
-// two-plane-ahead loads spill 48-84 bytes to L1; 26.8 us per iteration at 128^3). 640 threads at 96
-// registers without spills measured slower (fewer columns in flight), as did 1024 threads at 64
-// registers with one-plane-ahead loads (28.6 against 27.8 us).
+// threads per block of the persistent kernel (one block per SM): 768 at 80 registers. 640 threads at 96
+// registers measured slower (fewer columns in flight), as did 1024 threads at 64 registers with
+// one-plane-ahead loads (28.6 against 27.8 us, in the first layout).
 constexpr int MT = 768;
 // residual replacement when the iterated residual's square dropped by this factor since the last one
 // (10x in the residual norm; 100x saved 5 of 11 replacements at 128^3 but cost 10 % more iterations)
