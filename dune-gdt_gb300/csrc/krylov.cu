@@ -675,7 +675,7 @@ struct PcgArgs {
   KState* st;
   ExchangeView ex;    // the whole grid
   int cap;            // matrix entries a block may keep in shared memory (resident form)
-  int stream;         // the matrix exceeds L2: mark its lines evict-first
+  float keep;         // share of the matrix that L2 may keep; the rest is marked evict-first
   int qshared;        // the streaming form keeps q in shared memory
   int units;          // the most units of a block (streaming form by units)
   int first[257];     // the block's slices: first[block] .. first[block + 1] - 1
@@ -782,10 +782,11 @@ __device__ __forceinline__ double pcg_row(int w, const double* p, LoadV v, LoadC
   return s;
 }
 
-__device__ __forceinline__ unsigned long long matrix_policy(int stream) {
+__device__ __forceinline__ unsigned long long matrix_policy(float keep) {
   unsigned long long pol;
-  if (stream) asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
-  else asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(pol));
+  if (keep >= 1.f) asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(pol));
+  else if (keep <= 0.f) asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
+  else asm volatile("createpolicy.fractional.L2::evict_normal.L2::evict_first.b64 %0, %1;" : "=l"(pol) : "f"(keep));
   return pol;
 }
 __device__ __forceinline__ double ld_matrix(const double* a, unsigned long long pol) {
@@ -848,7 +849,7 @@ __global__ void __launch_bounds__(RT, 1) k_pcg_resident(const __grid_constant__ 
     }
   }
   __syncthreads();
-  const unsigned long long pol = matrix_policy(a.stream);
+  const unsigned long long pol = matrix_policy(a.keep);
   // (no block writes to the shared memory of one that has not started)
   if (CLUSTER) asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   double x[R], r[R], p[R], d[R];
@@ -1002,7 +1003,7 @@ __global__ void __launch_bounds__(PT, 1) k_pcg_stream(const __grid_constant__ Pc
   const int s0 = a.first[blockIdx.x], s1 = a.first[blockIdx.x + 1];
   const int row1 = min(a.n, s1 * 32);
   double* const q = !SPLIT && a.qshared ? reinterpret_cast<double*>(pcg_smem) : a.q + 32LL * s0;  // of row 32 s0 on
-  const unsigned long long pol = matrix_policy(a.stream);
+  const unsigned long long pol = matrix_policy(a.keep);
   if (threadIdx.x == 0) {
     sh.ex.fault = 0;
     sh.k.load(a.st);
@@ -1292,7 +1293,16 @@ gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, d
   a.ex.count = blocks;
   a.ex.wait_ns = ctx->persistent_wait_ns > 0 ? (unsigned long long)ctx->persistent_wait_ns : kBarrierNs;
   a.cap = cap;
-  a.stream = 12LL * m->sell_len > (64LL << 20);
+  {
+    // What of the matrix is not in shared memory stays in L2 where it fits beside the vectors (the resident form's p, five
+    // of the streaming form), four fifths of the room where it does not: a larger share evicts itself. 65^3
+    // Q1 rows (89 MB, 56 of them streamed): 41.8 us an iteration with every line evict-first, 30.6 kept;
+    // 81^3 (172 MB) 79.1, 73.5 with 65 MB kept, 79.3 with 90; 129^3, where the vectors fill L2, 155 and
+    // 163 with 64 MB.
+    const double vectors = (threads == PT ? 40.0 : 8.0) * double(m->rows), room = 80.0 * (1 << 20) - vectors;
+    const double streamed = (narrow ? 10.0 : 12.0) * std::max(0.0, double(m->sell_len) - double(cap) * blocks);
+    a.keep = streamed <= room ? 1.f : float(std::max(0.0, 0.8 * room / streamed));
+  }
   GDT_TRY_CUDA(ctx, cudaMemsetAsync(words, 0, sizeof(unsigned long long) * (packets + 16), s));
   void* args[] = {&a};
   const cudaError_t le = cudaLaunchKernelExC(&cfg, fn, args);
