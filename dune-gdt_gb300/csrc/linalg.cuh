@@ -117,12 +117,6 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
   const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
 }
-// 4-byte asynchronous copy; when `valid` is false nothing is read and the word is zero-filled
-__device__ __forceinline__ void cp_async4_zfill(void* smem, const void* gmem, bool valid) {
-  const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-  const int bytes = valid ? 4 : 0;
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(s), "l"(gmem), "r"(bytes) : "memory");
-}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
@@ -547,10 +541,6 @@ inline gdt_status iterate_chunks_cond(gdt_context ctx, cudaStream_t s, const int
 }
 
 // ------------------------------------------------------------- persistent (cooperative) kernels ---
-// Barrier words of a persistent launch (in the context scratch): the 64-bit arrival count at bar[0],
-// the generation the waiting blocks poll at bar[kBarGen] and the fault flag at bar[kBarFault], 4 KB
-// apart so the polls and the arrivals do not queue at the same L2 slice. All three start at zero.
-constexpr int kBarGen = 1024, kBarFault = 2048;
 constexpr unsigned long long kBarrierNs = 1000000000ull;  // default longest wait at a grid barrier (1 s)
 
 __device__ __forceinline__ unsigned long long global_ns() {
@@ -560,121 +550,5 @@ __device__ __forceinline__ unsigned long long global_ns() {
 }
 
 __device__ __forceinline__ void fence_acq_rel_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
-
-// Grid barrier (all blocks are co-resident: cooperative launch). Barrier number `epoch` (counted by
-// thread 0 of every block) is complete when the 64-bit arrival count reaches epoch * blocks; the last
-// block to arrive publishes the epoch as the generation the others poll (no reset of the count, so
-// the release is one store after the arrival). The waits are bounded by time (wait_ns, checked at the
-// first poll and every 256 polls) and by count, after which the fault flag is set and every block
-// returns false from then on. Data written before the barrier by any block is read after it with
-// plain (coherent) loads, not through the non-coherent read-only path.
-// Ordering: the block's writes are gathered by __syncthreads, released by thread 0 with
-// fence.acq_rel.gpu before its relaxed arrival (the last arrival acquires the others' releases through
-// the arrival count and releases the generation behind a second fence), and acquired by the waiters
-// with fence.acq_rel.gpu after they observe the generation; the closing __syncthreads passes that on
-// to the block (a sequentially consistent fence is not needed). The poll does not sleep: one thread
-// per SM polls one L2 line.
-__device__ inline bool grid_barrier(unsigned int* bar, unsigned int& epoch, unsigned long long wait_ns) {
-  __shared__ int ok;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    ++epoch;
-    volatile unsigned int* vgen = bar + kBarGen;
-    volatile unsigned int* vfault = bar + kBarFault;
-    fence_acq_rel_gpu();
-    int good = *vfault == 0u;
-    if (good) {
-      const unsigned long long target = (unsigned long long)epoch * gridDim.x;
-      if (atomicAdd(reinterpret_cast<unsigned long long*>(bar), 1ull) == target - 1) {
-        fence_acq_rel_gpu();
-        atomicExch(bar + kBarGen, epoch);
-      } else {
-        const unsigned long long t0 = global_ns();
-        unsigned int spins = 0;
-        while (*vgen != epoch) {
-          ++spins;
-          if ((spins & 255u) == 1u) {
-            if (*vfault) {
-              good = 0;
-              break;
-            }
-            if (spins > (1u << 26) || global_ns() - t0 > wait_ns) {
-              atomicExch(bar + kBarFault, 1u);
-              good = 0;
-              break;
-            }
-          }
-        }
-      }
-    }
-    fence_acq_rel_gpu();
-    ok = good;
-  }
-  __syncthreads();
-  return ok != 0;
-}
-
-// Sum of the per-block partials part[k * gridDim.x + b], the same bits in every block (a fixed order:
-// per lane the partials b = lane + 32 u in order of u, then a shuffle tree); result in every thread.
-// Warp k sums component k: its lanes issue all their loads before the first add (a loop that adds
-// each partial as it arrives waits one L2 latency per partial, several microseconds per iteration of
-// a persistent solver), and only these NV warps issue FP64 adds (this part runs one FP64 warp
-// instruction per 16 SM cycles). Needs blockDim.x >= 32 NV. bc: NV doubles of shared memory.
-template <int NV>
-__device__ __forceinline__ void grid_allreduce(const double* part, double (&v)[NV], double* bc) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp < NV) {
-    const double* pk = part + (long long)warp * gridDim.x;
-    constexpr int U = 8;
-    double s = 0.0;
-    int b = lane;
-    for (; b + 32 * (U - 1) < (int)gridDim.x; b += 32 * U) {
-      double t[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) t[u] = pk[b + 32 * u];
-#pragma unroll
-      for (int u = 0; u < U; ++u) s += t[u];
-    }
-    double t[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) t[u] = b + 32 * u < (int)gridDim.x ? pk[b + 32 * u] : 0.0;
-#pragma unroll
-    for (int u = 0; u < U; ++u) s += t[u];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) bc[warp] = s;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < NV; ++k) v[k] = bc[k];
-}
-
-// Block reduction of NV per-thread FP32 sums: FP32 shuffles inside each warp, the warps' sums added in
-// FP64 by warp 0 (the FP64 tree of block_reduce costs 16 SM cycles per warp instruction here). The
-// warp stage adds 32 FP32 values, a relative error of a few 1e-7, the precision of the FP32 vectors the
-// sums come from. Result valid in thread 0. smem: NV * 32 doubles.
-template <int NV>
-__device__ inline void block_reduce_f32(float (&v)[NV], double (&out)[NV], double* smem) {
-#pragma unroll
-  for (int k = 0; k < NV; ++k) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
-  }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-  if (lane == 0)
-#pragma unroll
-    for (int k = 0; k < NV; ++k) smem[k * 32 + warp] = double(v[k]);
-  __syncthreads();
-  if (warp == 0) {
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-      double s = lane < nw ? smem[k * 32 + lane] : 0.0;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-      out[k] = s;
-    }
-  }
-  __syncthreads();
-}
 
 }  // namespace gdt

@@ -270,7 +270,6 @@ struct MfPArgs {
   MfState* st;
   ExchangeView ex;  // the whole grid
   int start;        // MF3_INIT / MF3_REPLACE: the first pass is the operator alone
-  int shared;       // how many of s, p, x32 live in shared memory during the launch
 };
 
 // The solver scalars live in shared memory (thread 0 updates them after each reduction), so the
@@ -841,7 +840,6 @@ gdt_status solve_mixed_mf(gdt_context ctx, gdt_matrix m, const double* b, double
   a.ex.first = 0;
   a.ex.count = blocks;
   a.ex.wait_ns = ctx->persistent_wait_ns > 0 ? (unsigned long long)ctx->persistent_wait_ns : kBarrierNs;
-  a.shared = shared;
   MfState fin{};
   unsigned int fault = 0;
   int cycles = 0;
