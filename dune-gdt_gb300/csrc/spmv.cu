@@ -190,6 +190,7 @@ gdt_status sell_prepare_nonzero(gdt_context ctx, gdt_matrix m, cudaStream_t s, i
   if (st != GDT_OK) return st;
   const int n = int(m->rows), nslices = (n + 31) / 32;
   m->sell_version = -1;  // not the full copy: the next reader of that one refills it
+  m->csr_version = -1;   // and products count anew towards what the fill costs
   const int blocks = (nslices * 32 + 255) / 256;
   const int2* meta = reinterpret_cast<const int2*>(m->sell_meta);
   if (narrow)
