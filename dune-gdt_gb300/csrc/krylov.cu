@@ -653,7 +653,7 @@ void ilu_apply(gdt_context ctx, gdt_matrix m, const Ilu& f, const double* r, dou
 //    systems, where the shorter alpha^2 (q.D^-1 q) - rho (z.q = p.q) needs up to 38 % more. The one exception
 //    seen: 1D with a constant coefficient, where the classical form ends after exactly n / 2 iterations (the
 //    mirrored halves round alike); here the solution after them is within 2e-11 of the exact one up to 40,001
-//    cells (4e-13 there), and a tolerance below the residual's own rounding takes as many again.
+//    cells (classical form: 4e-13), and a tolerance below the residual's own rounding takes as many again.
 //  * A grid-wide sum and the barrier it implies are one exchange (exchange.cuh), and the scalars
 //    that follow, a reciprocal and a few products, are formed by one thread.
 //  * A thread owns its rows for the whole solve: x, r, p, D^-1 and q of k_pcg_resident never leave its
