@@ -880,8 +880,10 @@ __global__ void __launch_bounds__(RT, 1) k_pcg_resident(const __grid_constant__ 
 #pragma unroll
     for (int i = 0; i < R; ++i) {
       const int ls = warp + RT / 32 * i;
-      const int off = s_off[ls], w = (s_off[ls + 1] - off) >> 5;  // 0 for a slice the block does not have
-      if (s_off[ls + 1] <= a.cap) {
+      const int off = s_off[ls], w = (s_off[ls + 1] - off) >> 5;
+      if (ls >= ns) {  // warp-uniform; the slice table may end here
+        q[i] = 0.0;
+      } else if (s_off[ls + 1] <= a.cap) {
         const double* sv = mv + off + lane;
         const int* sc = mc + off + lane;
         q[i] = pcg_row<CH>(w, a.p, [&](int t) { return sv[32 * t]; }, [&](int t) { return sc[32 * t]; });
