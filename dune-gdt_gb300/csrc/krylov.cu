@@ -14,6 +14,7 @@
 // iterative refinement with an FP64 residual r = b - A x from the FP64 matrix.
 #include <cfloat>
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 #include "exchange.cuh"
@@ -650,10 +651,7 @@ void ilu_apply(gdt_context ctx, gdt_matrix m, const Ilu& f, const double* r, dou
 //    and both products are summed together with p.q right after q = A p (cf. Meurant 1987). beta takes
 //    that value; alpha and the stopping test take the sums over the residual itself, so nothing
 //    accumulates: the iteration counts are those of the classical form, also on badly conditioned 1D
-//    systems, where the shorter alpha^2 (q.D^-1 q) - rho (z.q = p.q) needs up to 38 % more. The one exception
-//    seen: 1D with a constant coefficient, where the classical form ends after exactly n / 2 iterations (the
-//    mirrored halves round alike); here the solution after them is within 2e-11 of the exact one up to 40,001
-//    cells (classical form: 4e-13), and a tolerance below the residual's own rounding takes as many again.
+//    systems, where the shorter alpha^2 (q.D^-1 q) - rho (z.q = p.q) needs up to 38 % more.
 //  * A grid-wide sum and the barrier it implies are one exchange (exchange.cuh), and the scalars
 //    that follow, a reciprocal and a few products, are formed by one thread.
 //  * A thread owns its rows for the whole solve: x, r, p, D^-1 and q of k_pcg_resident never leave its
@@ -681,6 +679,7 @@ struct PcgArgs {
   float keep;         // share of the matrix that L2 may keep; the rest is marked evict-first
   int qshared;        // the streaming form keeps q in shared memory
   int units;          // the most units of a block (streaming form by units)
+  int short_rows;     // no row has more than three entries
   int first[257];     // the block's slices: first[block] .. first[block + 1] - 1
 };
 
@@ -763,10 +762,23 @@ __device__ __forceinline__ void pcg_publish(const PcgArgs& a, unsigned int& epoc
   if (threadIdx.x < 64 && (threadIdx.x & 31) == 0) sh.last[threadIdx.x >> 5] = total;
 }
 
+// Rows of at most three entries (1D grids): the two neighbours' products are added first and the diagonal's last. The
+// large terms then meet in one addition, which rounds mirrored rows alike: with a constant coefficient CG
+// ends after n / 2 iterations (4,001, 10,000 and 20,000 cells at a tolerance of 1e-12: 2,000, 5,000 and 10,000; one
+// sum in the order of the columns takes 3,926, 9,883 and 19,949, whichever form beta has).
+template <int CH>
+__device__ __forceinline__ double short_row(int w, const double (&v)[CH], const double (&p)[CH]) {
+  double s = 0.0;
+  if (w > 0) s = v[0] * p[0];
+  if (w > 2) s = fma(v[2], p[2], s);
+  if (w > 1) s += __dmul_rn(v[1], p[1]);
+  return s;
+}
+
 // sum of a row's products, entries t of the lane's row at v[32 t], c[32 t]; w is warp-uniform. All loads of
 // CH entries are issued before their FMAs. One accumulator: with 16 or more warps on the SM each
 // warp's turn at the FP64 pipe comes after the FMA's latency, and a second one would cost an add.
-template <int CH, class LoadV, class LoadC>
+template <bool SHORT, int CH, class LoadV, class LoadC>
 __device__ __forceinline__ double pcg_row(int w, const double* p, LoadV v, LoadC c) {
   double s = 0.0;
 #pragma unroll 1
@@ -780,7 +792,8 @@ __device__ __forceinline__ double pcg_row(int w, const double* p, LoadV v, LoadC
         pv[j] = p[c(t0 + j)];
       }
     }
-    fma_chain<0>(w - t0, vv, pv, s);
+    if (SHORT) s = short_row(w, vv, pv);
+    else fma_chain<0>(w - t0, vv, pv, s);
   }
   return s;
 }
@@ -877,24 +890,28 @@ __global__ void __launch_bounds__(RT, 1) k_pcg_resident(const __grid_constant__ 
   while (true) {
     double q[R];
     double v3[3] = {0.0, 0.0, 0.0};
+    auto product = [&](auto short_rows) {
+      constexpr bool SHORT = decltype(short_rows)::value;
 #pragma unroll
-    for (int i = 0; i < R; ++i) {
-      const int ls = warp + RT / 32 * i;
-      const int off = s_off[ls], w = (s_off[ls + 1] - off) >> 5;
-      if (ls >= ns) {  // warp-uniform; the slice table may end here
+      for (int i = 0; i < R; ++i) {
+        const int ls = warp + RT / 32 * i;
+        const int off = s_off[ls], w = (s_off[ls + 1] - off) >> 5;
         q[i] = 0.0;
-      } else if (s_off[ls + 1] <= a.cap) {
-        const double* sv = mv + off + lane;
-        const int* sc = mc + off + lane;
-        q[i] = pcg_row<CH>(w, a.p, [&](int t) { return sv[32 * t]; }, [&](int t) { return sc[32 * t]; });
-      } else {
-        const int src = __ldg(&a.meta[s0 + ls].x) + lane;
-        const double* gv = a.val + src;
-        const int* gc = a.col + src;
-        q[i] = pcg_row<CH>(w, a.p, [&](int t) { return ld_matrix(gv + 32 * t, pol); },
-                           [&](int t) { return ld_matrix(gc + 32 * t, pol); });
+        if (s_off[ls + 1] <= a.cap) {
+          const double* sv = mv + off + lane;
+          const int* sc = mc + off + lane;
+          q[i] = pcg_row<SHORT, CH>(w, a.p, [&](int t) { return sv[32 * t]; }, [&](int t) { return sc[32 * t]; });
+        } else if (ls < ns) {  // (behind the last block's slices the table ends)
+          const int src = __ldg(&a.meta[s0 + ls].x) + lane;
+          const double* gv = a.val + src;
+          const int* gc = a.col + src;
+          q[i] = pcg_row<SHORT, CH>(w, a.p, [&](int t) { return ld_matrix(gv + 32 * t, pol); },
+                                    [&](int t) { return ld_matrix(gc + 32 * t, pol); });
+        }
       }
-    }
+    };
+    if (a.short_rows) product(std::true_type());
+    else product(std::false_type());
 #pragma unroll
     for (int i = 0; i < R; ++i)
       if (warp + RT / 32 * i < ns) {  // warp-uniform
@@ -946,7 +963,7 @@ __host__ __device__ constexpr int pcg_units(int width) { return width <= kUnit ?
 // are 16-bit differences; next(src, w, row) gives them one after the other): begin() where a segment starts, done(sum) where it ends. Groups of nine entries in three
 // buffers: the entries are loaded three steps of three before their products and the vector is gathered one step
 // before, across the ends of segments, so that neither latency is waited for.
-template <class Col, class Next, class Begin, class Done>
+template <class Col, bool SHORT, class Next, class Begin, class Done>
 __device__ __forceinline__ void pcg_segments(const PcgArgs& a, unsigned long long pol, Next next, Begin begin, Done done) {
   const int lane = threadIdx.x & 31;
   int src, w, row, nsrc = 0, nw = 0, nrow = 0;
@@ -977,7 +994,8 @@ __device__ __forceinline__ void pcg_segments(const PcgArgs& a, unsigned long lon
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
       gather((j + 1) % 3, j == 2 && last ? nrow : row);
-      fma_chain<0>(w - t - 3 * j, v[j], g[j], s);
+      if (SHORT && j == 0) s = short_row(w, v[0], g[0]);
+      else fma_chain<0>(w - t - 3 * j, v[j], g[j], s);
       load(j, base, left);
     }
     if (last) {
@@ -1032,7 +1050,7 @@ __global__ void __launch_bounds__(PT, 1) k_pcg_stream(const __grid_constant__ Pc
     double v3[3] = {0.0, 0.0, 0.0};
     if (SPLIT) {
       int u = warp, out = warp;
-      pcg_segments<Col>(
+      pcg_segments<Col, false>(
           a, pol,
           [&](int& src, int& w, int& row) {
             row = 0;
@@ -1079,17 +1097,16 @@ __global__ void __launch_bounds__(PT, 1) k_pcg_stream(const __grid_constant__ Pc
       }
     } else {
       int ahead = slice;
-      pcg_segments<Col>(
-          a, pol,
-          [&](int& src, int& w, int& row) {
-            if (ahead >= s1) return false;
-            row = sizeof(Col) == 2 ? min(ahead * 32 + lane, a.n - 1) : 0;  // (in bounds where there is no row)
-            src = __ldg(&a.meta[ahead].x);
-            w = __ldg(a.width + ahead);
-            ahead += PT / 32;
-            return true;
-          },
-          begin_row, end_row);
+      auto next = [&](int& src, int& w, int& row) {
+        if (ahead >= s1) return false;
+        row = sizeof(Col) == 2 ? min(ahead * 32 + lane, a.n - 1) : 0;  // (in bounds where there is no row)
+        src = __ldg(&a.meta[ahead].x);
+        w = __ldg(a.width + ahead);
+        ahead += PT / 32;
+        return true;
+      };
+      if (a.short_rows) pcg_segments<Col, true>(a, pol, next, begin_row, end_row);
+      else pcg_segments<Col, false>(a, pol, next, begin_row, end_row);
     }
     if (!pcg_step<false>(a, epoch, v3, PT / 32, sh)) break;
     const double alpha = sh.k.alpha, beta = sh.k.beta;
@@ -1213,6 +1230,7 @@ gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, d
   int cap = 0;
   size_t dyn = 0;
   a.units = 0;
+  a.short_rows = m->max_row <= 3;
   // long rows: eight warps cannot hide the latency of what does not stay in shared memory (20^3 Q2 cubes, four slices a
   // warp: 25 us an iteration resident, 33 streaming by slices; 24^3, eight: 48 resident, 38 streaming by units)
   if (m->max_row > 32 && per_warp > 4) {
