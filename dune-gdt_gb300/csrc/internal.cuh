@@ -212,12 +212,16 @@ gdt_status tune_spmv(gdt_context ctx, gdt_matrix m, double* times_ms = nullptr);
 // SELL-32 copy of m: slice table built once per pattern (GDT_EUNSUPPORTED when there is no room or the
 // offsets do not fit 32 bits), values and columns copied when the values changed or `refill` is set
 gdt_status sell_prepare(gdt_context ctx, gdt_matrix m, cudaStream_t s, bool refill);
-// its slice table and memory alone
+// its slice table alone
 gdt_status sell_table(gdt_context ctx, gdt_matrix m, cudaStream_t s);
-// the copy without the zero values, for solves whose vectors are finite by their own checks (a product
-// keeps them: 0 * inf is not 0): width (device, one per 32-row slice) receives the entries per row
-// with `narrow` (sell_band of at most 32767) the columns are stored as 16-bit differences to the row
-gdt_status sell_prepare_nonzero(gdt_context ctx, gdt_matrix m, cudaStream_t s, int* width, bool narrow = false);
+// A solver's own copy (sell_table must have succeeded; col and val have room for sell_len entries) without the zero
+// values, for solves whose vectors are finite by their own checks (a product keeps them: 0 * inf is not 0):
+// width (device, one per 32-row slice) receives the entries per row; with `narrow` (sell_band of at most
+// 32767) the columns are 16-bit differences to the row, else ints. Not the product's copy: products on
+// another stream, or captured in a graph that is replayed later, read that one.
+gdt_status sell_fill_nonzero(gdt_context ctx, gdt_matrix m, cudaStream_t s, void* col, double* val, int* width,
+                             bool narrow);
+void sell_release(gdt_matrix m);  // the copy, not the table
 void sell_free(gdt_matrix m);
 // index of the SELL-32 schedule in gdt_matrix_tune / gdt_matrix_set_schedule
 constexpr int kSellSchedule = 8;

@@ -1187,7 +1187,7 @@ int pcg_partition(gdt_matrix m, int blocks, bool by_work, int* first) {
 // Runs the iterations after residual_init; the caller reads the final state from st. Returns
 // GDT_EUNSUPPORTED, before anything ran, where no cooperative launch of the kernel can be made
 // (the caller then runs the graph form).
-gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, double* p, double* q, int* width,
+gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, double* p, double* q,
                           const double* dinv, KState* st, cudaStream_t s) {
   int dev = 0, coop = 0, per_sm = 0;
   long long room = 0;
@@ -1211,7 +1211,6 @@ gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, d
   GDT_CHECK(ctx, sell_table(ctx, m, s));
   if (m->max_row > 32 && m->sell_len - m->nnz > m->nnz / 2 + 32768) {  // padding is work
     m->sell_padded = true;
-    if (!m->use_sell) sell_free(m);
     return GDT_EUNSUPPORTED;
   }
   PcgArgs a;
@@ -1290,16 +1289,30 @@ gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, d
     GDT_TRY_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, dyn));
   }
   if (per_sm < 1) return GDT_EUNSUPPORTED;
-  {
-    // the values are copied at every solve: the caller may have written them through the CSR pointer
-    const gdt_status ss = sell_prepare_nonzero(ctx, m, s, width, narrow);
-    if (ss != GDT_OK) return ss;
+  // The solve's copy of the matrix, from the pool: values, columns, entries per row of the slices. The values are copied
+  // at every solve: the caller may have written them through the CSR pointer.
+  struct Copy {
+    double* val = nullptr;
+    cudaStream_t s;
+    ~Copy() {
+      if (val) cudaFreeAsync(val, s);
+    }
+  } copy;
+  copy.s = s;
+  const size_t entries = size_t(std::max(m->sell_len, 32LL));  // (a multiple of 32: every part is aligned)
+  const size_t col_bytes = (narrow ? sizeof(short) : sizeof(int)) * entries;
+  if (pool_malloc(ctx, &copy.val, sizeof(double) * entries + col_bytes + sizeof(int) * nslices, s) != cudaSuccess) {
+    cudaGetLastError();
+    return GDT_EUNSUPPORTED;  // no room for it
   }
+  int* const col = reinterpret_cast<int*>(copy.val + entries);
+  int* const width = reinterpret_cast<int*>(reinterpret_cast<unsigned char*>(col) + col_bytes);
+  GDT_CHECK(ctx, sell_fill_nonzero(ctx, m, s, col, copy.val, width, narrow));
   a.n = int(m->rows);
   a.meta = reinterpret_cast<const int2*>(m->sell_meta);
   a.width = width;
-  a.col = m->sell_col;
-  a.val = m->sell_val;
+  a.col = col;
+  a.val = copy.val;
   a.dinv = dinv;
   a.x = x;
   a.r = r;
@@ -1544,9 +1557,7 @@ gdt_status solve(gdt_context ctx, gdt_matrix m, const double* b, double* x, cons
         bool persistent = persistent_applies(ctx, m);
         if (persistent) {
           residual_init<double>(L, m->rp, m->col, m->val, x, b, r, one, p, st);
-          int* width = (int*)alloc(sizeof(int) * ((n + 31) / 32));
-          if (!width) return fail(ctx, GDT_ENOMEM, "solver vectors");
-          const gdt_status ps = pcg_persistent(ctx, m, x, r, p, q, width, one, st, s);
+          const gdt_status ps = pcg_persistent(ctx, m, x, r, p, q, one, st, s);
           if (ps == GDT_EUNSUPPORTED) persistent = false;  // x untouched: the graph form starts afresh
           else if (ps != GDT_OK) return ps;
           else ctx->last_solver_launch = GDT_SOLVER_LAUNCH_PERSISTENT;

@@ -105,18 +105,23 @@ __global__ void k_sell_fill_nonzero(int n, int nslices, const int* __restrict__ 
   if (lane == 0) width[slice] = w;
 }
 
-void sell_free(gdt_matrix m) {
-  if (m->sell_meta) cudaFree(m->sell_meta);
+void sell_release(gdt_matrix m) {
   if (m->sell_col) cudaFree(m->sell_col);
   if (m->sell_val) cudaFree(m->sell_val);
-  m->sell_meta = m->sell_col = nullptr;
+  m->sell_col = nullptr;
   m->sell_val = nullptr;
-  m->sell_len = 0;
-  m->sell_off.clear();
   m->sell_version = -1;
 }
 
-// the slice table of the pattern and room for the copy (its values are filled by the callers below)
+void sell_free(gdt_matrix m) {
+  sell_release(m);
+  if (m->sell_meta) cudaFree(m->sell_meta);
+  m->sell_meta = nullptr;
+  m->sell_len = 0;
+  m->sell_off.clear();
+}
+
+// the slice table of the pattern
 gdt_status sell_table(gdt_context ctx, gdt_matrix m, cudaStream_t s) {
   const int n = int(m->rows);
   const int nslices = (n + 31) / 32;
@@ -145,29 +150,20 @@ gdt_status sell_table(gdt_context ctx, gdt_matrix m, cudaStream_t s) {
     }
     if (off >= (1LL << 31)) return GDT_EUNSUPPORTED;  // offsets are 32-bit
     int* dmeta = nullptr;
-    int* dcol = nullptr;
-    double* dval = nullptr;
     e = cudaMalloc(&dmeta, sizeof(int) * meta.size());
-    if (e == cudaSuccess) e = cudaMalloc(&dcol, sizeof(int) * std::max(off, 1LL));
-    if (e == cudaSuccess) e = cudaMalloc(&dval, sizeof(double) * std::max(off, 1LL));
     if (e == cudaSuccess) e = cudaMemcpyAsync(dmeta, meta.data(), sizeof(int) * meta.size(), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) {
       cudaFree(dmeta);
-      cudaFree(dcol);
-      cudaFree(dval);
       cudaGetLastError();
-      return GDT_EUNSUPPORTED;  // no room for the copy
+      return GDT_EUNSUPPORTED;  // no room for it
     }
     m->sell_meta = dmeta;
-    m->sell_col = dcol;
-    m->sell_val = dval;
     m->sell_len = off;
     m->sell_band = w[nslices];
     m->sell_off.resize(nslices + 1);
     for (int i = 0; i < nslices; ++i) m->sell_off[i] = meta[2 * i];
     m->sell_off[nslices] = int(off);
-    m->sell_version = -1;
   }
   return GDT_OK;
 }
@@ -175,6 +171,17 @@ gdt_status sell_table(gdt_context ctx, gdt_matrix m, cudaStream_t s) {
 gdt_status sell_prepare(gdt_context ctx, gdt_matrix m, cudaStream_t s, bool refill) {
   const gdt_status st = sell_table(ctx, m, s);
   if (st != GDT_OK) return st;
+  if (!m->sell_col) {
+    const long long len = std::max(m->sell_len, 1LL);
+    cudaError_t e = cudaMalloc(&m->sell_col, sizeof(int) * len);
+    if (e == cudaSuccess) e = cudaMalloc(&m->sell_val, sizeof(double) * len);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      sell_release(m);
+      return GDT_EUNSUPPORTED;  // no room for the copy
+    }
+    m->sell_version = -1;
+  }
   if (refill || m->sell_version != m->val_version) {
     const int n = int(m->rows), nslices = (n + 31) / 32;
     k_sell_fill<<<(nslices * 32 + 255) / 256, 256, 0, s>>>(
@@ -185,19 +192,15 @@ gdt_status sell_prepare(gdt_context ctx, gdt_matrix m, cudaStream_t s, bool refi
   return GDT_OK;
 }
 
-gdt_status sell_prepare_nonzero(gdt_context ctx, gdt_matrix m, cudaStream_t s, int* width, bool narrow) {
-  const gdt_status st = sell_table(ctx, m, s);
-  if (st != GDT_OK) return st;
+gdt_status sell_fill_nonzero(gdt_context ctx, gdt_matrix m, cudaStream_t s, void* col, double* val, int* width,
+                             bool narrow) {
   const int n = int(m->rows), nslices = (n + 31) / 32;
-  m->sell_version = -1;  // not the full copy: the next reader of that one refills it
-  m->csr_version = -1;   // and products count anew towards what the fill costs
   const int blocks = (nslices * 32 + 255) / 256;
   const int2* meta = reinterpret_cast<const int2*>(m->sell_meta);
   if (narrow)
-    k_sell_fill_nonzero<<<blocks, 256, 0, s>>>(n, nslices, m->rp, m->col, m->val, meta,
-                                               reinterpret_cast<short*>(m->sell_col), m->sell_val, width);
+    k_sell_fill_nonzero<<<blocks, 256, 0, s>>>(n, nslices, m->rp, m->col, m->val, meta, static_cast<short*>(col), val, width);
   else
-    k_sell_fill_nonzero<<<blocks, 256, 0, s>>>(n, nslices, m->rp, m->col, m->val, meta, m->sell_col, m->sell_val, width);
+    k_sell_fill_nonzero<<<blocks, 256, 0, s>>>(n, nslices, m->rp, m->col, m->val, meta, static_cast<int*>(col), val, width);
   return check_launch(ctx, "sell fill");
 }
 
@@ -309,8 +312,8 @@ gdt_status tune_spmv(gdt_context ctx, gdt_matrix m, double* times_ms) {
   cudaFreeAsync(y, s);
   m->spmv_sched = best_sched;
   m->use_sell = sell_best ? 1 : 0;
-  // keep the copy only where a solver or the SpMV reads it (the persistent CG takes rows of <= 32)
-  if (!sell_best && m->max_row > 32) sell_free(m);
+  // keep the copy only where the SpMV reads it (solves that need one fill their own, or allocate this one again)
+  if (!sell_best) sell_release(m);
   m->tuned = 1;
   return GDT_OK;
 }
