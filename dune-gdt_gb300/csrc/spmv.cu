@@ -320,15 +320,24 @@ gdt_status tune_spmv(gdt_context ctx, gdt_matrix m, double* times_ms) {
 
 gdt_status spmv(gdt_context ctx, gdt_matrix m, const double* x, double* y) {
   GDT_CHECK(ctx, tune_spmv(ctx, m));
-  bool sell = m->use_sell;
-  if (sell && m->sell_version != m->val_version && m->csr_products > 0) {
+  bool sell = m->use_sell, fill = sell && m->sell_version != m->val_version, captured = false;
+  if (fill && m->csr_products > 0) {
     if (m->csr_version != m->val_version) {
       m->csr_version = m->val_version;
       m->csr_done = 0;
     }
-    sell = m->csr_done++ >= m->csr_products;
+    sell = fill = m->csr_done >= m->csr_products;
+    if (!fill) m->csr_done++;
   }
-  if (sell && sell_prepare(ctx, m, ctx->stream, false) != GDT_OK) m->use_sell = sell = false;
+  if (fill) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &status) != cudaSuccess) cudaGetLastError();
+    captured = status != cudaStreamCaptureStatusNone;
+    // a captured product leaves the fill to one that runs now, or, where it has to read the copy, fills it in its graph
+    if (captured && (m->csr_products > 0 || !m->sell_col)) sell = fill = false;
+  }
+  if (fill && sell_prepare(ctx, m, ctx->stream, false) != GDT_OK) m->use_sell = sell = false;
+  if (fill && captured) m->sell_version = -1;
   timing_begin(ctx, ctx->stream, GDT_TIMING_SPMV_FP64);
   if (sell) launch_sell_spmv(m, x, y, ctx->num_sms, ctx->stream);
   else launch_spmv<double>(m->spmv_sched, int(m->rows), m->rp, m->col, m->val, x, y, ctx->num_sms, ctx->stream);

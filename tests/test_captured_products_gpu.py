@@ -41,3 +41,37 @@ def test_replayed_product_after_solves(gdt, precision, blocks):
     torch.cuda.synchronize()
     assert torch.equal(y, expected)
     assert torch.equal(op.apply(x), expected)
+
+
+# The products with changed values read the CSR arrays until the copy would have paid its fill; whichever of them is
+# captured, and not replayed, the next one must not take the copy for filled
+def test_captured_fill_does_not_count_as_done(gdt):
+    op, rhs, stream = _system(gdt, [97, 101, 53], simplex=False)
+    x = torch.randn(rhs.numel(), dtype=torch.float64, device="cuda", generator=torch.Generator("cuda").manual_seed(3))
+    y = torch.zeros_like(rhs)
+    torch.cuda.synchronize()
+    op.apply(x)  # tunes
+    val = op.csr()[2]
+    # the fill falls due at an even or an odd product: with one product more in front a captured one meets it
+    for schedule, before in ((None, 0), (None, 1), (8, 0)):
+        if schedule is not None:
+            op.set_spmv_schedule(schedule)
+        with torch.cuda.stream(stream):
+            expected = 2.0 * op.apply(x)  # a power of two: the same bits scaled
+            val *= 2.0
+        op.values_changed()
+        stream.synchronize()
+        for k in range(before):
+            op.apply(x)
+        for k in range(60):
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=stream):
+                op.apply(x, y)
+            got = op.apply(x)
+            torch.cuda.synchronize()
+            # (the schedules add in different orders)
+            assert float((got - expected).abs().max()) <= 1e-12 * float(expected.abs().max()), (schedule, k)
+            if k % 8 == 7:
+                graph.replay()
+                torch.cuda.synchronize()
+                assert float((y - expected).abs().max()) <= 1e-12 * float(expected.abs().max()), (schedule, k)
