@@ -86,8 +86,6 @@ struct gdt_batch_s {
   gdt::TeamPlace* d_place = nullptr;
   int* d_tprobs = nullptr;
   unsigned long long* d_exchange = nullptr;  // fault flag, list counters, packets
-  double* team_scratch = nullptr;
-  long long team_words = 0;
   int team_blocks = 0;                   // blocks of the cooperative launch (0: none can be made)
   int team_smem = 0;                     // its dynamic shared memory in doubles
   int* d_queue = nullptr;
@@ -96,7 +94,9 @@ struct gdt_batch_s {
   int* d_status = nullptr;
   int nclusters = 0;                     // clusters resident at once (the larger of the two kernels')
   int nclusters_prec[2] = {0, 0};        // per precision: FP64, mixed
-  double* scratch64 = nullptr;           // [nclusters][scratch_words]
+  // one allocation: [nclusters][scratch_words] doubles, then as many floats, of the fixed-size team kernel; the teams of
+  // batch_team_kernel, which runs before it, use it from its start
+  double* scratch64 = nullptr;
   float* scratch32 = nullptr;
   long long scratch_words = 0;
   cudaGraphExec_t exec = nullptr;
@@ -768,53 +768,35 @@ TeamPlan plan_teams(const gdt_batch_s& b, std::vector<int> subset, int blocks, l
   return plan;
 }
 
+// room for `words` per cluster (what build_items returned for the problems to solve); made where the queue is, so that a
+// solve allocates nothing and can be captured
 gdt_status ensure_scratch(gdt_context ctx, gdt_batch b, long long words) {
   if (words <= b->scratch_words) return GDT_OK;
   cudaFree(b->scratch64);
-  cudaFree(b->scratch32);
   b->scratch64 = nullptr;
   b->scratch32 = nullptr;
   b->scratch_words = 0;
-  cudaError_t e = cudaMalloc(&b->scratch64, sizeof(double) * words * b->nclusters);
-  if (e == cudaSuccess) e = cudaMalloc(&b->scratch32, sizeof(float) * words * b->nclusters);
+  const cudaError_t e = cudaMalloc(&b->scratch64, (sizeof(double) + sizeof(float)) * words * b->nclusters);
   if (e != cudaSuccess) {
     cudaGetLastError();
+    b->scratch64 = nullptr;
     return fail(ctx, e == cudaErrorMemoryAllocation ? GDT_ENOMEM : GDT_ECUDA, "batch scratch");
   }
+  b->scratch32 = reinterpret_cast<float*>(b->scratch64 + words * b->nclusters);
   b->scratch_words = words;
   return GDT_OK;
-}
-
-// words of the fixed-size team kernel's scratch per cluster for `items`, problems in `probs`
-long long words_of(const gdt_batch_s& b, const std::vector<BatchItem>& items) {
-  const long long words = stencil_of(b.element) + 5;
-  long long need = 0;
-  for (const BatchItem& it : items) need = std::max(need, it.count * words * it.stride);
-  return need;
 }
 
 // plan and lists of the problems `subset` for batch_team_kernel, on the device
 gdt_status upload_plan(gdt_context ctx, gdt_batch b, const std::vector<int>& subset) {
   b->plan = TeamPlan();
   if (subset.empty()) return GDT_OK;
-  // no more memory than the clusters of the fixed-size team kernel would take (in 8-byte words)
-  std::vector<BatchItem> items;
-  std::vector<int> probs;
-  const std::vector<int> saved = b->teams;
-  for (int p : subset) b->teams[p] = GDT_BATCH_TEAM_CLUSTER;
-  const long long most = build_items(*b, subset, items, probs) * b->nclusters / 2 * 3;
-  b->teams = saved;
+  // the memory of the fixed-size team kernel, in 8-byte words (a team's arrays are at most as long as a cluster's)
+  const long long most = b->scratch_words * b->nclusters / 2 * 3;
   b->plan = plan_teams(*b, subset, b->team_blocks, most);
-  if (b->plan.words > b->team_words) {
-    cudaFree(b->team_scratch);
-    b->team_scratch = nullptr;
-    b->team_words = 0;
-    const cudaError_t e = cudaMalloc(&b->team_scratch, sizeof(double) * b->plan.words);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      return fail(ctx, e == cudaErrorMemoryAllocation ? GDT_ENOMEM : GDT_ECUDA, "batch scratch");
-    }
-    b->team_words = b->plan.words;
+  if (b->plan.words > most) {
+    b->plan = TeamPlan();
+    return GDT_OK;
   }
   GDT_TRY_CUDA(ctx, cudaMemcpy(b->d_place, b->plan.places.data(), sizeof(TeamPlace) * b->plan.places.size(),
                                cudaMemcpyHostToDevice));
@@ -830,7 +812,8 @@ gdt_status upload_queue(gdt_context ctx, gdt_batch b) {
   std::vector<int> all(b->nprob), team, rest;
   std::iota(all.begin(), all.end(), 0);
   for (int p : all) (b->team_blocks > 0 && b->teams[p] == GDT_BATCH_TEAM_CLUSTER ? team : rest).push_back(p);
-  build_items(*b, all, b->items, b->probs);
+  const long long need = build_items(*b, all, b->items, b->probs);
+  GDT_CHECK(ctx, ensure_scratch(ctx, b, need));
   build_items(*b, rest, b->items_rest, b->probs_rest);
   GDT_TRY_CUDA(ctx, cudaMemcpy(b->d_items, b->items.data(), sizeof(BatchItem) * b->items.size(), cudaMemcpyHostToDevice));
   GDT_TRY_CUDA(ctx, cudaMemcpy(b->d_probs, b->probs.data(), sizeof(int) * b->probs.size(), cudaMemcpyHostToDevice));
@@ -959,7 +942,7 @@ TeamBatchArgs make_team_args(gdt_context ctx, gdt_batch b, const SolveArgs& s) {
   a.iters = b->d_iters;
   a.relres = b->d_relres;
   a.status = b->d_status;
-  a.scratch = b->team_scratch;
+  a.scratch = b->scratch64;
   a.ex.fault = reinterpret_cast<unsigned int*>(b->d_exchange);
   a.taken = reinterpret_cast<int*>(b->d_exchange + 1);
   a.ex.slots = b->d_exchange + kSlot;
@@ -1009,13 +992,6 @@ gdt_status launch(gdt_context ctx, gdt_batch b, const SolveArgs& sa, cudaStream_
   return GDT_OK;
 }
 
-// scratch of the fixed-size team kernel, where that kernel has something to do
-gdt_status prepare_scratch(gdt_context ctx, gdt_batch b, int precision) {
-  const bool planned = uses_plan(b, precision);
-  if (planned && b->items_rest.empty()) return GDT_OK;
-  return ensure_scratch(ctx, b, words_of(*b, planned ? b->items_rest : b->items));
-}
-
 // per-problem results of the last launch over `subset` into info; the status of the call
 gdt_status collect(gdt_context ctx, gdt_batch b, const std::vector<int>& subset, cudaStream_t s, gdt_batch_info* info) {
   std::vector<int> it(b->nprob), stv(b->nprob);
@@ -1055,8 +1031,6 @@ gdt_status collect(gdt_context ctx, gdt_batch b, const std::vector<int>& subset,
 
 gdt_status solve_impl(gdt_context ctx, gdt_batch b, const SolveArgs& sa, gdt_batch_info* info) {
   gdt_status st = check_solve_args(ctx, b, sa);
-  if (st != GDT_OK) return st;
-  st = prepare_scratch(ctx, b, sa.precision);
   if (st != GDT_OK) return st;
   cudaStream_t s = ctx->stream;
   cudaStream_t own = nullptr;
@@ -1226,7 +1200,6 @@ gdt_status gdt_batch_destroy(gdt_batch b) {
   cudaFree(b->d_place);
   cudaFree(b->d_tprobs);
   cudaFree(b->d_exchange);
-  cudaFree(b->team_scratch);
   cudaFree(b->d_off);
   cudaFree(b->d_eoff);
   cudaFree(b->d_cells);
@@ -1235,7 +1208,6 @@ gdt_status gdt_batch_destroy(gdt_batch b) {
   cudaFree(b->d_relres);
   cudaFree(b->d_status);
   cudaFree(b->scratch64);
-  cudaFree(b->scratch32);
   delete b;
   return GDT_OK;
 }
@@ -1317,11 +1289,10 @@ gdt_status gdt_batch_tune(gdt_context ctx, gdt_batch b, const double* kappa, int
         }
         const bool planned =
             b->team_blocks > 0 && team == GDT_BATCH_TEAM_CLUSTER && precision == GDT_PRECISION_FP64;
-        st = upload_plan(ctx, b, planned ? cls.second : std::vector<int>());
+        st = ensure_scratch(ctx, b, build_items(*b, cls.second, b->items, b->probs));
         if (st != GDT_OK) break;
-        build_items(*b, cls.second, b->items, b->probs);
         b->items_rest.clear();
-        st = prepare_scratch(ctx, b, precision);
+        st = upload_plan(ctx, b, planned ? cls.second : std::vector<int>());
         if (st != GDT_OK) break;
         if (cudaMemcpy(b->d_items, b->items.data(), sizeof(BatchItem) * b->items.size(), cudaMemcpyHostToDevice) !=
                 cudaSuccess ||
