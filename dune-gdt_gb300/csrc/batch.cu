@@ -964,9 +964,17 @@ bool uses_plan(gdt_batch b, int precision) {
   return precision == GDT_PRECISION_FP64 && !b->plan.places.empty();
 }
 
+// from now on every problem of the batch runs in the fixed-size team kernel, whose queue and scratch hold all of them
+void drop_teams(gdt_batch b) {
+  cudaGetLastError();
+  b->team_blocks = 0;
+  b->plan = TeamPlan();
+  b->generation++;
+}
+
 gdt_status launch(gdt_context ctx, gdt_batch b, const SolveArgs& sa, cudaStream_t s) {
   cudaError_t e = cudaSuccess;
-  const bool planned = uses_plan(b, sa.precision);
+  bool planned = uses_plan(b, sa.precision);
   if (planned) {
     TeamBatchArgs a = make_team_args(ctx, b, sa);
     void* args[] = {&a};
@@ -975,6 +983,11 @@ gdt_status launch(gdt_context ctx, gdt_batch b, const SolveArgs& sa, cudaStream_
     if (e == cudaSuccess)
       e = cudaLaunchCooperativeKernel(team_kernel_of(b->element), dim3(blocks), dim3(TB), args,
                                       sizeof(double) * size_t(b->team_smem), s);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {  // fewer SMs available than the device has
+      drop_teams(b);
+      planned = false;
+      e = cudaSuccess;
+    }
   }
   if (e == cudaSuccess && (!planned || !b->items_rest.empty())) {
     const BatchArgs a = make_args(b, sa, !planned);
@@ -1065,7 +1078,13 @@ gdt_status solve_impl(gdt_context ctx, gdt_batch b, const SolveArgs& sa, gdt_bat
     b->key = key;
   }
   if (b->exec) {
-    if (cudaGraphLaunch(b->exec, s) != cudaSuccess) st = fail(ctx, GDT_ECUDA, "batch graph launch");
+    const cudaError_t e = cudaGraphLaunch(b->exec, s);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {
+      drop_teams(b);  // (the next solve captures anew)
+      st = launch(ctx, b, sa, s);
+    } else if (e != cudaSuccess) {
+      st = fail(ctx, GDT_ECUDA, "batch graph launch");
+    }
   } else {
     st = launch(ctx, b, sa, s);
   }
