@@ -1188,7 +1188,7 @@ int pcg_partition(gdt_matrix m, int blocks, bool by_work, int* first) {
 // GDT_EUNSUPPORTED, before anything ran, where no cooperative launch of the kernel can be made
 // (the caller then runs the graph form).
 gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, double* p, double* q,
-                          const double* dinv, KState* st, cudaStream_t s) {
+                          const double* dinv, KState* st, cudaStream_t s, bool clusters = true) {
   int dev = 0, coop = 0, per_sm = 0;
   long long room = 0;
   GDT_TRY_CUDA(ctx, cudaGetDevice(&dev));
@@ -1200,10 +1200,10 @@ gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, d
   // four slices, one per scheduler, before the next block: 4,225 rows in 34 blocks of four warps take 5.6 us
   // an iteration, in 133 blocks of one warp 6.0 us
   blocks = std::max(1, std::min(blocks, (nslices + 3) / 4));
-  // Small systems on one cluster, unless the caller has set limits, which are the grid's. Per iteration on the grid and
+  // Small systems on one cluster, where one can be had and unless the caller has set limits, which are the grid's. Per iteration on the grid and
   // on a cluster: 20 slices of Q1 squares 4.6 and 3.5 us, 133 5.55 and 5.25, 259 5.6 and 6.3; 42 slices
   // of Q1 cubes 6.3 and 4.7, 106 6.4 and 5.6, 215 6.6 and 8.1 (16 SMs' FP64 pipes).
-  const bool cluster = ctx->persistent_blocks == 0 && ctx->persistent_wait_ns == 0 && m->max_row <= 32 &&
+  const bool cluster = clusters && ctx->persistent_blocks == 0 && ctx->persistent_wait_ns == 0 && m->max_row <= 32 &&
                        nslices <= kClusterSlices;
   if (cluster) blocks = std::min(16, std::max(1, nslices / 4));
   // slices per warp of the resident form; where a block has more rows than its registers hold, the
@@ -1281,8 +1281,11 @@ gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, d
     attr.id = cudaLaunchAttributeClusterDimension;
     attr.val.clusterDim.x = blocks;
     attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    GDT_TRY_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    GDT_TRY_CUDA(ctx, cudaOccupancyMaxActiveClusters(&per_sm, fn, &cfg));
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&per_sm, fn, &cfg) != cudaSuccess || per_sm < 1) {
+      cudaGetLastError();
+      return pcg_persistent(ctx, m, x, r, p, q, dinv, st, s, false);
+    }
   } else {
     attr.id = cudaLaunchAttributeCooperative;
     attr.val.cooperative = 1;

@@ -16,14 +16,18 @@ FAKES = {
     "cooperative": """
 int cudaLaunchCooperativeKernel(const void* f, ...) { (void)f; return 720; }
 """,
+    # no cluster of the size asked for fits
+    "cluster": """
+int cudaOccupancyMaxActiveClusters(int* n, const void* f, const void* cfg) { (void)f; (void)cfg; *n = 0; return 0; }
+""",
 }
 
 CHILD = """
 import importlib, sys
 import numpy as np, torch
 gdt = importlib.import_module("dune-gdt_gb300")
-out = {{}}
-{body}
+out = {}
+BODY
 np.savez(sys.argv[1], **out)
 """
 
@@ -43,6 +47,18 @@ for element in ("p1", "q1"):
 """
 
 
+CG = """
+for form in ("auto", "persistent"):
+    for n, simplex in (([12], False), ([64, 64], False), ([62, 80], True)):
+        g = gdt.make_cube_grid([0.0] * len(n), [1.0] * len(n), n, simplex=simplex)
+        prob = gdt.DiffusionProblem(g)
+        prob.assemble(torch.ones(g.num_elements, dtype=torch.float64, device="cuda"))
+        prob.op.ctx.set_solver_launch(form)
+        out[f"{form} {n}"] = prob.op.apply_inverse(prob.rhs, opts={"tol": 1e-11}).cpu().numpy()
+        out[f"{form} {n} launch"] = np.array(prob.op.last_solve_info["launch"])
+"""
+
+
 def _run(tmp_path, body, fake=None):
     env = dict(os.environ, PYTHONPATH=ROOT)
     if fake:
@@ -51,7 +67,7 @@ def _run(tmp_path, body, fake=None):
         subprocess.run(["gcc", "-shared", "-fPIC", "-o", str(lib), str(src)], check=True)
         env["LD_PRELOAD"] = str(lib)
     out = tmp_path / f"{fake}.npz"
-    r = subprocess.run([sys.executable, "-c", CHILD.format(body=body), str(out)], cwd=ROOT, env=env, capture_output=True,
+    r = subprocess.run([sys.executable, "-c", CHILD.replace('BODY', body), str(out)], cwd=ROOT, env=env, capture_output=True,
                        text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
     return dict(np.load(out))
@@ -65,4 +81,15 @@ def test_batch_without_cooperative_launch(tmp_path):
         if key.endswith("status"):
             assert (x == 0).all()
         else:  # both solved to 1e-11; the condition numbers are below 1e4
+            assert np.abs(x - free[key]).max() <= 1e-7 * np.abs(free[key]).max(), key
+
+
+def test_small_solves_without_cluster_run_on_the_grid(tmp_path):
+    free = _run(tmp_path, CG)
+    refused = _run(tmp_path, CG, "cluster")
+    assert free.keys() == refused.keys()
+    for key, x in refused.items():
+        if key.endswith("launch"):
+            assert str(x) == "persistent", key
+        else:
             assert np.abs(x - free[key]).max() <= 1e-7 * np.abs(free[key]).max(), key
