@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(MT, 1) k_mixed_resident(const __grid_constant_
       }
     }
     {
-      const double t = group_exchange_f32<false>(a.ex, epoch, v3, sh.ex);
+      const double t = group_exchange<false>(a.ex, epoch, v3, MW, sh.ex);
       if (threadIdx.x < 96) {
         const double inv = threadIdx.x == 0 ? 1.0 / t : 0.0;
         if (lane == 0) sh.total[warp] = t;
@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(MT, 1) k_mixed_resident(const __grid_constant_
         v[0] = fmaf(r[k], z, v[0]);
         v[1] = fmaf(r[k], r[k], v[1]);
       }
-    const double t = group_exchange_f32<true>(a.ex, epoch, v, sh.ex);
+    const double t = group_exchange<true>(a.ex, epoch, v, MW, sh.ex);
     if (threadIdx.x < 64 && lane == 0) sh.last[warp] = t;
     pending = true;
   }
