@@ -1334,11 +1334,14 @@ gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, d
   a.cap = cap;
   {
     // What of the matrix is not in shared memory stays in L2 where it fits beside the vectors (the resident form's p, five
-    // of the streaming form), four fifths of the room where it does not: a larger share evicts itself. 65^3
+    // of the streaming form) in 62 % of the cache (80 MB here: its two halves hold some lines twice), four
+    // fifths of the room where it does not: a larger share evicts itself. 65^3
     // Q1 rows (89 MB, 56 of them streamed): 41.8 us an iteration with every line evict-first, 30.6 kept;
     // 81^3 (172 MB) 79.1, 73.5 with 65 MB kept, 79.3 with 90; 129^3, where the vectors fill L2, 155 and
     // 163 with 64 MB.
-    const double vectors = (threads == PT ? 40.0 : 8.0) * double(m->rows), room = 80.0 * (1 << 20) - vectors;
+    int l2 = 0;
+    GDT_TRY_CUDA(ctx, cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev));
+    const double vectors = (threads == PT ? 40.0 : 8.0) * double(m->rows), room = 0.62 * double(l2) - vectors;
     const double streamed = (narrow ? 10.0 : 12.0) * std::max(0.0, double(m->sell_len) - double(cap) * blocks);
     a.keep = streamed <= room ? 1.f : float(std::max(0.0, 0.8 * room / streamed));
   }
