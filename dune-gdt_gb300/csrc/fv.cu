@@ -548,15 +548,32 @@ int march_chunk(gdt_context ctx, const GridDesc& g, long long nbatch) {
   return chosen;
 }
 
-// whether the tiled kernels take the grid: at least two cells per direction (a cell that neighbours itself has no
-// flux) and, in 1D and 3D, where the generic kernel takes any batch, as many blocks as a launch can have
+// Whether the tiled kernels take the grid: at least two cells per direction (a cell that neighbours itself has no
+// flux) and, in 1D and 3D, where the generic kernel takes any batch, as many blocks as a launch can have and less
+// time. Many small states leave most of their tiles empty: a tile's warp computes 32 cells of a row whether
+// they are there or not, the generic kernel each cell of the batch with every face twice. The estimates are of
+// an SSP-RK2 step in us, from these (generic and tiled; 1D: 40,000 states, 3D: 8,000, then 1,000 states):
+//   2 cells 25 and 89, 5 42 and 89, 10 72 and 88, 20 129 and 88, 64 387 and 99
+//   2^3 41 and 173, 4^3 239 and 366, 5^3 436 and 498, 6^3 748 and 650; 2 x 64 x 2 123 and 288,
+//   4 x 8 x 16 239 and 274, 8 x 8 x 2 74 and 42, 10^3 436 and 279, 32 x 4 x 4 240 and 58
+// A few states take the tiles in any case (one of 4^3 19 and 6.5, 300 of them 25 and 19).
 bool tiled_ok(gdt_context ctx, const GridDesc& g, long long nbatch) {
   for (int k = 0; k < g.dim; ++k)
     if (g.n[k] < 2) return false;
-  if (g.dim == 1) return (g.n[0] + SX - 1) / SX * nbatch < (1LL << 31);
+  const double cells = double(g.nelem) * double(nbatch);
+  if (g.dim == 1) {
+    const long long segments = (g.n[0] + SX - 1) / SX, last = g.n[0] - (segments - 1) * SX;
+    const double warps = double(segments - 1) * (SX / 32) + double((last + 31) / 32);
+    const double tiled = 4.6 + 1e-3 * double(nbatch) * (1.8 * double(segments) + 0.4 * warps);
+    return segments * nbatch < (1LL << 31) && tiled <= std::max(14.5, 10.0 + 0.15e-3 * cells);
+  }
   if (g.dim == 3) {
     const int chunk = march_chunk(ctx, g, nbatch);
-    return (g.n[1] + MY - 1) / MY <= 65535 && (g.n[2] + chunk - 1) / chunk * nbatch <= 65535;
+    const long long tiles_x = (g.n[0] + MX - 1) / MX, tiles_y = (g.n[1] + MY - 1) / MY;
+    const double plane = double(tiles_x) * (7.0 * double(tiles_y) + 1.4 * double(g.n[1]));
+    const double tiled = 6.0 + 1e-3 * double(nbatch) * double(g.n[2]) * plane;
+    return tiles_y <= 65535 && (g.n[2] + chunk - 1) / chunk * nbatch <= 65535 &&
+           tiled <= std::max(24.7, 11.0 + 0.43e-3 * cells);
   }
   return true;
 }
