@@ -19,7 +19,11 @@
 // small enough for the rounding not to matter, and there is enough of it to remove what has gathered
 // (replaced only 100x before the threshold it stays at 3e-12). It costs sixteen iterations' work.
 // A problem with a diagonal entry that is not positive (a coefficient <= 0) keeps the unscaled
-// preconditioned iteration.
+// preconditioned iteration. So does one whose tolerance is below what the rounding of the couplings leaves in the
+// residual, about n^2 eps where they are alike (kappa constant per quadrant): a replacement puts that back after CG
+// has done with the smooth part, which takes more iterations then. At 1e-12 256, 400 and 512 squares took 1,079,
+// 1,746 and 2,414 iterations scaled, with errors up to five times as large, and take 1,075, 1,674 and
+// 2,146 unscaled; 16 problems of 512 squares 254 and 287 ms, 32 of 256 65 and 80.
 #pragma once
 #include <type_traits>
 
@@ -123,6 +127,19 @@ struct TeamRow {
   __device__ __forceinline__ double dot(double s) const {
 #pragma unroll
     for (int k = 0; k < 2 * team_couplings<NS>(); ++k) s = fma(cp[k], pn[k], s);
+    return s;
+  }
+  // the whole row in the order of its columns, as batch_kernel adds it (the diagonal first leaves up to three times the
+  // error where kappa is constant per quadrant: 256 squares, tolerance 1e-12)
+  __device__ __forceinline__ double dot_by_column(double d, double p) const {
+    constexpr int C = team_couplings<NS>();
+    constexpr int order[8] = {5, 3, 7, 1, 0, 6, 2, 4};
+    double s = 0.0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      if (k == 4) s = fma(d, p, s);
+      if (order[k] < 2 * C) s = fma(cp[order[k]], pn[order[k]], s);
+    }
     return s;
   }
 };
@@ -307,7 +324,7 @@ __device__ void team_cg(const TeamBatchArgs& a, const ExchangeView& ex, unsigned
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const double q = row[u].dot(SCALED ? p[u] : d[u] * p[u]);
+        const double q = SCALED ? row[u].dot(p[u]) : row[u].dot_by_column(d[u], p[u]);
         const double mq = SCALED ? q : s[u] * q;
         wq[i0 + TB * u] = q;
         v3[0] = fma(p[u], q, v3[0]);
@@ -487,7 +504,8 @@ __device__ void team_solve(const TeamBatchArgs& a, const ExchangeView& ex, unsig
     if (threadIdx.x == 0) k.iter = k.conv = 0;
     __syncthreads();
   } else {
-    const bool scaled = nonpos == 0.0;
+    const double rounding = 2.5 * 1.1102230246251565e-16 * n * n;  // 7.3e-11 for 512 squares
+    const bool scaled = nonpos == 0.0 && a.tol2 >= rounding * rounding;
     if (scaled) team_cg<NS, true>(a, ex, epoch, prob, n, lo, hi, w, sh, total, k, b_inner);
     else team_cg<NS, false>(a, ex, epoch, prob, n, lo, hi, w, sh, total, k, b_inner);
     // the solution and its true relative residual
