@@ -17,10 +17,11 @@
 // state, Dirichlet: the prescribed one), for which the face flux is the boundary flux, since
 // g(u, v, n) = -g(v, u, -n) for all three fluxes; a prescribed flux, or none, is selected in place of the
 // computed face. Kernels: 2D tiles (fv2d_tile), 3D tiles that march along z (fv3d_march) and 1D
-// segments (fv1d_segment); grids with a single cell in some direction take fv_apply_kernel.
+// segments (fv1d_segment); grids with a single cell in some direction, and batches of many small 1D and 3D
+// states (tiled_ok), take fv_apply_kernel.
 // SSP-RK2 steps before (FP64 per face: three instructions; boundary fluxes and 1D / 3D in the generic
-// form, each face twice) and now: 2048^2 Burgers LF 197 and 162 us, with inflow and outflow 359 and 162;
-// 128 x 140 x 120 929 and 158; 100,000 cells 25 and 11; 120 x 97 with boundaries 28 and 7.5.
+// form, each face twice) and now: 2048^2 Burgers LF 197 and 161 us, with inflow and outflow 359 and 161;
+// 128 x 140 x 120 929 and 152; 100,000 cells 25 and 6.6; 120 x 97 with boundaries 28 and 7.1.
 #include <cmath>
 #include <limits>
 

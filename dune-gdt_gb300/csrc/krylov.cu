@@ -1144,13 +1144,13 @@ __global__ void __launch_bounds__(PT, 1) k_pcg_stream(const __grid_constant__ Pc
 }
 
 // Rows of at most 32 entries (the SELL-32 SpMV's limit). Per iteration, before (three counter barriers, shuffle
-// reductions, scalars in every thread) and now: 4,225 rows of Q1 squares 25.5 and 5.6 us; 68,921 of an
-// unstructured tetrahedral mesh 31.2 and 9.6; 98,304 of SWIPDG 26.0 and 9.9; 155,480 of P1 tetrahedra 29.7
-// and 11.5; 2,146,689 of 128^3 Q1 (streaming, 727.7 MB of matrix) 209 and 146
-// (178 before the gathers went ahead of the products, 154 with 32-bit columns). The graph form takes
-// 51.7 us for 393,216 rows of SWIPDG and 264 us for 128^3: AUTO takes this form wherever it applies.
+// reductions, scalars in every thread) and now, as slopes between two iteration counts: 4,225 rows of Q1 squares
+// 25.5 and 5.3 us on a cluster, 5.5 on the grid; 68,921 of an unstructured tetrahedral mesh 31.2 and 10.0;
+// 98,304 of SWIPDG 26.0 and 10.2; 155,480 of P1 tetrahedra 29.7 and 12.2; 2,146,689 of 128^3 Q1 (streaming,
+// 727.7 MB of matrix) 209 and 152, 156 with the setup of a solve. The graph form takes 51.7 us for
+// 393,216 rows of SWIPDG (27 here) and 264 us for 128^3: AUTO takes this form wherever it applies.
 // Longer rows too where the form is left to the library (28^3 Q2 cubes, 185,193 rows of up to 125 entries: 60 us in
-// the graph form, 48 here; 15,625 rows 37 and 21); a caller who asks for the persistent form gets it for rows of at most 32.
+// the graph form, 42 here; 15,625 rows 37 and 13); a caller who asks for the persistent form gets it for rows of at most 32.
 bool persistent_applies(gdt_context ctx, gdt_matrix m) {
   if (ctx->timing || ctx->solver_launch == GDT_SOLVER_LAUNCH_GRAPH) return false;
   return m->max_row >= 1 && m->rows >= 1 &&
@@ -1257,8 +1257,8 @@ gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, d
     dyn = size_t(cap) * 12;
   }
   // streaming by slices: the columns as 16-bit differences where they fit (10 bytes an entry instead of 12), q in shared
-  // memory where it fits. 128^3 Q1: 165 us an iteration, 160 and 161 with one of them, 156 with both; 91^3
-  // rows, which L2 holds better: 63 and 62.
+  // memory where it fits. 128^3 Q1, with the setup: 165 us an iteration, 160 and 161 with one of them, 156 with both;
+  // 91^3 rows, which L2 holds better: 63 and 62.
   const bool narrow = fn == reinterpret_cast<const void*>(&k_pcg_stream<false, int>) && m->sell_band <= 32767;
   if (narrow) fn = reinterpret_cast<const void*>(&k_pcg_stream<false, short>);
   a.qshared = 0;

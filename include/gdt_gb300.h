@@ -109,11 +109,12 @@ gdt_status gdt_measure_l2_bandwidth(gdt_context ctx, double* gbs);
 
 /* How gdt_solve runs FP64 CG with Jacobi or no preconditioner (no reference counterpart: the launch
  * form of the device solver). GRAPH: one kernel per step (SpMV, update, direction), iterations
- * captured in CUDA graphs. PERSISTENT: one cooperative launch runs every iteration, with grid
- * barriers between the steps and a SELL-32 copy of the matrix; it takes matrices whose rows hold at
- * most 32 entries. AUTO (default): PERSISTENT wherever it applies (it was faster both for systems
+ * captured in CUDA graphs. PERSISTENT: one cooperative launch (systems of up to 5,120 rows: one cluster) runs
+ * every iteration, with grid-wide sums between the steps and a SELL-32 copy of the matrix of its own (10 or 12
+ * bytes per padded entry, for the time of the solve); it takes matrices whose rows hold at most 32 entries. AUTO (default): PERSISTENT wherever it applies (it was faster both for systems
  * that stay in L2 and for ones streamed from HBM) and for rows of up to 512 entries that the copy pads by less
- * than half, GRAPH otherwise or where no cooperative launch or no room for the copy is available. Timing mode always runs GRAPH's kernels launched one by one. */
+ * than half, GRAPH otherwise or where no cooperative launch or no room for the copy is available. Timing
+ * mode always runs GRAPH's kernels launched one by one. */
 #define GDT_SOLVER_LAUNCH_AUTO 0
 #define GDT_SOLVER_LAUNCH_GRAPH 1
 #define GDT_SOLVER_LAUNCH_PERSISTENT 2
@@ -127,7 +128,9 @@ int gdt_context_last_solver_launch(gdt_context ctx);
  * tests of the launch form): blocks caps the grid (0: one block per SM, the default), wait_limit_ns
  * bounds every wait at a grid barrier (0: the default of one second). A wait that runs out sets a
  * device flag, every block leaves at its next barrier, and the solve returns GDT_ECUDA ("a grid
- * barrier wait ran out"); the context stays usable. */
+ * barrier wait ran out"); the context stays usable. Small systems, which take one cluster otherwise, run on the
+ * grid while a limit is set. A batch takes the wait limit at every solve, and the block limit when it is
+ * created. */
 gdt_status gdt_context_set_persistent_limits(gdt_context ctx, int blocks, int64_t wait_limit_ns);
 
 /* --------------------------------------------------------------------- grid --- */
