@@ -293,6 +293,7 @@ gdt_status tune_spmv(gdt_context ctx, gdt_matrix m, double* times_ms) {
   }
   // the SELL-32 copy, when there is room for it
   bool sell_best = false;
+  const bool kept = m->sell_col != nullptr;
   m->csr_products = 0;
   if (sell_prepare(ctx, m, s, false) == GDT_OK) {
     float ms = 0.f, fill = 0.f;
@@ -312,8 +313,9 @@ gdt_status tune_spmv(gdt_context ctx, gdt_matrix m, double* times_ms) {
   cudaFreeAsync(y, s);
   m->spmv_sched = best_sched;
   m->use_sell = sell_best ? 1 : 0;
-  // keep the copy only where the SpMV reads it (solves that need one fill their own, or allocate this one again)
-  if (!sell_best) sell_release(m);
+  // keep the copy only where the SpMV reads it (solves that need one fill their own, or allocate this one again), or where
+  // one was there before: a product captured in a caller's graph may read it
+  if (!sell_best && !kept) sell_release(m);
   m->tuned = 1;
   return GDT_OK;
 }

@@ -75,3 +75,26 @@ def test_captured_fill_does_not_count_as_done(gdt):
                 graph.replay()
                 torch.cuda.synchronize()
                 assert float((y - expected).abs().max()) <= 1e-12 * float(expected.abs().max()), (schedule, k)
+
+
+# Tuning anew may choose another schedule; the copy that a captured product reads stays
+@pytest.mark.parametrize("n,simplex", [([64, 63], True), ([17], False), ([30, 29, 31], False)])
+def test_replayed_product_after_tuning_anew(gdt, n, simplex):
+    op, rhs, stream = _system(gdt, n, simplex)
+    op.set_spmv_schedule(8)
+    x = torch.randn(rhs.numel(), dtype=torch.float64, device="cuda", generator=torch.Generator("cuda").manual_seed(5))
+    y = torch.zeros_like(rhs)
+    torch.cuda.synchronize()
+    expected = op.apply(x)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        op.apply(x, y)
+    for _ in range(3):
+        assert gdt._capi.load().gdt_matrix_tune(op.ctx.handle, op.handle, None, None) == gdt._capi.OK
+        stream.synchronize()
+        y.zero_()
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(y, expected)
