@@ -48,7 +48,7 @@ struct FvParams {
 };
 
 enum { FORM4_BURGERS_LF, FORM4_BURGERS_LF_FIXED, FORM4_BURGERS_EO, FORM4_BURGERS_UPWIND, FORM4_TRANSPORT_LINEAR,
-       FORM4_TRANSPORT_EO };
+       FORM4_TRANSPORT_UPWIND, FORM4_TRANSPORT_EO };
 
 __device__ __forceinline__ double f_of(const FvParams& p, double u, int d) {
   return p.flux == GDT_FLUX_BURGERS ? 0.5 * u * u : p.vel[d] * u;
@@ -114,7 +114,10 @@ __device__ __forceinline__ double boundary_face_flux(const FvParams& p, int dim,
 // The tiled kernels work with 4 g: the factors 1/2 of the flux formulas move into the 1/4 of the update
 // coefficients (scaling by powers of two is exact) and the transport fluxes collapse to precomputed
 // linear combinations.
-__device__ __forceinline__ bool positive(double u) { return __double_as_longlong(u) > 0; }
+// u > 0 on the bit pattern (false for NaN, as in the flux formulas)
+__device__ __forceinline__ bool positive(double u) {
+  return (unsigned long long)__double_as_longlong(u) - 1 < 0x7ffull << 52;
+}
 // 2 q for a square q >= 0 (or NaN) on its bit pattern: a normal number's exponent plus one, a subnormal's bits
 // shifted, infinity where that overflows
 __device__ __forceinline__ double twice(double q) {
@@ -176,6 +179,8 @@ __device__ __forceinline__ double fv_face4(const FvParams& p, int k, double u, d
     return fma(p.lam2, u - v, qu + qv);
   } else if constexpr (FORM == FORM4_TRANSPORT_LINEAR) {
     return fma(p.tu[k], u, p.tv[k] * v);
+  } else if constexpr (FORM == FORM4_TRANSPORT_UPWIND) {  // one of the states alone, whatever the other is
+    return p.tu[k] != 0.0 ? p.tu[k] * u : p.tv[k] * v;
   } else if constexpr (FORM == FORM4_BURGERS_EO) {  // 4 * (u > 0 ? u^2 / 2 : 0)
     return positive(u) ? qu : 0.0;
   } else if constexpr (FORM == FORM4_TRANSPORT_EO) {
@@ -506,7 +511,9 @@ FvParams make_params(const GridDesc& g, const gdt_fv_desc* d) {
     double lam = 0.0;
     for (int k = 0; k < g.dim; ++k) lam = std::max(lam, std::fabs(d->velocity[k]));
     if (d->lf_lambda != 0.0) lam = 1.0 / d->lf_lambda;
-    p.form4 = d->numflux == GDT_NUMFLUX_ENGQUIST_OSHER ? FORM4_TRANSPORT_EO : FORM4_TRANSPORT_LINEAR;
+    p.form4 = d->numflux == GDT_NUMFLUX_ENGQUIST_OSHER ? FORM4_TRANSPORT_EO
+              : d->numflux == GDT_NUMFLUX_UPWIND       ? FORM4_TRANSPORT_UPWIND
+                                                       : FORM4_TRANSPORT_LINEAR;
     for (int k = 0; k < 3; ++k) {
       const double a = d->velocity[k];
       if (d->numflux == GDT_NUMFLUX_LAX_FRIEDRICHS) {  // 2 (a (u + v) + lambda (u - v))
@@ -635,6 +642,7 @@ void launch_stage(gdt_context ctx, const GridDesc& g, const FvParams& p, long lo
     case FORM4_BURGERS_EO: launch_form<STAGE, FORM4_BURGERS_EO>(ctx, g, p, a, nbatch); break;
     case FORM4_BURGERS_UPWIND: launch_form<STAGE, FORM4_BURGERS_UPWIND>(ctx, g, p, a, nbatch); break;
     case FORM4_TRANSPORT_LINEAR: launch_form<STAGE, FORM4_TRANSPORT_LINEAR>(ctx, g, p, a, nbatch); break;
+    case FORM4_TRANSPORT_UPWIND: launch_form<STAGE, FORM4_TRANSPORT_UPWIND>(ctx, g, p, a, nbatch); break;
     default: launch_form<STAGE, FORM4_TRANSPORT_EO>(ctx, g, p, a, nbatch); break;
   }
 }
