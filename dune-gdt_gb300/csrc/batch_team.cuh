@@ -506,10 +506,14 @@ __device__ void team_solve(const TeamBatchArgs& a, const ExchangeView& ex, unsig
   } else {
     const double rounding = 2.5 * 1.1102230246251565e-16 * n * n;  // 7.3e-11 for 512 squares
     const bool scaled = nonpos == 0.0 && a.tol2 >= rounding * rounding;
-    if (scaled) team_cg<NS, true>(a, ex, epoch, prob, n, lo, hi, w, sh, total, k, b_inner);
+    // the scaled system with a load of about d^1/4 (a power of two times this one: the same bits): its sums go with b^2 / d
+    // and with b^2, and both stay in the range of a double for any coefficient
+    const int e = scaled && b_inner != 0.0 && isfinite(k.dmin) ? ilogb(k.dmin) / 4 - ilogb(b_inner) : 0;
+    const double unit = scalbn(1.0, -e);
+    if (scaled) team_cg<NS, true>(a, ex, epoch, prob, n, lo, hi, w, sh, total, k, scalbn(b_inner, e));
     else team_cg<NS, false>(a, ex, epoch, prob, n, lo, hi, w, sh, total, k, b_inner);
     // the solution and its true relative residual
-    for (int i = lo + threadIdx.x; i < hi; i += TB) x[i] = scaled ? w.s[i] * w.x[i] : w.x[i];
+    for (int i = lo + threadIdx.x; i < hi; i += TB) x[i] = scaled ? w.s[i] * w.x[i] * unit : w.x[i];
     double v[2] = {0.0, 0.0};
     double none[1] = {0.0};
     group_exchange<true>(ex, epoch, none, TB / 32, sh);

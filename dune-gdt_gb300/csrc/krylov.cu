@@ -686,7 +686,8 @@ struct PcgArgs {
 // The scalars of the iteration, kept by thread 0 of every block (the same bits in all of them).
 struct PcgScalars {
   double rho, alpha, beta, rr, stop;
-  int iter, max_iter, conv, brk;
+  int iter, max_iter, conv;
+  int brk;  // 1: breakdown; 2: alpha or beta left the range of a double, the iterate before it is good
   __device__ void load(const KState* st) {
     rho = st->rho;
     alpha = st->alpha;
@@ -717,6 +718,9 @@ struct PcgShared {
   int go;
 };
 
+// on the integer pipe: thread 0 decides while the others wait
+__device__ __forceinline__ bool finite_bits(double v) { return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000; }
+
 // v = (p.q, z.q, q.D^-1 q) over the rows of the thread: alpha and beta in sh.k; false when done. The stopping test
 // of the iteration before is made here too: its sums (sh.last) are formed while the other warps
 // already multiply, so a solve ends with one product it does not use.
@@ -738,12 +742,13 @@ __device__ __forceinline__ bool pcg_step(const PcgArgs& a, unsigned int& epoch, 
         k.rr = sh.last[1];
         k.iter += 1;
         if (k.rr <= k.stop || k.iter >= k.max_iter) k.conv = 1;
-        if (!isfinite(k.rr)) k.brk = k.conv = 1;
+        if (!finite_bits(k.rr)) k.brk = k.conv = 1;
       }
       if (!k.conv) {
         k.alpha = k.rho * inv;
         k.beta = fma(k.alpha * inv, sh.total[2], fma(-2.0 * inv, sh.total[1], 1.0));
-        if (!(total > 0.0) || !isfinite(total)) k.brk = k.conv = 1;
+        if (__double_as_longlong(total) <= 0 || !finite_bits(total)) k.brk = k.conv = 1;
+        else if (!finite_bits(k.alpha) || !finite_bits(k.beta)) k.brk = 2, k.conv = 1;
       }
       sh.go = !k.conv && !sh.ex.fault;
     }
@@ -1184,11 +1189,10 @@ int pcg_partition(gdt_matrix m, int blocks, bool by_work, int* first) {
   return slices;
 }
 
-// Runs the iterations after residual_init; the caller reads the final state from st. Returns
-// GDT_EUNSUPPORTED, before anything ran, where no cooperative launch of the kernel can be made
-// (the caller then runs the graph form).
+// Runs the iterations after residual_init; fin receives the final state. Returns GDT_EUNSUPPORTED, before anything ran,
+// where no cooperative launch of the kernel can be made (the caller then runs the graph form).
 gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, double* p, double* q,
-                          const double* dinv, KState* st, cudaStream_t s, bool clusters = true) {
+                          const double* dinv, KState* st, KState* fin, cudaStream_t s, bool clusters = true) {
   int dev = 0, coop = 0, per_sm = 0;
   long long room = 0;
   GDT_TRY_CUDA(ctx, cudaGetDevice(&dev));
@@ -1284,7 +1288,7 @@ gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, d
     if (cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&per_sm, fn, &cfg) != cudaSuccess || per_sm < 1) {
       cudaGetLastError();
-      return pcg_persistent(ctx, m, x, r, p, q, dinv, st, s, false);
+      return pcg_persistent(ctx, m, x, r, p, q, dinv, st, fin, s, false);
     }
   } else {
     attr.id = cudaLaunchAttributeCooperative;
@@ -1356,6 +1360,7 @@ gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, d
   ctx->launches++;
   unsigned int fault = 0;
   GDT_TRY_CUDA(ctx, cudaMemcpyAsync(&fault, a.ex.fault, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
+  GDT_TRY_CUDA(ctx, cudaMemcpyAsync(fin, st, sizeof(KState), cudaMemcpyDeviceToHost, s));
   GDT_TRY_CUDA(ctx, cudaStreamSynchronize(s));
   if (fault) return fail(ctx, GDT_ECUDA, "persistent solver: a grid barrier wait ran out");
   return GDT_OK;
@@ -1547,6 +1552,7 @@ gdt_status solve(gdt_context ctx, gdt_matrix m, const double* b, double* x, cons
       allocs.push_back(ilu.lorder);
       allocs.push_back(ilu.uorder);
     }
+    KState reached{};  // of a persistent launch
     const int chunk_used = (o->precond == GDT_PREC_ILU0) ? std::min(chunk, 2) : chunk;
     const int max_chunks = o->max_iter / chunk_used + 2;
     if (o->solver == GDT_SOLVER_CG) {
@@ -1560,13 +1566,17 @@ gdt_status solve(gdt_context ctx, gdt_matrix m, const double* b, double* x, cons
           GDT_TRY_CUDA(ctx, cudaMemcpyAsync(one, ones.data(), vb, cudaMemcpyHostToDevice, s));
           GDT_TRY_CUDA(ctx, cudaStreamSynchronize(s));
         }
-        bool persistent = persistent_applies(ctx, m);
+        bool persistent = persistent_applies(ctx, m), resumed = false;
         if (persistent) {
           residual_init<double>(L, m->rp, m->col, m->val, x, b, r, one, p, st);
-          const gdt_status ps = pcg_persistent(ctx, m, x, r, p, q, one, st, s);
+          const gdt_status ps = pcg_persistent(ctx, m, x, r, p, q, one, st, &reached, s);
           if (ps == GDT_EUNSUPPORTED) persistent = false;  // x untouched: the graph form starts afresh
           else if (ps != GDT_OK) return ps;
           else ctx->last_solver_launch = GDT_SOLVER_LAUNCH_PERSISTENT;
+          // coefficients of 1e260 or 1e-260 say: the products that beta is formed from leave the range of a double, those
+          // of the classical form need not. The graph form goes on from the last iterate.
+          resumed = persistent && reached.breakdown == 2;
+          if (resumed) persistent = false;
         }
         if (!persistent) {
           ctx->last_solver_launch = GDT_SOLVER_LAUNCH_GRAPH;
@@ -1575,6 +1585,10 @@ gdt_status solve(gdt_context ctx, gdt_matrix m, const double* b, double* x, cons
           const bool cg_sell = m->cg_sched == kSellSchedule && sell_prepare(ctx, m, s, true) == GDT_OK;
           L.sched = m->cg_sched == kSellSchedule ? m->spmv_sched : m->cg_sched;
           residual_init<double>(L, m->rp, m->col, m->val, x, b, r, one, p, st);
+          if (resumed) {  // (the tolerance is relative to the first residual)
+            GDT_TRY_CUDA(ctx, cudaMemcpyAsync(&st->rr0, &reached.rr0, sizeof(double), cudaMemcpyHostToDevice, s));
+            GDT_TRY_CUDA(ctx, cudaMemcpyAsync(&st->iter, &reached.iter, sizeof(int), cudaMemcpyHostToDevice, s));
+          }
           // pairs of rows per thread when every vector is 16-byte aligned (the solver's own are; x is
           // the caller's)
           const bool pairs = (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
@@ -1646,9 +1660,11 @@ gdt_status solve(gdt_context ctx, gdt_matrix m, const double* b, double* x, cons
         ctx->launches += 4;
       }));
     }
-    KState fin;
-    GDT_TRY_CUDA(ctx, cudaMemcpyAsync(&fin, st, sizeof(KState), cudaMemcpyDeviceToHost, s));
-    GDT_TRY_CUDA(ctx, cudaStreamSynchronize(s));
+    KState fin = reached;
+    if (ctx->last_solver_launch != GDT_SOLVER_LAUNCH_PERSISTENT) {
+      GDT_TRY_CUDA(ctx, cudaMemcpyAsync(&fin, st, sizeof(KState), cudaMemcpyDeviceToHost, s));
+      GDT_TRY_CUDA(ctx, cudaStreamSynchronize(s));
+    }
     {
       cudaError_t e = cudaGetLastError();
       if (e != cudaSuccess) return fail(ctx, GDT_ECUDA, std::string("krylov: ") + cudaGetErrorString(e));
