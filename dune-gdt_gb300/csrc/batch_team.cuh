@@ -506,9 +506,9 @@ __device__ void team_solve(const TeamBatchArgs& a, const ExchangeView& ex, unsig
   } else {
     const double rounding = 2.5 * 1.1102230246251565e-16 * n * n;  // 7.3e-11 for 512 squares
     const bool scaled = nonpos == 0.0 && a.tol2 >= rounding * rounding;
-    // the scaled system with a load of about d^1/4 (a power of two times this one: the same bits): its sums go with b^2 / d
-    // and with b^2, and both stay in the range of a double for any coefficient
-    const int e = scaled && b_inner != 0.0 && isfinite(k.dmin) ? ilogb(k.dmin) / 4 - ilogb(b_inner) : 0;
+    // the scaled system with d^1/4 times the load (a power of two: the same bits): its sums go with b^2 / d and with
+    // b^2, and both stay in the range of a double for any coefficient
+    const int e = scaled && isfinite(k.dmin) ? ilogb(k.dmin) / 4 : 0;
     const double unit = scalbn(1.0, -e);
     if (scaled) team_cg<NS, true>(a, ex, epoch, prob, n, lo, hi, w, sh, total, k, scalbn(b_inner, e));
     else team_cg<NS, false>(a, ex, epoch, prob, n, lo, hi, w, sh, total, k, b_inner);
