@@ -1204,9 +1204,9 @@ gdt_status pcg_persistent(gdt_context ctx, gdt_matrix m, double* x, double* r, d
   // four slices, one per scheduler, before the next block: 4,225 rows in 34 blocks of four warps take 5.6 us
   // an iteration, in 133 blocks of one warp 6.0 us
   blocks = std::max(1, std::min(blocks, (nslices + 3) / 4));
-  // Small systems on one cluster, where one can be had and unless the caller has set limits, which are the grid's. Per iteration on the grid and
-  // on a cluster: 20 slices of Q1 squares 4.6 and 3.5 us, 133 5.55 and 5.25, 259 5.6 and 6.3; 42 slices
-  // of Q1 cubes 6.3 and 4.7, 106 6.4 and 5.6, 215 6.6 and 8.1 (16 SMs' FP64 pipes).
+  // Small systems on one cluster, where one can be had and unless the caller has set limits, which are the grid's. Per
+  // iteration on the grid and on a cluster: 20 slices of Q1 squares 4.6 and 3.5 us, 133 5.5 and 5.3, 259 5.6 and
+  // 6.3; 42 slices of Q1 cubes 6.3 and 4.7, 106 6.4 and 5.6, 215 6.6 and 8.1 (16 SMs' FP64 pipes).
   const bool cluster = clusters && ctx->persistent_blocks == 0 && ctx->persistent_wait_ns == 0 && m->max_row <= 32 &&
                        nslices <= kClusterSlices;
   if (cluster) blocks = std::min(16, std::max(1, nslices / 4));
@@ -1573,8 +1573,8 @@ gdt_status solve(gdt_context ctx, gdt_matrix m, const double* b, double* x, cons
           if (ps == GDT_EUNSUPPORTED) persistent = false;  // x untouched: the graph form starts afresh
           else if (ps != GDT_OK) return ps;
           else ctx->last_solver_launch = GDT_SOLVER_LAUNCH_PERSISTENT;
-          // coefficients of 1e260 or 1e-260 say: the products that beta is formed from leave the range of a double, those
-          // of the classical form need not. The graph form goes on from the last iterate.
+          // coefficients near 1e290, say: the products that beta is formed from leave the range of a double, the
+          // quotients of the classical form need not. The graph form goes on from the last iterate.
           resumed = persistent && reached.breakdown == 2;
           if (resumed) persistent = false;
         }
